@@ -13,6 +13,7 @@
 // into shared memory tile by tile), and the lanes' sums meet in a shuffle tree.  How k is dealt out over the lanes depends on
 // nothing but k, so a row's result does not depend on what else is in the batch here either.
 #include "common.cuh"
+#include "sm100.cuh"
 #include "api.h"
 
 using namespace rb;
@@ -171,6 +172,243 @@ gemm_tn_large_kernel(const XT* __restrict__ x, const WT* __restrict__ w, const f
             out[(size_t)m * ldo + n] = from_f32<OT>(v);
         }
     }
+}
+
+// ---- more than 16 rows of 32-bit operands: tiles in a pipeline, k split over a cluster --------------------
+// Bound by the FMA lanes (128 a multiprocessor) once they have work: a prompt of a few hundred tokens has fewer
+// large tiles than the device has multiprocessors, and the plain tiles above ran such products at 10 TFLOP/s.
+// So the tiles are lower (32 or 64 rows: 181 rows are 3 x 64, not 2 x 128), and the sum over k is split over the
+// blocks of a thread-block cluster until about two blocks a multiprocessor are at work; the parts meet in shared
+// memory, added in the order of k, so that no partial sums go through global memory and the result is one piece.
+// Tiles of 32 k arrive by cp.async in their own layout (rows of 36 floats: eight neighbouring rows' 16-byte groups
+// fall on different banks), three stages deep.  A thread owns 8 x 8 (BM = 64) or 8 x 4 outputs, rows and columns
+// interleaved over the warp so that a warp's 16-byte read is 4 or 8 different groups; a 16-byte group is two
+// pairs of k, and each accumulator is a pair (even k, odd k) fed by the two-FMA instruction, so nothing is
+// packed or transposed anywhere.  At K = 2,048, before and after: 61 x 4,096 162 -> 35 us, 181 x 8,192 372 -> 164 us,
+// 500 x 2,048 304 -> 111 us, 4,096 x 4,096 1,558 -> 1,396 us (49 TFLOP/s); its error against 64 bits falls from 8e-7 to 2..6e-7.
+constexpr int FBN = 128, FBK = 32, FLD = FBK + 4, FSTAGES = 3, FTHREADS = 128;
+template <int BM_> struct F32Tile {
+    static constexpr int TJ = BM_ == 64 ? 8 : 4;                  // columns a thread
+    static constexpr int WARPS_N = BM_ == 64 ? 2 : 4;             // warps side by side
+    static constexpr int STAGE = (BM_ + FBN) * FLD;               // floats
+    static constexpr int SMEM = FSTAGES * STAGE * 4;
+    static_assert(BM_ * FBN <= FSTAGES * STAGE, "the finished tile reuses the stages");
+};
+
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+template <int BM_>
+__global__ void __launch_bounds__(FTHREADS, 2)
+gemm_f32_cluster_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                        float* __restrict__ out, int M, int N, int K, long long ldx, long long ldo) {
+    using T = F32Tile<BM_>;
+    constexpr int TJ = T::TJ;
+    extern __shared__ __align__(16) float fsm[];
+    pdl_trigger();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = blockIdx.y * BM_, n0 = blockIdx.x * FBN;
+    const int parts = gridDim.z, part = blockIdx.z;               // the cluster spans the whole of z
+    const int kt_total = (K + FBK - 1) / FBK;
+    const int kt0 = (int)((long long)part * kt_total / parts);
+    const int n_kt = (int)((long long)(part + 1) * kt_total / parts) - kt0;
+    const int ty = lane >> 3, tx = lane & 7;
+    const int wm = (warp / T::WARPS_N) * 32, wn = (warp % T::WARPS_N) * (8 * TJ);
+
+    // A thread copies one 16-byte group (the same columns of k) of every 16th row; the rows' addresses are a step apart.
+    // Beyond the matrix nothing is read (the first row's address stands in) and zeros are written.
+    const int cr = tid >> 3, cc = (tid & 7) * 4;
+    const float* wp = w + (size_t)(n0 + min(cr, N - 1 - n0)) * K + kt0 * FBK + cc;
+    const float* xp = x + (size_t)(m0 + min(cr, M - 1 - m0)) * ldx + kt0 * FBK + cc;
+    const long long w_step = 16ll * K, x_step = 16ll * ldx;
+    const int w_left = N - n0 - cr, x_left = M - m0 - cr;         // rows from this thread's first to the matrix's end
+    int k_left = K - kt0 * FBK - cc;                              // the same for k, at the tile that is requested next
+    const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(fsm + cr * FLD + cc);
+    auto copy = [](uint32_t dst, const float* src, bool in) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+    };
+    auto fetch_w = [&](int stage, int ahead) {                    // `ahead`: k tiles beyond the one the pointers stand at
+        const uint32_t d = dst0 + (stage * T::STAGE + BM_ * FLD) * 4;
+        const bool k_in = ahead * FBK < k_left;
+        const float* base = k_in ? wp + ahead * FBK : w;
+#pragma unroll
+        for (int u = 0; u < FBN / 16; ++u) {
+            const bool in = k_in && u * 16 < w_left;
+            copy(d + u * 16 * FLD * 4, in ? base + u * w_step : w, in);
+        }
+    };
+    auto fetch_x = [&](int stage, int ahead) {
+        const uint32_t d = dst0 + stage * T::STAGE * 4;
+        const bool k_in = ahead * FBK < k_left;
+        const float* base = k_in ? xp + ahead * FBK : x;
+#pragma unroll
+        for (int u = 0; u < BM_ / 16; ++u) {
+            const bool in = k_in && u * 16 < x_left;
+            copy(d + u * 16 * FLD * 4, in ? base + u * x_step : x, in);
+        }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    // the weight does not depend on the kernel before this one
+#pragma unroll
+    for (int kt = 0; kt < FSTAGES - 1; ++kt)
+        if (kt < n_kt) fetch_w(kt, kt);
+    pdl_wait();
+#pragma unroll
+    for (int kt = 0; kt < FSTAGES - 1; ++kt) {
+        if (kt < n_kt) fetch_x(kt, kt);
+        commit();                                                 // group 0 also holds every weight tile requested above
+    }
+    unsigned long long acc[8][TJ];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < TJ; ++j) acc[i][j] = 0ull;
+    wp += (FSTAGES - 1) * FBK; xp += (FSTAGES - 1) * FBK; k_left -= (FSTAGES - 1) * FBK;
+    int use = 0, refill = FSTAGES - 1;                            // stages
+    for (int kt = 0; kt < n_kt; ++kt) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
+        __syncthreads();          // tile kt is here, and nobody reads the stage that is refilled next any more
+        if (kt + FSTAGES - 1 < n_kt) {
+            fetch_w(refill, 0);
+            fetch_x(refill, 0);
+            wp += FBK; xp += FBK; k_left -= FBK;
+        }
+        commit();                                                 // an empty group at the end keeps the count
+        const float* xs = fsm + use * T::STAGE + (wm + ty) * FLD;
+        const float* ws = fsm + use * T::STAGE + (BM_ + wn + tx) * FLD;
+        use = use + 1 == FSTAGES ? 0 : use + 1;
+        refill = refill + 1 == FSTAGES ? 0 : refill + 1;
+#pragma unroll
+        for (int c = 0; c < FBK; c += 4) {
+            ulonglong2 a[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 4 * FLD + c);
+#pragma unroll
+            for (int j = 0; j < TJ; ++j) {
+                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ws + j * 8 * FLD + c);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i][j] = fma2(a[i].x, b.x, acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i][j] = fma2(a[i].y, b.y, acc[i][j]);
+            }
+        }
+    }
+    // the finished part goes to this block's shared memory, row by row ...
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < TJ; ++j) {
+            const float lo = __uint_as_float((unsigned)acc[i][j]), hi = __uint_as_float((unsigned)(acc[i][j] >> 32));
+            fsm[(wm + ty + 4 * i) * FBN + wn + tx + 8 * j] = lo + hi;
+        }
+    // ... and every block adds and writes its share of the tile, four columns at a time
+    if (parts > 1) { sm100::cluster_arrive(); sm100::cluster_wait(); }
+    else __syncthreads();
+    const bool vec = (((uintptr_t)out | ((uintptr_t)ldo * 4)) & 15) == 0;
+    for (int g = part * FTHREADS + tid; g < BM_ * FBN / 4; g += parts * FTHREADS) {
+        const int r = g / (FBN / 4), c = (g % (FBN / 4)) * 4;
+        const int m = m0 + r, n = n0 + c;
+        if (m >= M || n >= N) continue;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (parts > 1) {
+            const uint32_t here = (uint32_t)__cvta_generic_to_shared(fsm + g * 4);
+#pragma unroll 1
+            for (int z = 0; z < parts; ++z) {
+                float4 p;
+                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(sm100::map_to_cta(here, z)) : "memory");
+                v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
+            }
+        } else {
+            const float4 p = *reinterpret_cast<const float4*>(fsm + g * 4);
+            v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w;
+        }
+        float* o = out + (size_t)m * ldo + n;
+        if (bias != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] += n + i < N ? bias[n + i] : 0.f;
+        }
+        if (vec && n + 4 <= N) {
+            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (n + i < N) o[i] = v[i];
+        }
+    }
+    __syncwarp();
+    if (parts > 1) { sm100::cluster_arrive(); sm100::cluster_wait(); }       // nobody leaves while its part may still be read
+}
+
+// In how many parts the sum over k is split (1 to 8): the cheapest of the parts that leave at least four k tiles each,
+// counted in k tiles: rounds of resident clusters times a part's tiles, with a block's start, end and meeting taken
+// as four tiles.  clusters[p] is asked of the driver: odd sizes leave multiprocessors empty (296 blocks of two,
+// 279 of three, 284 of four, 264 of eight).  A second block on a multiprocessor costs the first nothing (61 x 4,096 on 128
+// blocks and 61 x 8,192 on 256 both take 58 us at K = 2,048), so a round is a round however full it is.
+int f32_parts(long long tiles, int k_tiles, const int* clusters, long long& best_cost) {
+    int best = 1;
+    best_cost = -1;
+    for (int p = 1; p <= 8 && (p == 1 || k_tiles / p >= 4); ++p) {
+        if (clusters[p] < 1) continue;
+        const long long cost = (tiles + clusters[p] - 1) / clusters[p] * ((k_tiles + p - 1) / p + 4);
+        if (best_cost < 0 || cost < best_cost) { best = p; best_cost = cost; }
+    }
+    return best;
+}
+
+template <typename XT, typename WT, typename OT>
+int launch(const void* x, const void* w, const void* bias, void* out, int M, int N, int K, long long ldx, long long ldo, cudaStream_t s);
+
+template <int BM_>
+int launch_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, long long ldx, long long ldo,
+               cudaStream_t s) {
+    // what the device holds at once, asked once a process (one kind of device)
+    struct Facts { int error = 0, clusters[9] = {}; };
+    static const Facts facts = [] {
+        Facts f;
+        auto k = gemm_f32_cluster_kernel<BM_>;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Tile<BM_>::SMEM);
+        for (int p = 1; p <= 8 && e == cudaSuccess; ++p) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(8, 1, p);
+            cfg.blockDim = dim3(FTHREADS);
+            cfg.dynamicSmemBytes = F32Tile<BM_>::SMEM;
+            cudaLaunchAttribute a[1];
+            a[0].id = cudaLaunchAttributeClusterDimension;
+            a[0].val.clusterDim.x = 1;
+            a[0].val.clusterDim.y = 1;
+            a[0].val.clusterDim.z = p;
+            cfg.attrs = a;
+            cfg.numAttrs = 1;
+            e = cudaOccupancyMaxActiveClusters(&f.clusters[p], k, &cfg);
+        }
+        f.error = (int)e;
+        return f;
+    }();
+    if (facts.error) return facts.error;
+    const long long tiles = (long long)((N + FBN - 1) / FBN) * ((M + BM_ - 1) / BM_);
+    const int k_tiles = (K + FBK - 1) / FBK;
+    long long cost;
+    const int parts = f32_parts(tiles, k_tiles, facts.clusters, cost);
+    // The plain 128 x 128 tiles take 1.85 times a round's time; they stay where they need one round and these nearly two
+    // (500 x 8,192 at K = 2,048: 256 tiles against 512; 395 against 410 us).
+    const long long large = (long long)((N + LBN - 1) / LBN) * ((M + LBM - 1) / LBM);
+    if (large <= facts.clusters[1] && 20 * cost > 37ll * k_tiles)
+        return launch<float, float, float>(x, w, bias, out, M, N, K, ldx, ldo, s);
+    dim3 grid((N + FBN - 1) / FBN, (M + BM_ - 1) / BM_, parts);
+    if (grid.y > 65535) return RB_ERR_BAD_SIZE;
+    cudaError_t e = parts > 1 ? launch_clustered(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), dim3(1, 1, parts), F32Tile<BM_>::SMEM, s,
+                                                 x, w, bias, out, M, N, K, ldx, ldo)
+                              : rb::launch(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), F32Tile<BM_>::SMEM, s, x, w, bias, out, M, N,
+                                           K, ldx, ldo);
+    if (e != cudaSuccess) return (int)e;
+    RB_LAUNCH_CHECK();
+    return RB_OK;
 }
 
 // ---- few rows, 32-bit: one pass over the weight ----------------------------------------------------
@@ -332,6 +570,10 @@ extern "C" int rb_gemm_generic(const void* x, int x_dtype, const void* w, int w_
             if (M <= 8) return launch_rows<8>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, s);
             return launch_rows<16>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, s);
         }
+        // more rows, and enough columns to fill a tile's (the same loads); 32 rows a tile while they hold all of them
+        if (M > 16 && N > 64 && K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0)
+            return M <= 32 ? launch_f32<32>((const float*)x, (const float*)w, (const float*)bias, (float*)out, M, N, K, ldx, ldo, s)
+                           : launch_f32<64>((const float*)x, (const float*)w, (const float*)bias, (float*)out, M, N, K, ldx, ldo, s);
         RB_G(float, float, float);
     }
     if (x_dtype == RB_F32 && w_dtype == RB_BF16 && out_dtype == RB_F32) RB_G(float, bf, float);

@@ -268,6 +268,25 @@ def test_gemm_of_few_32_bit_rows_reads_the_weight_once(M, N, K):
     assert torch.equal(alone[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M,N,K", [(17, 65, 4), (17, 2048, 2048), (32, 130, 36), (33, 129, 2044), (61, 4096, 512), (64, 128, 128),
+                                   (65, 67, 132), (181, 2048, 4096), (226, 1000, 2052), (2049, 66, 260)])
+def test_gemm_of_more_32_bit_rows_splits_k_over_a_cluster(M, N, K):
+    """More than 16 rows of 32-bit operands on 16 bytes: tiles of 32 and 64 rows, k in one part up to eight, ragged rows,
+    columns and k, an output whose rows start off 16 bytes, a strided input; nothing outside the result is written.
+    The bound: K products summed in 32 bits are off by at most K 2^-24 of the sum of their sizes; parts and pairs make it less."""
+    from rocml_b200 import kernels
+    x = rnd((M, K + 4), 1).to(DEV)[:, :K]
+    w = rnd((N, K), 2).to(DEV)
+    bias = rnd((N,), 3).to(DEV)
+    sizes = x.cpu().double().abs() @ w.cpu().double().abs().t() + bias.cpu().double().abs()
+    want = x.cpu().double() @ w.cpu().double().t() + bias.cpu().double()
+    for pad in (0, 1):
+        wide = torch.full((M + 1, N + pad), float("nan"), dtype=torch.float32, device=DEV)
+        kernels.gemm_generic(x, w, wide[:M, :N], bias)
+        assert ((wide[:M, :N].cpu().double() - want).abs() / sizes).max().item() < max(K, 4) * 2.0 ** -24
+        assert torch.isnan(wide[M]).all() and torch.isnan(wide[:M, N:]).all()
+
+
 @pytest.mark.parametrize("M,N,K,S", [(1, 37, 2048, 2), (8, 4096, 4096, 4), (5, 129, 1100, 3), (16, 1001, 12288, 8), (3, 64, 520, 2), (8, 264, 7616, 7)])
 def test_gemm_of_few_32_bit_rows_in_parts_of_k(M, N, K, S):
     """The same product with the sum over K in S parts, each a partial result of its own (the bias in the
