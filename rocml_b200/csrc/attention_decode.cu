@@ -49,6 +49,13 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_cluster(float* local, unsigned rank, float v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(local)), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+}
 __device__ __forceinline__ float ld_cluster(const float* local, unsigned rank) {
     uint32_t remote;
     float v;
@@ -103,74 +110,121 @@ struct Projections {
     float softcap;            // > 0: scores become softcap * tanh(score / softcap)
 };
 
-// One head of 128 values, 4 per lane: the sum of the partial sums, then (what != 2) RMSNorm with `w`
-// and the rotation by the token's angles.  what: 0 query, 1 key, 2 value.
-__device__ __forceinline__ void project_head(const Projections& pj, const float* src, int what, int t, int lane,
-                                             float sumsq_share, float* v, int pos) {
-    v[0] = v[1] = v[2] = v[3] = 0.f;
-    // the norm's weights and the token's angles do not depend on the sums: their loads go out first
+// One head of 128 values by half a warp, so that a block's four warps make eight heads at once: lane i (0 to 15) holds the
+// values 4 i .. 4 i + 3 in v[0..3] and 64 + 4 i .. in v[4..7] (the two members of a whole head's rotation pairs).
+// The sum of the partial sums (in order), then (what != 2) RMSNorm with the weights and the rotation by the token's angles.
+// what: 0 query, 1 key, 2 value, per half; all 32 lanes call it.  row_sums: this lane's share (of 32) of the row's sum of
+// squares, for the rows' 1/RMS; called for after the loads have gone out.
+template <typename RowSums>
+__device__ __forceinline__ void project_head(const Projections& pj, const float* src, int what, int t, int lane, RowSums row_sums,
+                                             float* v, int pos) {
+    const int i = lane & 15;
+    float4 f[2][8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            f[h][j] = j < pj.n_in ? *reinterpret_cast<const float4*>(src + (size_t)j * pj.in_stride + h * 64 + i * 4)
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
     const void* w = what == 0 ? pj.q_norm_w : (what == 1 ? pj.k_norm_w : nullptr);
     const bool rotate = what != 2 && pj.cos_sin != nullptr;
-    float wj[4] = {1.f, 1.f, 1.f, 1.f};
-    float2 cs[4];
+    float wj[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) wj[j] = 1.f;
     if (w != nullptr) {
-        if (pj.w_f32) {
-            const float4 f = *reinterpret_cast<const float4*>(static_cast<const float*>(w) + lane * 4);
-            wj[0] = f.x; wj[1] = f.y; wj[2] = f.z; wj[3] = f.w;
-        } else {
-            const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(w) + lane * 4);
-            const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-            const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-            wj[0] = a.x; wj[1] = a.y; wj[2] = b.x; wj[3] = b.y;
+        load4_any(w, pj.w_f32, i * 4, wj);
+        load4_any(w, pj.w_f32, 64 + i * 4, wj + 4);
+    }
+    // the angles of the first members of this lane's pairs: for a whole head those of its low values
+    const int pair_lanes = pj.rot_dim > 0 ? pj.rot_dim >> 3 : 16;   // groups of four between the two members of a pair
+    float4 cs[2][2];
+    if (rotate) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4* c4 = reinterpret_cast<const float4*>(pj.cos_sin + (size_t)t * (pair_lanes * 4) + ((h * 16 + i) % pair_lanes) * 4);
+            cs[h][0] = c4[0]; cs[h][1] = c4[1];
         }
     }
-    const int pair_lanes = pj.rot_dim > 0 ? pj.rot_dim >> 3 : 16;   // lanes between the two members of a rotation pair
-    if (rotate) {
-        const float4* c4 = reinterpret_cast<const float4*>(pj.cos_sin + (size_t)t * (pair_lanes * 4) + (lane % pair_lanes) * 4);
-        const float4 a = c4[0], b = c4[1];
-        cs[0] = make_float2(a.x, a.y); cs[1] = make_float2(a.z, a.w);
-        cs[2] = make_float2(b.x, b.y); cs[3] = make_float2(b.z, b.w);
-    }
-    for (int s = 0; s < pj.n_in; s += 8) {                  // eight partial sums in flight, added in order
-        float4 f[8];
+    const float share = row_sums();
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            f[j] = s + j < pj.n_in ? *reinterpret_cast<const float4*>(src + (size_t)(s + j) * pj.in_stride)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { v[0] += f[j].x; v[1] += f[j].y; v[2] += f[j].z; v[3] += f[j].w; }
-    }
-    // the rows' 1/RMS, if it is still to be applied: reduced here, after the loads above went out
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) { v[h * 4] += f[h][j].x; v[h * 4 + 1] += f[h][j].y; v[h * 4 + 2] += f[h][j].z; v[h * 4 + 3] += f[h][j].w; }
+#pragma unroll 1
+    for (int s = 8; s < pj.n_in; ++s)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4 g = *reinterpret_cast<const float4*>(src + (size_t)s * pj.in_stride + h * 64 + i * 4);
+            v[h * 4] += g.x; v[h * 4 + 1] += g.y; v[h * 4 + 2] += g.z; v[h * 4 + 3] += g.w;
+        }
+    auto squares = [&] {                                    // of the head, over its 16 lanes
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        return ss;
+    };
     if (pj.row_sumsq != nullptr) {
-        const float rstd = rsqrtf(warp_sum(sumsq_share) * pj.row_inv_width + pj.row_eps);
-        v[0] *= rstd; v[1] *= rstd; v[2] *= rstd; v[3] *= rstd;
-    }
-    if (w != nullptr) {
-        const float ss = warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
-        const float inv = rsqrtf(ss / 128.f + pj.eps);
+        const float rstd = rsqrtf(warp_sum(share) * pj.row_inv_width + pj.row_eps);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = v[j] * inv * wj[j];
+        for (int j = 0; j < 8; ++j) v[j] *= rstd;
     }
-    if (rotate) {
-        // the whole head: dimension i < 64 pairs with i + 64, lanes 0-15 hold x_i, lanes 16-31 the partners
-        const bool turns = lane < 2 * pair_lanes, first = lane < pair_lanes;
-        const int partner = first ? lane + pair_lanes : (turns ? lane - pair_lanes : lane);
+    if (pj.q_norm_w != nullptr) {                           // (both norms exist or neither)
+        const float ss = squares();
+        const float inv = what == 2 ? 1.f : rsqrtf(ss / 128.f + pj.eps);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float other = __shfl_sync(0xffffffffu, v[j], partner);
-            if (turns) v[j] = first ? v[j] * cs[j].x - other * cs[j].y : other * cs[j].y + v[j] * cs[j].x;
+        for (int j = 0; j < 8; ++j) v[j] = v[j] * inv * wj[j];
+    }
+    if (pj.cos_sin != nullptr) {
+        if (pair_lanes == 16) {                             // the whole head: i pairs with i + 64, the same lane's
+            if (rotate) {
+                const float2 c[4] = {make_float2(cs[0][0].x, cs[0][0].y), make_float2(cs[0][0].z, cs[0][0].w),
+                                     make_float2(cs[0][1].x, cs[0][1].y), make_float2(cs[0][1].z, cs[0][1].w)};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float a = v[j], b = v[4 + j];
+                    v[j] = a * c[j].x - b * c[j].y;
+                    v[4 + j] = a * c[j].y + b * c[j].x;
+                }
+            }
+        } else {                                            // its first 8 pair_lanes dimensions: group Q pairs with Q +- pair_lanes
+            float other[8];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int Q = h * 16 + i, P = Q < pair_lanes ? Q + pair_lanes : (Q < 2 * pair_lanes ? Q - pair_lanes : Q);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float lo = __shfl_sync(0xffffffffu, v[j], P & 15, 16), hi = __shfl_sync(0xffffffffu, v[4 + j], P & 15, 16);
+                    other[h * 4 + j] = P < 16 ? lo : hi;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int Q = h * 16 + i;
+                const float2 c[4] = {make_float2(cs[h][0].x, cs[h][0].y), make_float2(cs[h][0].z, cs[h][0].w),
+                                     make_float2(cs[h][1].x, cs[h][1].y), make_float2(cs[h][1].z, cs[h][1].w)};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (rotate && Q < 2 * pair_lanes) {
+                        const float x = v[h * 4 + j], y = other[h * 4 + j];
+                        v[h * 4 + j] = Q < pair_lanes ? x * c[j].x - y * c[j].y : y * c[j].y + x * c[j].x;
+                    }
+            }
         }
     }
-    if (what != 2 && pj.post_norm) {
-        const float ss = warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
-        const float inv = rsqrtf(ss / 128.f + pj.eps);
+    if (pj.post_norm) {
+        const float ss = squares();
+        const float inv = what == 2 ? 1.f : rsqrtf(ss / 128.f + pj.eps);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] *= inv;
+        for (int j = 0; j < 8; ++j) v[j] *= inv;
     }
     if (what == 0 && pj.temp_coef != 0.f) {
         const float f = query_temperature(pos, pj.temp_coef, pj.temp_every);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] *= f;
+        for (int j = 0; j < 8; ++j) v[j] *= f;
     }
 }
 __device__ __forceinline__ uint2 pack4_bf16(const float* v) {
@@ -211,6 +265,13 @@ __device__ __forceinline__ float finished(float A, float L, float M, float sink)
     return L > 0.f ? A / L : 0.f;
 }
 
+// Dynamic shared memory: the query tile and two buffers a warp, or what the merge of the warps' results needs instead.
+template <int HD>
+__host__ __device__ constexpr size_t decode_region() {
+    const size_t kv = (size_t)WARPS * 4 * WK * HD * sizeof(__nv_bfloat16), merge = (size_t)WARPS * ROWS * HD * sizeof(float);
+    return (size_t)ROWS * HD * sizeof(__nv_bfloat16) + (kv > merge ? kv : merge);
+}
+
 template <int HD, bool CL, bool FQ, bool PROP, bool TR>
 __global__ void __launch_bounds__(WARPS * 32, HD <= 128 ? 3 : 1)
 attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
@@ -229,8 +290,13 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);        // [16][HD]
     __nv_bfloat16* KVs = Qs + ROWS * HD;                                    // per warp: K [32][HD], V [32][HD]
     float* s_o = reinterpret_cast<float*>(KVs);                            // reused after the products: [4][16][HD]
-    float* s_part = s_o + WARPS * ROWS * HD;                               // beside it (CL): this block's part [16][HD]
-    __shared__ float s_pm_own[ROWS], s_pl_own[ROWS];                       // its maxima and sums
+    // CL: where the parts of this block's slice of the head size land (TR: pushed by their blocks, [blocks][heads][slice],
+    // beyond everything that is in use before), or this block's own part [16][HD], which the others read
+    constexpr bool PUSH = CL && TR;
+    float* s_part = PUSH ? reinterpret_cast<float*>(smem_raw + decode_region<HD>()) : s_o + WARPS * ROWS * HD;
+    // the parts' (or its own) maxima and sums
+    __shared__ float s_pm[PUSH ? MAX_CLUSTER : 1][PUSH ? 8 : ROWS], s_pl[PUSH ? MAX_CLUSTER : 1][PUSH ? 8 : ROWS];
+    if (PUSH) cluster_arrive_relaxed();                                    // (a block's memory may be written once it runs)
     __shared__ float s_m[WARPS][ROWS], s_l[WARPS][ROWS];
     __shared__ int s_last;
 
@@ -274,7 +340,10 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         b = seq_next;
     }
     const int slot = seq_slot[b];
-    if (slot < 0) return;
+    if (slot < 0) {
+        if (PUSH) cluster_wait_acquire();                   // (the arrival above is always waited for)
+        return;
+    }
     const int t = cu_q[b];
     const int pos = kv_len[b] - 1;
     const int win_lo = span_lo(pos, window);
@@ -309,7 +378,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     // Each warp owns 16 keys of every page and two shared-memory buffers for them: while it
     // works on one page its copies of the next are in flight.
     __nv_bfloat16* KVw = KVs + warp * 4 * WK * HD;          // [2 buffers][K 16 x HD | V 16 x HD]
-    auto issue = [&](int page_idx, int buf) {
+    auto issue = [&](int page_idx, int buf, int without_new) {
         const int j0 = page_idx * CHUNK + warp * WK;
         const int hi = min(pos, (page_idx + 1) * CHUNK - 1);
         const bool any = page_idx <= page_last && j0 <= hi && (j0 + WK - 1 >= win_lo || j0 < keep);
@@ -317,7 +386,8 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
             const int page = table[page_idx];
             const size_t off = (((size_t)(page < 0 ? 0 : page) * n_stored + kh) * RB_PAGE + warp * WK) * HD;
             const size_t off_v = (((size_t)(page < 0 ? 0 : page) * n_stored + vh) * RB_PAGE + warp * WK) * HD;
-            const int valid = page < 0 ? 0 : min(WK, hi - j0 + 1);   // rows past the sequence's end are zero-filled
+            // rows past the sequence's end are zero-filled; with without_new the step's own row is too
+            const int valid = page < 0 ? 0 : min(WK, hi - j0 + 1 - without_new);
             __nv_bfloat16* Kw = KVw + buf * 2 * WK * HD;
             load_tile<HD>(Kw, k_cache + off, HD, WK, valid, lane, 32);
             load_tile<HD>(Kw + WK * HD, v_cache + off_v, HD, WK, valid, lane, 32);
@@ -325,72 +395,108 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         cp_async_commit();
     };
     // Two pages in flight per warp.  A page below the one that holds position `pos` was complete
-    // before this step began, so its copies start at once; the others start after the wait.
+    // before this step began, so its copies start at once.  So do those of the page that holds `pos` when this
+    // block itself makes the new token's key and value (FQ): its other rows are as old, and the new row is put into
+    // shared memory beside them when it is ready.  Any other page waits for the kernels before this one.
     const int new_page = pos / CHUNK;
-    const bool early0 = page_first < new_page, early1 = page_first + 1 < new_page;
-    if (early0) issue(page_first, 0);
-    if (early1) issue(page_first + 1, 1);
+    const bool owner = FQ && pj.write_kv && hc == 0 && page_first <= new_page && new_page <= page_last;
+    const bool patch = owner && new_page < page_first + 2;     // (a block's third page is copied after its row was written)
+    const bool early0 = page_first < new_page || (patch && page_first == new_page);
+    const bool early1 = page_first + 1 < new_page || (patch && page_first + 1 == new_page);
+    const bool idle = CL && page_first > page_last;            // a block of the cluster beyond the sequence
+    if (early0) issue(page_first, 0, page_first == new_page);
+    if (early1) issue(page_first + 1, 1, page_first + 1 == new_page);
+    // a sequence that one block of the cluster covers needs no merge: the others leave
+    const bool alone = CL && parts_hi == 0;
+    if (alone && idle) {
+        if (PUSH) cluster_wait_acquire();
+        return;
+    }
+    if (FQ && !idle)                                           // the tile's rows without a query head
+        for (int r = rows_valid + warp; r < ROWS; r += WARPS)
+            *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(Qs) + r * (HD * 2) + lane * 8) = make_uint2(0u, 0u);
     pdl_wait();
     if (FQ) {
         const float* row = pj.proj + (size_t)t * pj.row_stride;
-        float share = 0.f;                                  // this lane's share of the row's sum of squares
-        if (pj.row_sumsq != nullptr) {
-            for (int g0 = 0; g0 < pj.row_groups; g0 += 256) {   // eight loads a lane in flight, not one after another
-                float x[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int gi = g0 + j * 32 + lane;
-                    x[j] = gi < pj.row_groups ? pj.row_sumsq[(size_t)gi * pj.row_sumsq_ld + t] : 0.f;
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) share += x[j];
-            }
+        // Tasks: this block's query heads, then the new token's key and value (the one block that reads their page), a
+        // half warp each, all their loads in flight together.  This is the longest stretch of a step with few
+        // keys: one round trip to memory, then arithmetic.  (A warp a head took two rounds, the key and value before the
+        // queries, and the page was copied after its row was written: one sequence of 60 keys, 9.6 -> 5.6 us a layer with 16
+        // heads on 8, 9.9 -> 9.0 with 32 on 8, where the next products' weights are being read meanwhile.)
+        const int n_tasks = idle ? 0 : rows_valid + (owner ? 2 : 0);
+        const int owner_page = owner ? table[new_page] : -1;
+        const int sub = lane & 15;
+        if (patch) {                                            // the copies that the new row is put into have landed (long ago)
+            cp_async_wait<0>();
+            __syncthreads();
         }
-        // The new token's key and value first, by the one block that reads their page (its last two
-        // warps), so that the page's copies are on their way while the query heads are made.
-        const bool owner = pj.write_kv && hc == 0 && page_first <= new_page && new_page <= page_last;
-        if (owner) {
-            if (warp >= WARPS - 2) {
-                const int page = table[new_page];
-                if (page >= 0) {
-                    float v[4];
-                    const bool is_k = warp == WARPS - 2;
-                    const int head = is_k ? nq + kvh : nq + nkv + kvh;
-                    project_head(pj, row + (size_t)head * HD + lane * 4, is_k ? 1 : 2, t, lane, share, v, pos);
-                    if (!is_k && (pj.v_keep || pj.v_first)) {
-                        const size_t vrow = ((size_t)t * nkv + kvh) * HD + lane * 4;
-                        if (pj.v_keep) *reinterpret_cast<float4*>(pj.v_keep + vrow) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll 1
+        for (int first = warp; first < n_tasks; first += 2 * WARPS) {
+            const int mine = first + (lane >> 4) * WARPS;
+            const bool real = mine < n_tasks;
+            const int task = real ? mine : first;               // (the second half repeats the first's and drops the result)
+            const int kind = task < rows_valid ? 0 : task - rows_valid + 1;
+            const int head = kind == 0 ? h0 + task : (kind == 1 ? nq + kvh : nq + nkv + kvh);
+            float v[8];
+            project_head(pj, row + (size_t)head * HD, kind, t, lane, [&] {
+                float share = 0.f;                              // this lane's share of the row's sum of squares
+                if (pj.row_sumsq != nullptr) {
+                    for (int g0 = 0; g0 < pj.row_groups; g0 += 256) {   // eight loads a lane in flight, not one after another
+                        float x[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int gi = g0 + j * 32 + lane;
+                            x[j] = gi < pj.row_groups ? pj.row_sumsq[(size_t)gi * pj.row_sumsq_ld + t] : 0.f;
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) share += x[j];
+                    }
+                }
+                return share;
+            }, v, pos);
+            if (real && (kind == 0 || owner_page >= 0)) {
+                if (kind == 2 && (pj.v_keep || pj.v_first)) {
+                    const size_t vrow = ((size_t)t * nkv + kvh) * HD + sub * 4;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float* x = v + h * 4;
+                        if (pj.v_keep) *reinterpret_cast<float4*>(pj.v_keep + vrow + h * 64) = make_float4(x[0], x[1], x[2], x[3]);
                         if (pj.v_first) {
                             const float lam = pj.v_lambda[0];
-                            const float4 f = *reinterpret_cast<const float4*>(pj.v_first + vrow);
-                            v[0] = (1.f - lam) * v[0] + lam * f.x; v[1] = (1.f - lam) * v[1] + lam * f.y;
-                            v[2] = (1.f - lam) * v[2] + lam * f.z; v[3] = (1.f - lam) * v[3] + lam * f.w;
+                            const float4 f = *reinterpret_cast<const float4*>(pj.v_first + vrow + h * 64);
+                            x[0] = (1.f - lam) * x[0] + lam * f.x; x[1] = (1.f - lam) * x[1] + lam * f.y;
+                            x[2] = (1.f - lam) * x[2] + lam * f.z; x[3] = (1.f - lam) * x[3] + lam * f.w;
                         }
                     }
-                    __nv_bfloat16* dst = (is_k ? pj.k_out : pj.v_out) +
-                                         (((size_t)page * nkv + kvh) * RB_PAGE + (pos % RB_PAGE)) * HD;
-                    *reinterpret_cast<uint2*>(dst + lane * 4) = pack4_bf16(v);
-                    __threadfence_block();
+                }
+                const uint2 packed[2] = {pack4_bf16(v), pack4_bf16(v + 4)};
+                // a row of a swizzled tile: queries to their own, a new key or value into the copy of its page ...
+                const int r = kind == 0 ? task : pos % WK;
+                __nv_bfloat16* tile = kind == 0 ? Qs : KVs + ((pos % CHUNK) / WK * 4 + (new_page - page_first) * 2 + (kind - 1)) * WK * HD;
+                if (kind == 0 || patch) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)                 // 8 values per 16-byte chunk, 4 per lane
+                        *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(tile) + r * (HD * 2) +
+                                                  (((h * 8 + (sub >> 1)) ^ (r & 7)) << 4) + (sub & 1) * 8) = packed[h];
+                }
+                if (kind != 0) {                                // ... and into the page itself
+                    __nv_bfloat16* dst = (kind == 1 ? pj.k_out : pj.v_out) +
+                                         (((size_t)owner_page * nkv + kvh) * RB_PAGE + (pos % RB_PAGE)) * HD;
+                    *reinterpret_cast<uint2*>(dst + sub * 4) = packed[0];
+                    *reinterpret_cast<uint2*>(dst + 64 + sub * 4) = packed[1];
+                    if (!patch) __threadfence_block();
                 }
             }
-            __syncthreads();                                // before the page of the new token is copied
+            __syncwarp();
         }
-        if (!early0) issue(page_first, 0);
-        if (!early1) issue(page_first + 1, 1);              // commits an empty group beyond page_last
-        for (int r = warp; r < ROWS; r += WARPS) {          // the query heads of this block
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            if (r < rows_valid) project_head(pj, row + (size_t)(h0 + r) * HD + lane * 4, 0, t, lane, share, v, pos);
-            const int chunk = lane >> 1;                    // 8 values per 16-byte chunk, 4 per lane
-            *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(Qs) + r * (HD * 2) + ((chunk ^ (r & 7)) << 4) +
-                                      (lane & 1) * 8) = pack4_bf16(v);
-        }
+        // (a page that is neither early nor patched is copied in the loop below, after the barrier that follows)
+        if (!early0) issue(page_first, 0, 0);
+        if (!early1) issue(page_first + 1, 1, 0);           // commits an empty group beyond page_last
     } else {
         load_tile<HD>(Qs, q + (size_t)t * q_stride + (size_t)q_h0 * HD, HD, ROWS, rows_valid, threadIdx.x, WARPS * 32);
-    }
-    if (!FQ) {
         cp_async_commit();                                  // a group of its own: the wait below covers committed groups only
-        if (!early0) issue(page_first, 0);
-        if (!early1) issue(page_first + 1, 1);              // commits an empty group beyond page_last
+        if (!early0) issue(page_first, 0, 0);
+        if (!early1) issue(page_first + 1, 1, 0);           // commits an empty group beyond page_last
     }
     cp_async_wait<0>();
     __syncthreads();                                        // the query heads are in place for every warp
@@ -576,7 +682,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         }
         attend_page(pg, buf);
         __syncwarp();                                       // the buffer is free again
-        issue(pg + 2, buf);
+        issue(pg + 2, buf, 0);
     }
     cp_async_wait<0>();
 #pragma unroll
@@ -619,6 +725,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     }
     __syncthreads();
     const size_t row0 = (size_t)b * nq;                   // the work space is indexed by sequence, whatever cu_q says
+    if (PUSH) cluster_wait_acquire();                     // every block of the cluster runs by now
     for (int idx = threadIdx.x; idx < rows_valid * HD; idx += WARPS * 32) {
         const int r = idx / HD, d = idx % HD;
         float M = NEG_BIG;
@@ -632,10 +739,18 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
             A = fmaf(wt, s_o[((size_t)w * ROWS + r) * HD + d], A);
         }
         const int head = h0 + r;
-        if (CL) {
-            s_part[r * HD + d] = A;
-            if (d == 0) { s_pm_own[r] = M; s_pl_own[r] = L; }
-        } else if (PROP ? parts_hi > 0 : n_chunks > 1) {
+        if (CL && !alone) {
+            if (PUSH) {
+                // to the block that owns d's slice; every block needs every part's maximum and sum
+                const int n = (int)gridDim.x;
+                const int to = ((d + 1) * n - 1) / HD, d_lo = to * HD / n, width = (to + 1) * HD / n - d_lo;
+                st_cluster(s_part + ((size_t)c * rows_valid + r) * width + (d - d_lo), (unsigned)to, A);
+                if (d < n) { st_cluster(&s_pm[c][r], (unsigned)d, M); st_cluster(&s_pl[c][r], (unsigned)d, L); }
+            } else {
+                s_part[r * HD + d] = A;
+                if (d == 0) { s_pm[0][r] = M; s_pl[0][r] = L; }
+            }
+        } else if (!CL && (PROP ? parts_hi > 0 : n_chunks > 1)) {
             const size_t pidx = (row0 + head) * n_chunks + c;
             part_acc[pidx * HD + d] = A;
             if (d == 0) { part_ml[pidx * 2] = M; part_ml[pidx * 2 + 1] = L; }
@@ -646,25 +761,25 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         }
     }
     if (CL) {
-        // The blocks of this (sequence, head group) are one cluster: each keeps its partial result in
-        // its own shared memory, and after a cluster barrier each block merges one slice of the head
-        // size, reading every block's part (in ascending order) through distributed shared memory.
-        // Nothing goes through global memory, no counter is needed.
+        if (alone) return;
+        // The blocks of this (sequence, head group) are one cluster and each merges one slice of the head size, from every
+        // block's part in ascending order.  Groups of up to 8 heads: the parts have been pushed into their owner's shared
+        // memory, so one cluster barrier is all (before: a barrier, remote reads, a second barrier).  Wider groups, whose parts have no room beside the pages, read one
+        // another's.  Nothing goes through global memory, no counter is needed.
         cluster_sync_all();
         const int n = (int)gridDim.x;                        // = the cluster's size, at most MAX_CLUSTER
         const int d_lo = c * HD / n, d_hi = (c + 1) * HD / n;
         const int width = d_hi - d_lo;
         for (int idx = threadIdx.x; idx < rows_valid * width; idx += WARPS * 32) {
             const int r = idx / width, d = d_lo + idx % width;
-            // every block's maximum, sum and value for this (row, dimension): all remote reads go out
-            // together, one round trip
+            // every block's maximum, sum and value for this (row, dimension): all reads go out together
             float pm[MAX_CLUSTER], pl[MAX_CLUSTER], pa[MAX_CLUSTER];
 #pragma unroll
             for (int i = 0; i < MAX_CLUSTER; ++i) {
                 if (i < n) {
-                    pm[i] = ld_cluster(&s_pm_own[r], (unsigned)i);
-                    pl[i] = ld_cluster(&s_pl_own[r], (unsigned)i);
-                    pa[i] = ld_cluster(&s_part[r * HD + d], (unsigned)i);
+                    pm[i] = PUSH ? s_pm[PUSH ? i : 0][r] : ld_cluster(&s_pm[0][r], (unsigned)i);
+                    pl[i] = PUSH ? s_pl[PUSH ? i : 0][r] : ld_cluster(&s_pl[0][r], (unsigned)i);
+                    pa[i] = PUSH ? s_part[((size_t)i * rows_valid + r) * width + (d - d_lo)] : ld_cluster(&s_part[r * HD + d], (unsigned)i);
                 }
             }
             float MM = NEG_BIG;
@@ -684,6 +799,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
             if (pj.gate.raw) y *= gate_factor(pj.gate, (size_t)t, (size_t)(h0 + r) * HD + d);
             out[(size_t)t * o_stride + (size_t)(h0 + r) * HD + d] = __float2bfloat16_rn(y);
         }
+        if (PUSH) return;                                    // nothing of this block is read any more
         cluster_sync_all();                                  // nobody leaves while its part may still be read
         return;
     }
@@ -792,14 +908,14 @@ int launch(const void* q, int q_stride, const void* k_cache, const void* v_cache
     if (keep < 0 || (keep > 0 && (proportional || window < 0))) return RB_ERR_BAD_SIZE;
     dim3 grid(n_chunks, nkv * ((g + ROWS - 1) / ROWS), proportional ? 1 : B);
     if (grid.y > 65535 || grid.z > 65535) return RB_ERR_BAD_SIZE;
-    const size_t kv_bytes = (size_t)WARPS * 4 * WK * HD * sizeof(__nv_bfloat16);   // two buffers per warp
-    const size_t merge_bytes = (size_t)WARPS * ROWS * HD * sizeof(float);
-    const size_t smem = (size_t)ROWS * HD * sizeof(__nv_bfloat16) + (kv_bytes > merge_bytes ? kv_bytes : merge_bytes);
-    const size_t region = kv_bytes > merge_bytes ? kv_bytes : merge_bytes;
-    const int rows_max = g < ROWS ? g : ROWS;
-    if ((size_t)n_chunks * rows_max * 2 * sizeof(float) > region) return RB_ERR_BAD_SIZE;  // the merge's work space
+    const size_t region = decode_region<HD>() - (size_t)ROWS * HD * sizeof(__nv_bfloat16);
     // up to 16 blocks per (sequence, head group): one cluster, merged through shared memory
     const bool clustered = !proportional && n_chunks > 1 && n_chunks <= MAX_CLUSTER && cluster_enabled();
+    // groups of up to 8 heads in clusters: room for the pushed parts, blocks x 8 rows x the widest slice (three such blocks
+    // still fit a multiprocessor)
+    const size_t smem = decode_region<HD>() + (clustered && g <= 8 ? (size_t)8 * (HD + MAX_CLUSTER - 1) * sizeof(float) : 0);
+    const int rows_max = g < ROWS ? g : ROWS;
+    if ((size_t)n_chunks * rows_max * 2 * sizeof(float) > region) return RB_ERR_BAD_SIZE;  // the merge's work space
     const bool fused = pj.proj != nullptr;
     if (fused && HD != 128) return RB_ERR_BAD_SIZE;
     // More than 16 query heads a key/value head: several blocks read the page of the new token, and only

@@ -175,6 +175,10 @@ __device__ __forceinline__ void load4(const __nv_bfloat16* p, float* x) {
     x[0] = __uint_as_float(raw.x << 16); x[1] = __uint_as_float(raw.x & 0xFFFF0000u);
     x[2] = __uint_as_float(raw.y << 16); x[3] = __uint_as_float(raw.y & 0xFFFF0000u);
 }
+__device__ __forceinline__ void load4_any(const void* p, int f32, int i, float* x) {      // four values from element i of either type
+    if (f32) load4(static_cast<const float*>(p) + i, x);
+    else load4(static_cast<const __nv_bfloat16*>(p) + i, x);
+}
 __device__ __forceinline__ void store4(float* p, const float* x) {
     *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
 }

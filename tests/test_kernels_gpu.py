@@ -869,6 +869,18 @@ def test_attention_decode_takes_the_projections_itself(lens, nq, nkv, window, S,
             assert (outs[1][b, h * hd:(h + 1) * hd].double() - want).abs().max().item() < 2e-2, (b, h)
 
 
+@pytest.mark.parametrize("nq,nkv,S", [(2, 1, 3), (8, 2, 9), (16, 2, 2), (20, 2, 1)])
+@pytest.mark.parametrize("lens,window,grid", [
+    ([1, 2, 16, 17, 63, 64], None, (1, 1)),             # one block a sequence
+    ([1, 64, 65, 128, 129, 192, 193], None, (1, 1)),    # the new row first, last and alone in its page; clusters with blocks beyond the sequence
+    ([1, 65, 128, 129, 193, 257], None, (2, 1)),        # in the first or the second page of its block
+    ([1, 65, 129, 193, 256], None, (4, 1)),             # ... or in a later one; one block a sequence
+    ([65, 130, 200, 961], 70, (1, 1)),                  # a window, clusters of 16
+])
+def test_attention_decode_puts_the_new_row_beside_its_page(lens, window, grid, nq, nkv, S):
+    test_attention_decode_takes_the_projections_itself(lens, nq, nkv, window, S, True, True, grid, 1e-6)
+
+
 def test_attention_decode_leaves_wide_groups_to_the_two_kernels():
     """More than 16 query heads a key/value head: several blocks would read the new token's page while
     one of them writes it, so the kernel that takes the projections declines (the caller then writes
