@@ -82,6 +82,7 @@ struct Params {
     float norm_eps;
     const float2* cos_sin;        // [tokens][64] (cos, sin), or null
     int nq, nkv;
+    int tma_out;                  // pair kernel: results leave through map_o
     // persistent kernel, grouped: the rows of A are sorted by group, every group starting at a multiple of 128
     // rows; row tile i is multiplied with the weight of group tile_group[i] (rows group * group_rows .. of the
     // stacked B operand), a tile of group -1 is skipped.  b_rows is then one group's feature count.
@@ -705,26 +706,41 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
 // the single-CTA kernel (128 x 256 tiles read 96 bytes per clock of a 128-byte-per-clock port).
 // Persistent, two accumulators, as the single-CTA kernel above.  Barriers: full[] is counted on the
 // leader (both CTAs' TMA loads report there), empty[] and acc_full[] exist in both CTAs and are
-// signalled by multicast commits, acc_empty[] lives in the leader and collects the 8 epilogue warps
+// signalled by multicast commits, acc_empty[] lives in the leader and collects the 16 epilogue warps
 // of the pair.  No TMA multicast is used anywhere.
 constexpr int PAIR_BN = 256;
 constexpr int PAIR_STAGE = 2 * BM * BK * 2;       // A 128 x 64 + B half 128 x 64, bf16: 32 KB
 constexpr int PAIR_STAGES = 6;
-constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE + 1024 + 256;
+constexpr int PAIR_WARPS = 8;                     // epilogue warps: four a half of the tile's columns
+constexpr int PAIR_THREADS = (2 + PAIR_WARPS) * 32;
+constexpr int PAIR_OUT = PAIR_WARPS * 4096;       // a 4 KB piece of 32 rows x 128 bytes for each
+constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE + PAIR_OUT + 1024 /*norm weights*/ + 1024 /*align slack*/ + 256;
 
 // EPI: 0 plain, 4 through an activation of its own (act_kind 0 gelu with erf, 1 gelu in its tanh form, 2 silu), 3 added into `out` (the float32 residual stream) instead of written, 1 SiLU(gate) * up (rows
 // of the weight interleaved by 16), 2 a prompt's q | k | v projection
 // with heads of 128: a tile's 256 columns are two whole heads and an epilogue thread owns a token, so
 // the per-head RMSNorm and the rotation (pairs i, i + 64) are done on the accumulator itself, and
 // the queries go to their own tensor, keys and values straight into their cache pages.
+//
+// How results leave (p.tma_out; EPI 2 always): an epilogue thread owns a row, so storing from its registers touches 32 lines an
+// instruction, and for K of 2,000 to 4,000 that took longer than a tile's products (added into the stream: 43 us for
+// 4,096 x 2,048 x 2,048, 85 for K = 6,144).  So a warp writes pieces of 32 rows x 128 bytes into shared memory (swizzled)
+// and the copy engine stores them, or adds them to the stream in the L2 cache, where the stream need
+// not be read into the multiprocessor at all.  Rows that the copy engine cannot address (off 16 bytes) go the old way.
+// Eight warps share a tile, four a half of its columns: with four, the gate's arithmetic of a tile took as long as the
+// products of K = 2,048, and a launch of one or two tiles a block waited for all of the last one.
+// Microseconds before and after at 4,096 tokens of a 2,048 wide model (4,096 wide, 2,048 tokens): q | k | v with rotation 96 -> 65
+// (98 -> 78), added K = 2,048 43 -> 33 (K = 4,096: 61 -> 50), K = 6,144 86 -> 76 (K = 12,288: 158 -> 139), gated 150 -> 137 (286 -> 261).
 template <typename OT, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                         OT* __restrict__ out, const Params p) {
+                         const __grid_constant__ CUtensorMap map_o, OT* __restrict__ out, const Params p) {
     constexpr int BN = PAIR_BN, S = PAIR_STAGES, A_BYTES = BM * BK * 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = (uint64_t*)(smem + S * PAIR_STAGE);
+    uint8_t* pieces = smem + S * PAIR_STAGE;
+    float* s_norm = (float*)(pieces + PAIR_OUT);          // EPI 2: the query norm's and the key norm's weights
+    uint64_t* full = (uint64_t*)(pieces + PAIR_OUT + 1024);
     uint64_t* empty = full + S;
     uint64_t* acc_full = empty + S;      // [2]
     uint64_t* acc_empty = acc_full + 2;  // [2], used in the leader
@@ -741,13 +757,20 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * PAIR_WARPS); }
         *abort_flag = 0;
         fence_barrier_init();
     }
     if (warp == 1) {
         tmem_alloc_pair(tmem_slot, 512);
         tmem_relinquish_pair();
+    }
+    if (EPI == 2 && warp >= 2 && warp < 6 && p.q_norm_w != nullptr) {
+        const int i = threadIdx.x - 64;
+        for (int j = 0; j < 2; ++j) {
+            const void* w = j == 0 ? p.q_norm_w : p.k_norm_w;
+            s_norm[j * 128 + i] = p.norm_w_f32 ? static_cast<const float*>(w)[i] : __bfloat162float(static_cast<const __nv_bfloat16*>(w)[i]);
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -760,21 +783,38 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (lane == 0) {
             tma_prefetch_desc(&map_a);
             tma_prefetch_desc(&map_b);
+            // the weight does not depend on the kernel before this one: the ring's first tiles of it are sent for at once
+            const long long mine = pair < n_total ? (long long)((n_total - 1 - pair) / n_pairs + 1) * n_kb : 0;
+            const int pre = mine < S ? (int)mine : S;
+            auto a_row = [&](int tile) { return (tile % m_pairs) * 2 * BM + (int)rank * BM; };
+            auto b_row = [&](int tile) { return (tile / m_pairs) * BN + (int)rank * (BN / 2); };
+            for (int j = 0; j < pre; ++j) {
+                const uint32_t bar = smem_u32(&full[j]) & PEER_BIT_MASK;       // the leader's barrier
+                if (rank == 0) mbar_arrive_expect_tx(&full[j], 2 * PAIR_STAGE);   // both CTAs' bytes
+                tma_load_2d_pair(smem + j * PAIR_STAGE + A_BYTES, &map_b, (j % n_kb) * BK, b_row(pair + (j / n_kb) * n_pairs), bar);
+            }
             rb::pdl_wait();
-            long long it = 0;
+            for (int j = 0; j < pre; ++j)
+                tma_load_2d_pair(smem + j * PAIR_STAGE, &map_a, (j % n_kb) * BK, a_row(pair + (j / n_kb) * n_pairs),
+                                 smem_u32(&full[j]) & PEER_BIT_MASK);
             bool ok = true;
+            int s = 0, skip = pre;           // the ring's stage, and how many K blocks are on their way already
+            uint32_t par = 1;
             for (int tile = pair; tile < n_total && ok; tile += n_pairs) {
-                const int a0 = (tile % m_pairs) * 2 * BM + (int)rank * BM;
-                const int b0 = (tile / m_pairs) * BN + (int)rank * (BN / 2);
-                for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                    const int s = (int)(it % S);
-                    ok = mbar_wait(&empty[s], (uint32_t)(((it / S) & 1) ^ 1), p.wait_cycles);
-                    if (!ok) break;
-                    uint8_t* sa = smem + s * PAIR_STAGE;
-                    const uint32_t bar = smem_u32(&full[s]) & PEER_BIT_MASK;   // the leader's barrier
-                    if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * PAIR_STAGE);   // both CTAs' bytes
-                    tma_load_2d_pair(sa + A_BYTES, &map_b, kb * BK, b0, bar);
-                    tma_load_2d_pair(sa, &map_a, kb * BK, a0, bar);
+                const int a0 = a_row(tile), b0 = b_row(tile);
+                for (int kb = 0; kb < n_kb; ++kb) {
+                    if (skip > 0) {
+                        --skip;
+                    } else {
+                        ok = mbar_wait(&empty[s], par, p.wait_cycles);
+                        if (!ok) break;
+                        uint8_t* sa = smem + s * PAIR_STAGE;
+                        const uint32_t bar = smem_u32(&full[s]) & PEER_BIT_MASK;
+                        if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * PAIR_STAGE);
+                        tma_load_2d_pair(sa + A_BYTES, &map_b, kb * BK, b0, bar);
+                        tma_load_2d_pair(sa, &map_a, kb * BK, a0, bar);
+                    }
+                    if (++s == S) { s = 0; par ^= 1u; }
                 }
             }
             if (!ok) {
@@ -785,8 +825,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
             constexpr uint32_t idesc = idesc_bf16_f32(2 * BM, BN);
-            long long it = 0;
-            int local = 0;
+            int local = 0, s = 0;
+            uint32_t par = 0;
             bool ok = true;
             for (int tile = pair; tile < n_total && ok; tile += n_pairs, ++local) {
                 const int acc = local & 1;
@@ -795,9 +835,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + acc * BN;
-                for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                    const int s = (int)(it % S);
-                    ok = mbar_wait(&full[s], (uint32_t)((it / S) & 1), p.wait_cycles);
+                for (int kb = 0; kb < n_kb; ++kb) {
+                    ok = mbar_wait(&full[s], par, p.wait_cycles);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem + s * PAIR_STAGE);
@@ -807,6 +846,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     for (int k = 0; k < BK / UMMA_K; ++k)
                         mma_bf16_pair(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     mma_commit_pair(&empty[s]);          // frees the stage in both CTAs
+                    if (++s == S) { s = 0; par ^= 1u; }
                 }
                 if (!ok) break;
                 mma_commit_pair(&acc_full[acc]);         // wakes both CTAs' epilogue warps
@@ -819,7 +859,33 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
         }
     } else {
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, half = (warp - 2) >> 2;      // its tensor memory lanes, its columns of the tile
+        // this warp's piece: row r of 128 bytes at r * 128, its 16-byte groups swizzled as the copy engine has them
+        uint8_t* const piece = pieces + (warp - 2) * 4096;
+        auto group = [&](int row, int g16) { return reinterpret_cast<uint4*>(piece + row * 128 + ((g16 ^ (row & 7)) << 4)); };
+        auto piece_free = [&] {                          // the copy before has read its shared memory
+            if (lane == 0) bulk_wait_read<0>();
+            __syncwarp();
+        };
+        auto piece_done = [&](int col, int row) {
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                if (EPI == 3) tma_add_2d(&map_o, piece, col, row);
+                else tma_store_2d(&map_o, piece, col, row);
+                bulk_commit();
+            }
+        };
+        auto put8 = [&](int g16, const float* v) {       // eight values as one 16-byte group of bfloat16
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            *group(lane, g16) = make_uint4(w[0], w[1], w[2], w[3]);
+        };
+        if (EPI == 3) rb::pdl_wait();   // these threads add to what earlier kernels wrote: returns at once by the first tile's end
         int local = 0;
         for (int tile = pair; tile < n_total; tile += n_pairs, ++local) {
             const int acc = local & 1;
@@ -830,176 +896,190 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 if (!ok && lane == 0) atomicExch(p.status, RB_ERR_TIMEOUT);
                 break;
             }
-            const int a0 = (tile % m_pairs) * 2 * BM + (int)rank * BM, b0 = (tile / m_pairs) * BN;
+            const int a0 = (tile % m_pairs) * 2 * BM + (int)rank * BM, b0 = (tile / m_pairs) * BN + half * 128;
             const int ar = a0 + quarter * 32 + lane;
+            const int row0 = a0 + quarter * 32;          // this warp's first row
             const bool add_bias = p.bias != nullptr;
-            const uint32_t lane_addr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
-            const bool vec_ok = (((uintptr_t)out | ((uintptr_t)p.ldo * sizeof(OT))) & 15) == 0;
+            const uint32_t lane_addr = tmem_base + acc * BN + half * 128 + ((uint32_t)(quarter * 32) << 16);
             OT* row = out + (size_t)(ar < p.a_rows ? ar : 0) * p.ldo;
+            // bias and activation of a group of columns from f0
+            auto dress = [&](float* v, int n, int f0) {
+                if (add_bias) {
+#pragma unroll
+                    for (int i = 0; i < n; ++i) v[i] += (f0 + i < p.b_rows) ? p.bias[f0 + i] : 0.f;
+                }
+                if (EPI == 4) {
+                    if (p.act_kind == 0) {
+#pragma unroll
+                        for (int i = 0; i < n; ++i) v[i] = rb::gelu_erf(v[i]);
+                    } else if (p.act_kind == 1) {
+#pragma unroll
+                        for (int i = 0; i < n; ++i) v[i] = rb::gelu_tanh(v[i]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < n; ++i) v[i] = rb::silu(v[i]);
+                    }
+                }
+            };
+            // the gated value of 16 gate columns and the 16 up columns after them
+            auto gated = [&](float* g, float* u, int f0) {
+                if (add_bias) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) { g[i] += p.bias[f0 + i]; u[i] += p.bias[f0 + 16 + i]; }
+                }
+                if (p.act_kind == 2) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) g[i] = rb::gelu_tanh(g[i]) * u[i];
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) g[i] = g[i] / (1.f + expf(-g[i])) * u[i];
+                }
+            };
             if (EPI == 2) {
                 rb::pdl_wait();   // these threads read what an earlier kernel wrote (the angles' table): returns at once by now
-                int slot = -1, pos = 0, page = -2;         // page -2: not looked up yet
+                int slot = -1, pos = 0, page = -1;
                 if (ar < p.a_rows) { slot = p.slot_of_token[ar]; pos = p.positions[ar]; }
-#pragma unroll 1
-                for (int hh = 0; hh < BN / 128; ++hh) {
-                    const int col0 = b0 + hh * 128;
-                    if (col0 >= p.b_rows) break;
-                    const int head = col0 >> 7;
-                    const int kind = head < p.nq ? 0 : (head < p.nq + p.nkv ? 1 : 2);
-                    __nv_bfloat16* dst = nullptr;
-                    if (slot >= 0) {
-                        if (kind == 0) {
-                            dst = p.q_out + (size_t)ar * p.q_ld + (size_t)head * 128;
-                        } else {
-                            if (page == -2) page = p.block_table[(size_t)slot * p.max_pages + (pos / RB_PAGE)];
-                            const int hk = kind == 1 ? head - p.nq : head - p.nq - p.nkv;
-                            if (page >= 0)
-                                dst = (kind == 1 ? p.k_cache : p.v_cache) +
-                                      (((size_t)page * p.nkv + hk) * RB_PAGE + (pos % RB_PAGE)) * 128;
-                        }
+                const int head = b0 >> 7;                // this half of the tile is one head
+                const int kind = head < p.nq ? 0 : (head < p.nq + p.nkv ? 1 : 2);
+                __nv_bfloat16* dst = nullptr;            // this token's row of the head
+                if (slot >= 0 && b0 < p.b_rows) {
+                    if (kind == 0) {
+                        dst = p.q_out + (size_t)ar * p.q_ld + (size_t)head * 128;
+                    } else {
+                        const int page = p.block_table[(size_t)slot * p.max_pages + (pos / RB_PAGE)];
+                        const int hk = kind == 1 ? head - p.nq : head - p.nq - p.nkv;
+                        if (page >= 0)
+                            dst = (kind == 1 ? p.k_cache : p.v_cache) + (((size_t)page * p.nkv + hk) * RB_PAGE + (pos % RB_PAGE)) * 128;
                     }
-                    const uint32_t hbase = lane_addr + hh * 128;
-                    const void* w = kind == 0 ? p.q_norm_w : (kind == 1 ? p.k_norm_w : nullptr);
-                    float inv = 1.f;
-                    if (w != nullptr) {
-                        float ss = 0.f;
-#pragma unroll 1
-                        for (int c = 0; c < 8; ++c) {
-                            float v[16];
-                            tmem_ld16(hbase + c * 16, v);
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                const float x = v[i] + (add_bias ? p.bias[col0 + c * 16 + i] : 0.f);
-                                ss += x * x;
-                            }
-                        }
-                        inv = rsqrtf(ss / 128.f + p.norm_eps);
-                    }
-                    const bool rotate = kind != 2 && p.cos_sin != nullptr;
+                }
+                const float2* angles = p.cos_sin != nullptr ? p.cos_sin + (size_t)(ar < p.a_rows ? ar : 0) * 64 : nullptr;
+                const bool angles16 = ((uintptr_t)p.cos_sin & 15) == 0;
+                auto two_angles = [&](int i) {           // pairs 2 i and 2 i + 1
+                    if (angles16) return reinterpret_cast<const float4*>(angles)[i];
+                    const float2 a = angles[2 * i], b = angles[2 * i + 1];
+                    return make_float4(a.x, a.y, b.x, b.y);
+                };
+                const bool normed = kind != 2 && p.q_norm_w != nullptr;
+                const bool rotate = kind != 2 && angles != nullptr;
+                float inv = 1.f;
+                if (normed && b0 < p.b_rows) {
+                    float ss = 0.f;
 #pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
+                        float v[32];
+                        tmem_ld32(lane_addr + c * 32, v);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            const float x = v[i] + (add_bias ? p.bias[b0 + c * 32 + i] : 0.f);
+                            ss += x * x;
+                        }
+                    }
+                    inv = rsqrtf(ss / 128.f + p.norm_eps);
+                }
+                const float* wn = s_norm + kind * 128;
+                if (b0 < p.b_rows) {
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        float4 cs[8];                    // (cos, sin) of 16 pairs
+                        if (rotate) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) cs[i] = two_angles(c * 8 + i);
+                        }
                         float lo[16], hi[16];
-                        tmem_ld16(hbase + c * 16, lo);
-                        tmem_ld16(hbase + (c + 4) * 16, hi);
+                        tmem_ld16(lane_addr + c * 16, lo);
+                        tmem_ld16(lane_addr + (c + 4) * 16, hi);
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             const int d = c * 16 + i;
                             float a = lo[i], b = hi[i];
-                            if (add_bias) { a += p.bias[col0 + d]; b += p.bias[col0 + 64 + d]; }
-                            if (w != nullptr) {
-                                const float wa = p.norm_w_f32 ? static_cast<const float*>(w)[d]
-                                                              : __bfloat162float(static_cast<const __nv_bfloat16*>(w)[d]);
-                                const float wb = p.norm_w_f32 ? static_cast<const float*>(w)[64 + d]
-                                                              : __bfloat162float(static_cast<const __nv_bfloat16*>(w)[64 + d]);
-                                a = a * inv * wa;
-                                b = b * inv * wb;
-                            }
+                            if (add_bias) { a += p.bias[b0 + d]; b += p.bias[b0 + 64 + d]; }
+                            if (normed) { a = a * inv * wn[d]; b = b * inv * wn[64 + d]; }
                             if (rotate) {
-                                const float2 cs = p.cos_sin[(size_t)(ar < p.a_rows ? ar : 0) * 64 + d];
-                                const float ra = a * cs.x - b * cs.y, rb2 = a * cs.y + b * cs.x;
+                                const float4 f = cs[i >> 1];
+                                const float cx = i & 1 ? f.z : f.x, sx = i & 1 ? f.w : f.y;
+                                const float ra = a * cx - b * sx, rb2 = a * sx + b * cx;
                                 a = ra; b = rb2;
                             }
                             lo[i] = a; hi[i] = b;
                         }
-                        if (dst != nullptr) {
-                            store16(dst + c * 16, lo);
-                            store16(dst + 64 + c * 16, hi);
+                        // the piece holds 32 values of the head's first half (groups 0 to 3) and the 32 they pair with
+                        put8((c & 1) * 2, lo); put8((c & 1) * 2 + 1, lo + 8);
+                        put8(4 + (c & 1) * 2, hi); put8(5 + (c & 1) * 2, hi + 8);
+                        if (c & 1) {
+                            // eight lanes write a row's two stretches of 64 bytes
+                            __syncwarp();
+                            const unsigned long long mine = (unsigned long long)dst;
+                            const int g16 = lane & 7;
+                            const int at = (c >> 1) * 64 + (g16 & 3) * 16 + (g16 >> 2) * 128;      // bytes into the row
+#pragma unroll
+                            for (int r0 = 0; r0 < 32; r0 += 4) {
+                                const int r = r0 + (lane >> 3);
+                                char* to = (char*)__shfl_sync(0xffffffffu, mine, r);
+                                if (to != nullptr) *reinterpret_cast<uint4*>(to + at) = *group(r, g16);
+                            }
+                            __syncwarp();
                         }
                     }
                 }
+            } else if (p.tma_out) {
+                constexpr int COLS = EPI == 1 ? 128 : 128 / (int)sizeof(OT);      // columns of the product that fill a piece
+#pragma unroll 1
+                for (int c = 0; c < BN / 2; c += COLS) {
+                    if (b0 + c >= p.b_rows || row0 >= p.a_rows) break;
+                    piece_free();
+#pragma unroll 1
+                    for (int k = 0; k < COLS; k += 32) {
+                        float v[32];
+                        tmem_ld32(lane_addr + c + k, v);
+                        const int f0 = b0 + c + k;
+                        if (EPI == 1) {
+                            // (columns come in whole groups of 32; a row of zeros beyond the matrix would take the division's slow path)
+                            if (f0 < p.b_rows && ar < p.a_rows) gated(v, v + 16, f0);
+                            put8(k / 16, v); put8(k / 16 + 1, v + 8);
+                        } else {
+                            dress(v, 32, f0);
+                            if constexpr (std::is_same<OT, float>::value) {
+#pragma unroll
+                                for (int i = 0; i < 8; ++i)
+                                    *group(lane, i) = make_uint4(__float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]),
+                                                                       __float_as_uint(v[4 * i + 2]), __float_as_uint(v[4 * i + 3]));
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) put8(k / 8 + i, v + 8 * i);
+                            }
+                        }
+                    }
+                    piece_done(EPI == 1 ? (b0 + c) >> 1 : b0 + c, row0);
+                }
             } else if (EPI == 1) {
 #pragma unroll 1
-                for (int c = 0; c < BN / 16; c += 2) {
+                for (int c = 0; c < BN / 32; c += 2) {
                     float g[16], u[16];
                     tmem_ld16(lane_addr + c * 16, g);
                     tmem_ld16(lane_addr + (c + 1) * 16, u);
                     const int f0 = b0 + c * 16;
                     if (ar < p.a_rows && f0 + 32 <= p.b_rows) {
-                        if (add_bias) {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) { g[i] += p.bias[f0 + i]; u[i] += p.bias[f0 + 16 + i]; }
-                        }
-                        if (p.act_kind == 2) {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) g[i] = rb::gelu_tanh(g[i]) * u[i];
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) g[i] = g[i] / (1.f + expf(-g[i])) * u[i];
-                        }
+                        gated(g, u, f0);
                         OT* dst = row + (f0 >> 1);
-                        if (vec_ok) store16(dst, g);
-                        else {
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) dst[i] = rb::from_f32<OT>(g[i]);
-                        }
+                        for (int i = 0; i < 16; ++i) dst[i] = rb::from_f32<OT>(g[i]);
                     }
                 }
-            } else if (EPI == 3) {
-                // out is the residual stream: out += product.  Every element belongs to one tile and one
-                // thread, so nothing else touches it meanwhile; the old values of two column groups are
-                // requested before the accumulator is read, so their latency overlaps it.
-                if constexpr (std::is_same<OT, float>::value) {
-                    rb::pdl_wait();   // these threads read what earlier kernels wrote (the residual): returns at once by now
+            } else {
 #pragma unroll 1
-                    for (int c = 0; c < BN / 16; c += 2) {
-                        const int f0 = b0 + c * 16;
-                        const bool whole = vec_ok && f0 + 32 <= p.b_rows && ar < p.a_rows;
-                        float r[32];
-                        if (whole) {
-                            load16(row + f0, r);
-                            load16(row + f0 + 16, r + 16);
-                        }
-                        float v[32];
-                        tmem_ld16(lane_addr + c * 16, v);
-                        tmem_ld16(lane_addr + (c + 1) * 16, v + 16);
-                        if (ar < p.a_rows) {
-                            if (add_bias) {
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) v[i] += (f0 + i < p.b_rows) ? p.bias[f0 + i] : 0.f;
-                            }
-                            if (whole) {
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) v[i] += r[i];
-                                store16(row + f0, v);
-                                store16(row + f0 + 16, v + 16);
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 32; ++i)
-                                    if (f0 + i < p.b_rows) row[f0 + i] += v[i];
-                            }
-                        }
-                    }
-                }
-} else {
-#pragma unroll 1
-                for (int c = 0; c < BN / 16; ++c) {
+                for (int c = 0; c < BN / 32; ++c) {
                     float v[16];
                     tmem_ld16(lane_addr + c * 16, v);
                     const int f0 = b0 + c * 16;
                     if (ar < p.a_rows) {
-                        if (add_bias) {
+                        dress(v, 16, f0);
+                        // EPI 3: every element belongs to one tile and one thread, so nothing else touches it meanwhile
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) v[i] += (f0 + i < p.b_rows) ? p.bias[f0 + i] : 0.f;
-                        }
-                        if (EPI == 4) {
-                            if (p.act_kind == 0) {
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) v[i] = rb::gelu_erf(v[i]);
-                            } else if (p.act_kind == 1) {
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) v[i] = rb::gelu_tanh(v[i]);
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) v[i] = rb::silu(v[i]);
+                        for (int i = 0; i < 16; ++i)
+                            if (f0 + i < p.b_rows) {
+                                if constexpr (EPI == 3) row[f0 + i] += v[i];
+                                else row[f0 + i] = rb::from_f32<OT>(v[i]);
                             }
-                        }
-                        if (vec_ok && f0 + 16 <= p.b_rows) {
-                            store16(row + f0, v);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i)
-                                if (f0 + i < p.b_rows) row[f0 + i] = rb::from_f32<OT>(v[i]);
-                        }
                     }
                 }
             }
@@ -1011,6 +1091,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 else mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[acc]), 0));
             }
         }
+        if (EPI != 2 && p.tma_out && lane == 0) bulk_wait_all();      // what this thread sent off has been written
+        __syncwarp();
     }
     // neither CTA may leave while the other can still read its shared memory or signal its barriers
     tc_fence_before();
@@ -1049,9 +1131,9 @@ EncodeTiledFn encode_fn() {
 struct MapKey {
     const void* ptr;
     long long rows, K, ld;
-    int box_rows;
+    int box_rows, f32;
     bool operator==(const MapKey& o) const {
-        return ptr == o.ptr && rows == o.rows && K == o.K && ld == o.ld && box_rows == o.box_rows;
+        return ptr == o.ptr && rows == o.rows && K == o.K && ld == o.ld && box_rows == o.box_rows && f32 == o.f32;
     }
 };
 struct MapKeyHash {
@@ -1060,17 +1142,17 @@ struct MapKeyHash {
         h = h * 1000003u ^ (size_t)k.rows;
         h = h * 1000003u ^ (size_t)k.K;
         h = h * 1000003u ^ (size_t)k.ld;
-        return h * 1000003u ^ (size_t)k.box_rows;
+        return h * 1000003u ^ (size_t)(k.box_rows * 2 + k.f32);
     }
 };
 
-// A [rows, K] bf16 matrix with row stride `ld` elements, read in boxes of box_rows x 64 with the
-// 128-byte swizzle.  Rows and columns outside the matrix read as zero.  Maps are cached: a
+// A [rows, K] bf16 (or float32) matrix with row stride `ld` elements, read or written in boxes of box_rows x 128 bytes with the
+// 128-byte swizzle.  Rows and columns outside the matrix read as zero and are not written.  Maps are cached: a
 // weight's map is built once.
-int tensor_map(const void* ptr, long long rows, long long K, long long ld, int box_rows, CUtensorMap* out) {
+int tensor_map(const void* ptr, long long rows, long long K, long long ld, int box_rows, CUtensorMap* out, bool f32 = false) {
     static std::mutex mu;
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-    MapKey key{ptr, rows, K, ld, box_rows};
+    MapKey key{ptr, rows, K, ld, box_rows, f32 ? 1 : 0};
     {
         std::lock_guard<std::mutex> g(mu);
         auto it = cache.find(key);
@@ -1079,10 +1161,10 @@ int tensor_map(const void* ptr, long long rows, long long K, long long ld, int b
     EncodeTiledFn fn = encode_fn();
     if (!fn) return RB_ERR_NO_DRIVER_FN;
     cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
+    cuuint32_t box[2] = {(cuuint32_t)(f32 ? 32 : BK), (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+    CUresult r = fn(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return RB_ERR_BAD_SIZE;
@@ -1172,9 +1254,16 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, void* out, Params 
         if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
         attr_done = true;
     }
+    // results leave through the copy engine where it can address them
+    CUtensorMap mo = ma;
+    p.tma_out = EPI != 2 && (((uintptr_t)out | ((uintptr_t)p.ldo * sizeof(OT))) & 15) == 0;
+    if (p.tma_out) {
+        const int rc = tensor_map(out, p.a_rows, EPI == 1 ? p.b_rows / 2 : p.b_rows, p.ldo, 32, &mo, sizeof(OT) == 4);
+        if (rc != RB_OK) return rc;
+    }
     const long long tiles = (long long)((p.a_rows + 2 * BM - 1) / (2 * BM)) * ((p.b_rows + PAIR_BN - 1) / PAIR_BN);
     const int pairs = (int)(tiles < sms / 2 ? tiles : sms / 2);
-    RB_LAUNCH((k), dim3(2 * pairs), dim3(192), PAIR_SMEM, s, ma, mb, (OT*)out, p);
+    RB_LAUNCH((k), dim3(2 * pairs), dim3(PAIR_THREADS), PAIR_SMEM, s, ma, mb, mo, (OT*)out, p);
     return RB_OK;
 }
 

@@ -51,10 +51,10 @@ from .base import BuildEnv, DeferredNorm, Mixer, build_position, register_mixer
 from .linear import Linear
 
 # From this many tokens in a step the q | k | v projection normalises, rotates and caches in its own
-# epilogue.  With fewer tokens a block has too few tiles to hide that epilogue behind the next tile's
-# main loop, and the rotation kernel after a plain product is as fast or faster (measured at 1,024 and
-# 2,048 tokens against 4,096).
-PROMPT_FUSED_MIN_TOKENS = 4096
+# epilogue; from eight times as many if its sum over K is split for want of tiles (the partial sums go to the rotation kernel).
+# Product and rotation kernel against one: 37 and 37 us at 760 tokens of a 4,096 wide model, 87 and 78 at 2,048; 65 and 56 at
+# 2,048 of a 2,560 wide one, 80 and 65 at 4,096 of a 2,048 wide one.
+PROMPT_FUSED_MIN_TOKENS = 512
 
 # Tensor-name stems by role, unless the spec's ``names`` says otherwise (the defaults are those of
 # Hugging Face's Qwen3 checkpoints: rocml/src/weights/layer.rs:47-58 lists the same tensors under GGUF names).
@@ -470,7 +470,7 @@ class Attention(Mixer):
         if rot not in (0, self.hd) or writes != (self.qkv.n == (self.nq + 2 * self.nkv) * self.hd):
             return False
         T = batch.n_tokens
-        if T < PROMPT_FUSED_MIN_TOKENS:
+        if T < PROMPT_FUSED_MIN_TOKENS * (8 if self.qkv._splits(T) > 1 else 1):
             return False
         q = torch.empty((T, self.nq * self.hd), dtype=torch.bfloat16, device=xn.device)
         cos_sin = self.position.cos_sin(batch) if rot else None

@@ -221,6 +221,41 @@ def test_gemm_tcgen05_qkv_projection_rotates_and_caches(M, nq, nkv, K, norm, rop
         assert int((kc.float().abs().sum(-1) > 0).sum()) <= seen * nkv     # nothing written elsewhere
 
 
+@pytest.mark.parametrize("M,N,K", [(257, 256, 64), (289, 288, 72), (300, 352, 520), (513, 1056, 128), (1100, 256, 448)])
+@pytest.mark.parametrize("pad", [0, 8, 1])
+def test_gemm_tcgen05_pair_results_leave_whole(M, N, K, pad):
+    """The kernel of CTA pairs hands its results to the copy engine in pieces of 32 rows (float32 and bfloat16, gated, added
+    into what is there), or stores them itself when the rows are off 16 bytes (pad 1): ragged rows and columns, and nothing
+    outside the matrix is touched.  The bounds: bfloat16 results 2^-8 of their size, float32 ones K 2^-24 of the sum of sizes."""
+    from rocml_b200 import kernels
+    x, w = rnd((M, K), 1, torch.bfloat16).to(DEV), rnd((N, K), 2, torch.bfloat16).to(DEV)
+    bias = rnd((N,), 3).to(DEV)
+    xd, wd, bd = x.cpu().double(), w.cpu().double(), bias.cpu().double()
+    want, sizes = xd @ wd.t() + bd, xd.abs() @ wd.abs().t() + bd.abs()
+    slack = sizes * (K * 2.0 ** -24)
+
+    def frame(cols, dtype, fill):
+        wide = torch.full((M + 40, cols + pad), fill, dtype=dtype, device=DEV)
+        return wide, wide[:M, :cols]
+
+    for dtype, rounding in ((torch.float32, 0.0), (torch.bfloat16, 2.0 ** -8)):
+        wide, out = frame(N, dtype, 7.0)
+        assert kernels.gemm_tcgen05(x, w, out, bias, M)
+        assert ((out.cpu().double() - want).abs() <= slack + want.abs() * rounding + 1e-30).all()
+        assert (wide[M:] == 7.0).all() and (wide[:, N:] == 7.0).all()
+    wide, out = frame(N, torch.float32, 0.5)
+    assert kernels.gemm_tcgen05_add(x, w, out, bias, M)
+    assert ((out.cpu().double() - want - 0.5).abs() <= slack + (want.abs() + 1) * 2.0 ** -22).all()
+    assert (wide[M:] == 0.5).all() and (wide[:, N:] == 0.5).all()
+    g, u = (want.reshape(M, N // 32, 2, 16)[:, :, j].reshape(M, N // 2) for j in (0, 1))
+    slack_g, slack_u = (slack.reshape(M, N // 32, 2, 16)[:, :, j].reshape(M, N // 2) for j in (0, 1))
+    gated = g / (1 + torch.exp(-g)) * u
+    wide, out = frame(N // 2, torch.bfloat16, 7.0)
+    assert kernels.gemm_tcgen05(x, w, out, bias, M, gated=True)
+    assert ((out.cpu().double() - gated).abs() <= gated.abs() * 2.0 ** -7.9 + 1.1 * u.abs() * slack_g + g.abs() * slack_u + 1e-6).all()
+    assert (wide[M:] == 7.0).all() and (wide[:, N // 2:] == 7.0).all()
+
+
 def test_gemm_tcgen05_refuses_unaligned_k():
     from rocml_b200 import kernels
     x = rnd((4, 100), 1, torch.bfloat16).to(DEV)  # K = 100: rows are not a multiple of 16 bytes
