@@ -140,7 +140,7 @@ int rb_gemm_tcgen05(const void* x, const void* w, const float* bias, void* out, 
 
 int rb_gemm_tcgen05_gated_pair(const void* x, const void* w, const float* bias, void* h, int M, int N, int K,
                                long long ldx, long long ldh, const float* row_sumsq, int row_groups,
-                               long long row_sumsq_ld, float row_eps, int stages, int* status, void* stream);
+                               long long row_sumsq_ld, float row_eps, int parts, int stages, int* status, void* stream);
 
 int rb_gemm_tcgen05_residual(const void* x, const void* w, const float* bias, int M, int N, int K, long long ldx,
                              int splits, float* resid, long long ld_resid, const void* next_w, int next_w_f32,

@@ -129,6 +129,9 @@ __device__ __forceinline__ void store16(__nv_bfloat16* dst, const float* v) {
 // residual (float32), and for the norm that follows: residual * weight in bfloat16 (the next product's
 // input, to be scaled by the row's 1/RMS in that product's epilogue) and its share of the row's sum
 // of squares.  No partial sums go through global memory and no norm kernel runs in between.
+// CS = 4 and GATED: the same exchange for a gate/up weight whose sum over K is in four parts: an owner's 32 rows are the
+// gates and the ups of 16 outputs, and it writes silu(gate) * up of them.  Two kernels fewer a layer than four partial
+// sums, a norm and an activation of their own: 6,144 x 1,024 and one token, a layer 29 -> 26 us; 12,288 x 2,048 and eight, 50 -> 43.
 template <int BN, bool SWAP, typename OT, bool GATED, int CS>
 __global__ void __launch_bounds__(192, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -143,7 +146,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint32_t* tmem_slot = (uint32_t*)(acc_ready + 1);
     uint32_t* abort_flag = tmem_slot + 1;
     float* handover = (float*)(smem + S * C::STAGE + 256);   // CS: [BN][128] floats from the other half
-    __shared__ float s_rstd[CS == 2 ? BN : 1];               // CS == 2: the tokens' 1/RMS
+    constexpr bool SCALED = CS == 2 || (CS == 4 && GATED);
+    __shared__ float s_rstd[SCALED ? BN : 1];                // the tokens' 1/RMS
 
     rb::pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -249,6 +253,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tc_fence_after();
         const bool aborted = !ok || *(volatile uint32_t*)abort_flag != 0;
         if (!ok && lane == 0) atomicExch(p.status, RB_ERR_TIMEOUT);
+        if (SCALED && (CS == 4 || blockIdx.z == 0) && p.row_sumsq != nullptr) {
+            // the 1/RMS of this tile's tokens, from the shares the kernel before left
+            rb::pdl_wait();
+            for (int j = quarter; j < BN; j += 4) {
+                const int tok = b0 + j;
+                float acc = 0.f;
+                if (tok < p.b_rows)
+                    for (int gi = lane; gi < p.row_groups; gi += 32) acc += p.row_sumsq[(size_t)gi * p.row_sumsq_ld + tok];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0) s_rstd[j] = rsqrtf(acc * p.row_inv_width + p.row_eps);
+            }
+        }
         if (CS >= 4) {
             // every block sends each owner its rows of the accumulator
             if (!aborted && n_kb > 0) {
@@ -266,19 +283,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         } else if (CS != 0) {
             // the second half hands its accumulator over; the first half goes on after the barrier
-            if (blockIdx.z == 0 && p.row_sumsq != nullptr) {
-                // meanwhile: the 1/RMS of this tile's tokens, from the shares the kernel before left
-                rb::pdl_wait();
-                for (int j = quarter; j < BN; j += 4) {
-                    const int tok = b0 + j;
-                    float acc = 0.f;
-                    if (tok < p.b_rows)
-                        for (int gi = lane; gi < p.row_groups; gi += 32) acc += p.row_sumsq[(size_t)gi * p.row_sumsq_ld + tok];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                    if (lane == 0) s_rstd[j] = rsqrtf(acc * p.row_inv_width + p.row_eps);
-                }
-            }
             if (!aborted && n_kb > 0 && blockIdx.z != 0) {
                 const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
                 const uint32_t dst = map_to_cta(smem_u32(handover + quarter * 32 + lane), 0);
@@ -389,7 +393,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // what the first round below reads from global memory is requested before the barrier, so that it
         // arrives while the blocks wait for one another (a block is the only writer of its residual rows)
         float first_r = 0.f, first_w = 1.f, first_b = 0.f;
-        if (CS >= 4 && warp >= 2) {
+        if (CS >= 4 && !GATED && warp >= 2) {
             rb::pdl_wait();   // these threads read what earlier kernels wrote (the residual): returns at once by now
             constexpr int RPC = 128 / (CS >= 4 ? CS : 4);
             const int e = (warp & 3) * 32 + lane;
@@ -405,7 +409,29 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         __syncwarp();
         cluster_arrive();
         cluster_wait();
-        if (CS >= 4 && warp >= 2) {
+        if (CS >= 4 && GATED && warp >= 2) {
+            const int e = (warp & 3) * 32 + lane;                   // 0..127 among the epilogue threads
+            const int f = e & 15, ar = a0 + (int)blockIdx.z * 32 + f;        // the output's gate row; its up row is 16 further
+            const float bg = (p.bias != nullptr && ar < p.a_rows) ? p.bias[ar] : 0.f;
+            const float bu = (p.bias != nullptr && ar < p.a_rows) ? p.bias[ar + 16] : 0.f;
+            if (*(volatile uint32_t*)abort_flag == 0) {
+#pragma unroll 1
+                for (int j = e >> 4; j < BN; j += 8) {
+                    const int tok = b0 + j;
+                    float g = 0.f, u = 0.f;
+#pragma unroll
+                    for (int src = 0; src < CS; ++src) {
+                        g += handover[((size_t)src * BN + j) * 32 + f];
+                        u += handover[((size_t)src * BN + j) * 32 + 16 + f];
+                    }
+                    const float rs = p.row_sumsq != nullptr ? s_rstd[j] : 1.f;
+                    g = g * rs + bg;
+                    u = u * rs + bu;
+                    if (tok < p.b_rows && ar < p.a_rows)
+                        out[(size_t)tok * p.ldo + (ar >> 5) * 16 + f] = rb::from_f32<OT>(g / (1.f + expf(-g)) * u);
+                }
+            }
+        } else if (CS >= 4 && !GATED && warp >= 2) {
             constexpr int RPC = 128 / (CS >= 4 ? CS : 4);
             const int e = (warp & 3) * 32 + lane;                   // 0..127 among the epilogue threads
 #pragma unroll 1
@@ -435,7 +461,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (row_in == 0 && tok < p.b_rows && p.sumsq != nullptr)
                     p.sumsq[((size_t)blockIdx.x * CS + blockIdx.z) * p.sumsq_ld + tok] = sq;
             }
-        } else if (blockIdx.z == 0 && warp >= 2 && n_kb > 0 && *(volatile uint32_t*)abort_flag == 0) {
+        } else if (CS == 2 && blockIdx.z == 0 && warp >= 2 && n_kb > 0 && *(volatile uint32_t*)abort_flag == 0) {
             // features on the TMEM lanes: lanes 0-15 of a warp hold gates, lanes 16-31 the ups
             const int quarter = warp & 3;
             const int ar = a0 + quarter * 32 + lane;
@@ -1370,7 +1396,7 @@ static int gemm_entry(const void* x, const void* w, const float* bias, void* out
     }
     p.row_sumsq = nullptr; p.row_groups = 0; p.row_sumsq_ld = 0; p.row_eps = 0.f; p.row_inv_width = 0.f;
     if (rsc != nullptr && rsc->sumsq != nullptr) {
-        if (cluster_split != 2 || rsc->groups < 1 || rsc->width < 1) return RB_ERR_BAD_SIZE;
+        if ((cluster_split != 2 && cluster_split != 4) || ro != nullptr || rsc->groups < 1 || rsc->width < 1) return RB_ERR_BAD_SIZE;
         p.row_sumsq = rsc->sumsq; p.row_groups = rsc->groups; p.row_sumsq_ld = rsc->ld;
         p.row_eps = rsc->eps; p.row_inv_width = 1.f / (float)rsc->width;
     }
@@ -1397,8 +1423,11 @@ static int gemm_entry(const void* x, const void* w, const float* bias, void* out
 #undef RB_RS
     }
     if (cluster_split != 0) {
-        if (cluster_split != 2 || !swap || bn > 32 || out_dtype != RB_BF16 || N % 32 || kb_total < 2) return RB_ERR_BAD_SIZE;
-        p.splits = 2;
+        if ((cluster_split != 2 && cluster_split != 4) || !swap || bn > (cluster_split == 4 ? 16 : 32) || out_dtype != RB_BF16 ||
+            N % 32 || kb_total < cluster_split)
+            return RB_ERR_BAD_SIZE;
+        p.splits = cluster_split;
+        if (cluster_split == 4) return launch<16, true, __nv_bfloat16, true, 4>(ma, mb, out, p, 4, s);
         return bn == 16 ? launch<16, true, __nv_bfloat16, false, 2>(ma, mb, out, p, 2, s)
                         : launch<32, true, __nv_bfloat16, false, 2>(ma, mb, out, p, 2, s);
     }
@@ -1490,14 +1519,16 @@ extern "C" int rb_gemm_tcgen05_add(const void* x, const void* w, const float* bi
 // thread-block cluster (see the kernel).  With row_sumsq (shares [row_groups][>= M] of the sums of squares
 // of the rows that x was made from, row_sumsq_ld apart) x is taken as not yet divided by its rows' RMS
 // over K values: the product is scaled by rsqrt(sum / K + row_eps) before the bias.
-// RB_ERR_BAD_SIZE for more rows, N not a multiple of 32, or K of a single 64-wide block;
+// parts: 2, or 4 (at most 16 rows) for the sum over K in four parts.
+// RB_ERR_BAD_SIZE for more rows, N not a multiple of 32, or fewer 64-wide blocks of K than parts;
 // RB_ERR_BAD_ALIGN as rb_gemm_tcgen05.
 extern "C" int rb_gemm_tcgen05_gated_pair(const void* x, const void* w, const float* bias, void* h, int M, int N,
                                           int K, long long ldx, long long ldh, const float* row_sumsq,
-                                          int row_groups, long long row_sumsq_ld, float row_eps, int stages,
+                                          int row_groups, long long row_sumsq_ld, float row_eps, int parts, int stages,
                                           int* status, void* stream) {
+    if (parts != 2 && parts != 4) return RB_ERR_BAD_SIZE;
     RowScale rsc{row_sumsq, row_groups, row_sumsq_ld, row_eps, K};
-    return gemm_entry(x, w, bias, h, RB_BF16, M, N, K, ldx, ldh, 1, 0, stages, 0, status, stream, 2, nullptr, &rsc);
+    return gemm_entry(x, w, bias, h, RB_BF16, M, N, K, ldx, ldh, 1, 0, stages, 0, status, stream, parts, nullptr, &rsc);
 }
 
 // resid[M, N] += x[M, K] . w[N, K]^T (+ bias) for at most 64 rows, the sum over K in `splits` (4, 8

@@ -151,7 +151,7 @@ def _lib():
         lib.rb_sample.argtypes = [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp]
         lib.rb_gemm_tcgen05.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _ll, _i, _i, _vp, _vp]
         lib.rb_gemm_tcgen05_add.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _i, _vp, _vp]
-        lib.rb_gemm_tcgen05_gated_pair.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _vp, _i, _ll, _f, _i, _vp, _vp]
+        lib.rb_gemm_tcgen05_gated_pair.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _vp, _i, _ll, _f, _i, _i, _vp, _vp]
         lib.rb_gemm_tcgen05_qkv_rope.argtypes = [_vp, _vp, _vp, _i, _i, _i, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _i, _vp,
                                                  _vp, _i, _f, _vp, _i, _i, _i, _vp, _vp]
         lib.rb_gemm_tcgen05_residual.argtypes = [_vp, _vp, _vp, _i, _i, _i, _ll, _i, _vp, _ll, _vp, _i, _vp, _ll, _vp,
@@ -898,13 +898,14 @@ def gemm_tcgen05_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: s
 
 @_profiled(lambda a, facts: _cost.gated_linear(_rows(a), a["w"].shape[0], a["w"].shape[1], 2, 2, 2))
 def gemm_tcgen05_gated_pair(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                            m: Optional[int] = None, rowscale=None) -> bool:
+                            m: Optional[int] = None, rowscale=None, parts: int = 2) -> bool:
     """h = silu(gate) * up for at most 32 rows, w's rows alternating in blocks of 16 between gate and
     up, with the sum over K done in two halves by two blocks that form a thread-block cluster: the
     second hands its half to the first through shared memory, so no partial sums go through global
     memory.  h is bfloat16 [M, N / 2].  ``rowscale`` = (sumsq float32 [G, >= M], eps): x's rows are
     residual * norm weight, not yet divided by their RMS; column m of sumsq sums to row m's sum of
     squares over K values, and the product is scaled by rsqrt(sum / K + eps) before the bias.
+    ``parts`` = 4 (at most 16 rows): the sum in four parts by clusters of four blocks.
     Returns False when the kernel refuses the sizes or the layout."""
     M = x.shape[0] if m is None else m
     N, K = w.shape
@@ -918,7 +919,7 @@ def gemm_tcgen05_gated_pair(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor, b
     if M > 32 or N % 32 or K <= 64:
         return False
     rc = _lib().rb_gemm_tcgen05_gated_pair(_ptr(x), _ptr(w), _ptr(bias), _ptr(h), M, N, K, x.stride(0), h.stride(0),
-                                           *_row_scale(rowscale, M, "gemm_tcgen05_gated_pair"), 0,
+                                           *_row_scale(rowscale, M, "gemm_tcgen05_gated_pair"), parts, 0,
                                            _ptr(status_word(x.device)), _stream())
     if rc in (10001, 10003):
         return False

@@ -156,13 +156,23 @@ class Linear:
 
     @_labelled
     def forward_gated_pair(self, x: torch.Tensor, m: int, rowscale=None) -> Optional[torch.Tensor]:
-        """The same for few rows when the sum over K is split in two: the two halves' blocks form a
+        """The same for few rows when the sum over K is split: the parts' blocks form a
         cluster and the activation is applied where they meet, so no second kernel waits for partial
-        sums.  None when this step's product is split otherwise or the kernel refuses."""
-        if not (self.paired and self._tensor_core(x)) or self._splits(m) != 2 or m > GATED_PAIR_MAX_ROWS:
+        sums.  None when this step's product is not split or the kernel refuses."""
+        parts = self.gated_parts(m)
+        if not (self.paired and self._tensor_core(x)) or not parts:
             return None
         out = torch.empty((m, self.n // 2), dtype=torch.bfloat16, device=x.device)
-        return out if kernels.gemm_tcgen05_gated_pair(x, self.weight, out, self.bias, m, rowscale=rowscale) else None
+        return out if kernels.gemm_tcgen05_gated_pair(x, self.weight, out, self.bias, m, rowscale=rowscale, parts=parts) else None
+
+    def gated_parts(self, m: int) -> int:
+        """In how many parts ``forward_gated_pair`` would take the sum over K for m rows: two, or four where more would be
+        in flight otherwise (a step of 8 rows and 28 layers with 12,288 x 2,048 weights: 1.42 ms with four partial sums and
+        the activation's kernel, 1.48 in two parts, which are half the blocks, 1.31 in four); 0: not at all."""
+        s = self._splits(m)
+        if s < 2 or m > GATED_PAIR_MAX_ROWS or self.k <= 64:
+            return 0
+        return 2 if s == 2 else (4 if self.k // 64 >= 8 else 0)
 
     def residual_splits(self, m: int) -> int:
         """In how many parts ``forward_residual`` would split the sum over K for m rows (0: it would not
@@ -172,7 +182,7 @@ class Linear:
         # clusters of 8: larger ones leave too few of them resident at once (a cluster needs all its
         # blocks on neighbouring multiprocessors)
         s = self._splits(m)
-        s = 8 if s >= 8 else (4 if s >= 4 else 0)
+        s = 8 if s >= 6 else (4 if s >= 4 else 0)
         return s if s and self.k // 64 >= s else 0
 
     @_labelled

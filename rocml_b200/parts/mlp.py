@@ -11,7 +11,7 @@ from ..errors import ConfigError
 from ..profile import scope
 from ..weights.decl import TensorDecl
 from .base import BuildEnv, DeferredNorm, FeedForward, register_feed_forward
-from .linear import GATED_PAIR_MAX_ROWS, Linear
+from .linear import Linear
 
 
 # Tensor-name stems by role, unless the spec's ``names`` says otherwise (rocml/src/weights/layer.rs:59-62).
@@ -73,8 +73,8 @@ class GatedMLP(FeedForward):
         """Whether forward() can be handed a DeferredNorm for this step: only the product of two blocks
         that applies the activation itself also applies the rows' 1/RMS."""
         T = batch.n_tokens
-        return (self.act == "silu" and self.gate_up.paired and T <= GATED_PAIR_MAX_ROWS and self.gate_up.weight.dtype == torch.bfloat16
-                and self.gate_up._splits(T) == 2 and self.gate_up.k > 64)
+        return (self.act == "silu" and self.gate_up.paired and self.gate_up.weight.dtype == torch.bfloat16
+                and self.gate_up.gated_parts(T) > 0)
 
     can_add_into = True    # forward() accepts add_into=residual (see parts.base)
 

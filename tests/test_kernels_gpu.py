@@ -96,6 +96,29 @@ def test_gemm_tcgen05_gated_pair_of_blocks(M, I, K):
                                            torch.empty((40, I), dtype=torch.bfloat16, device=DEV)) is False
 
 
+@pytest.mark.parametrize("M,I,K", [(1, 208, 256), (16, 48, 264), (8, 3072, 1024), (9, 6144, 2048)])
+def test_gemm_tcgen05_gated_by_clusters_of_four(M, I, K):
+    """The same with the sum over K in four parts, every block of the cluster writing a quarter of the tile's outputs; with
+    and without the rows' 1/RMS still to be applied.  The bound is the two-part test's."""
+    from rocml_b200 import kernels
+    x = rnd((M, K), 1, torch.bfloat16).to(DEV)
+    w, b = rnd((2 * I, K), 2, torch.bfloat16, 0.2).to(DEV), rnd((2 * I,), 4).to(DEV)
+    sumsq = rnd((5, M + 3), 6).abs().to(DEV)
+    raw = (x.cpu().double() @ w.cpu().double().t()).reshape(M, I // 16, 2, 16)
+    bias = b.cpu().double().reshape(I // 16, 2, 16)
+    for rowscale, factor in ((None, 1.0), ((sumsq, 1e-3), (sumsq[:, :M].cpu().double().sum(0) / K + 1e-3).rsqrt()[:, None])):
+        g, u = ((raw[:, :, j].reshape(M, I) * factor + bias[:, j].reshape(I)) for j in (0, 1))
+        want = g / (1 + torch.exp(-g)) * u
+        out = torch.full((M + 1, I), float("nan"), dtype=torch.bfloat16, device=DEV)
+        assert kernels.gemm_tcgen05_gated_pair(x, w, out, b, M, rowscale=rowscale, parts=4)
+        kernels.check_status(DEV)
+        scale = torch.maximum(want.abs(), g.abs().clamp_min(1.0) * u.abs().clamp_min(1.0) * 2.0 ** -2)
+        assert ((out[:M].cpu().double() - want).abs() / scale.clamp_min(1.0)).max().item() < 2 ** -7
+        assert torch.isnan(out[M]).all()
+    assert kernels.gemm_tcgen05_gated_pair(rnd((17, K), 1, torch.bfloat16).to(DEV), w, torch.empty((17, I), dtype=torch.bfloat16, device=DEV),
+                                           parts=4) is False
+
+
 @pytest.mark.parametrize("M,N,K,S,wdt", [(1, 4096, 4096, 8, torch.bfloat16), (8, 520, 1024, 4, torch.float32),
                                          (16, 256, 12288, 16, torch.bfloat16), (3, 1000, 512, 8, torch.float32),
                                          (33, 520, 1024, 8, torch.bfloat16), (64, 4096, 512, 8, torch.float32),
