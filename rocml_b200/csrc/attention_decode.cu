@@ -265,15 +265,16 @@ __device__ __forceinline__ float finished(float A, float L, float M, float sink)
     return L > 0.f ? A / L : 0.f;
 }
 
-// Dynamic shared memory: the query tile and two buffers a warp, or what the merge of the warps' results needs instead.
-template <int HD>
+// Dynamic shared memory: the query tile and NB buffers a warp, or what the merge of the warps' results needs instead.
+template <int HD, int NB = 2>
 __host__ __device__ constexpr size_t decode_region() {
-    const size_t kv = (size_t)WARPS * 4 * WK * HD * sizeof(__nv_bfloat16), merge = (size_t)WARPS * ROWS * HD * sizeof(float);
+    const size_t kv = (size_t)WARPS * NB * 2 * WK * HD * sizeof(__nv_bfloat16), merge = (size_t)WARPS * ROWS * HD * sizeof(float);
     return (size_t)ROWS * HD * sizeof(__nv_bfloat16) + (kv > merge ? kv : merge);
 }
 
-template <int HD, bool CL, bool FQ, bool PROP, bool TR>
-__global__ void __launch_bounds__(WARPS * 32, HD <= 128 ? 3 : 1)
+// NB: pages in flight a warp.  Two, three blocks a multiprocessor; or one, so that four fit: see `launch`.
+template <int HD, bool CL, bool FQ, bool PROP, bool TR, int NB = 2>
+__global__ void __launch_bounds__(WARPS * 32, HD <= 128 ? (NB == 1 ? 4 : 3) : 1)
 attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
                         const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
                         const int* __restrict__ block_table, int max_pages, const int* __restrict__ seq_slot,
@@ -293,7 +294,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     // CL: where the parts of this block's slice of the head size land (TR: pushed by their blocks, [blocks][heads][slice],
     // beyond everything that is in use before), or this block's own part [16][HD], which the others read
     constexpr bool PUSH = CL && TR;
-    float* s_part = PUSH ? reinterpret_cast<float*>(smem_raw + decode_region<HD>()) : s_o + WARPS * ROWS * HD;
+    float* s_part = PUSH ? reinterpret_cast<float*>(smem_raw + decode_region<HD, NB>()) : s_o + WARPS * ROWS * HD;
     // the parts' (or its own) maxima and sums
     __shared__ float s_pm[PUSH ? MAX_CLUSTER : 1][PUSH ? 8 : ROWS], s_pl[PUSH ? MAX_CLUSTER : 1][PUSH ? 8 : ROWS];
     if (PUSH) cluster_arrive_relaxed();                                    // (a block's memory may be written once it runs)
@@ -377,7 +378,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
 
     // Each warp owns 16 keys of every page and two shared-memory buffers for them: while it
     // works on one page its copies of the next are in flight.
-    __nv_bfloat16* KVw = KVs + warp * 4 * WK * HD;          // [2 buffers][K 16 x HD | V 16 x HD]
+    __nv_bfloat16* KVw = KVs + warp * (NB * 2) * WK * HD;   // [NB buffers][K 16 x HD | V 16 x HD]
     auto issue = [&](int page_idx, int buf, int without_new) {
         const int j0 = page_idx * CHUNK + warp * WK;
         const int hi = min(pos, (page_idx + 1) * CHUNK - 1);
@@ -400,12 +401,12 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     // shared memory beside them when it is ready.  Any other page waits for the kernels before this one.
     const int new_page = pos / CHUNK;
     const bool owner = FQ && pj.write_kv && hc == 0 && page_first <= new_page && new_page <= page_last;
-    const bool patch = owner && new_page < page_first + 2;     // (a block's third page is copied after its row was written)
+    const bool patch = owner && new_page < page_first + NB;    // (a block's later pages are copied after their rows were written)
     const bool early0 = page_first < new_page || (patch && page_first == new_page);
-    const bool early1 = page_first + 1 < new_page || (patch && page_first + 1 == new_page);
+    const bool early1 = NB == 1 || page_first + 1 < new_page || (patch && page_first + 1 == new_page);
     const bool idle = CL && page_first > page_last;            // a block of the cluster beyond the sequence
     if (early0) issue(page_first, 0, page_first == new_page);
-    if (early1) issue(page_first + 1, 1, page_first + 1 == new_page);
+    if (NB == 2 && early1) issue(page_first + 1, 1, page_first + 1 == new_page);
     // a sequence that one block of the cluster covers needs no merge: the others leave
     const bool alone = CL && parts_hi == 0;
     if (alone && idle) {
@@ -472,7 +473,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
                 const uint2 packed[2] = {pack4_bf16(v), pack4_bf16(v + 4)};
                 // a row of a swizzled tile: queries to their own, a new key or value into the copy of its page ...
                 const int r = kind == 0 ? task : pos % WK;
-                __nv_bfloat16* tile = kind == 0 ? Qs : KVs + ((pos % CHUNK) / WK * 4 + (new_page - page_first) * 2 + (kind - 1)) * WK * HD;
+                __nv_bfloat16* tile = kind == 0 ? Qs : KVs + ((pos % CHUNK) / WK * (NB * 2) + (new_page - page_first) * 2 + (kind - 1)) * WK * HD;
                 if (kind == 0 || patch) {
 #pragma unroll
                     for (int h = 0; h < 2; ++h)                 // 8 values per 16-byte chunk, 4 per lane
@@ -675,14 +676,14 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         }
     };
     for (int pg = page_first; pg <= page_last; ++pg) {
-        const int buf = (pg - page_first) & 1;
-        if (pg >= page_first + 2) {
-            cp_async_wait<1>();                             // page pg has landed; page pg + 1 may be on its way
+        const int buf = NB == 2 ? (pg - page_first) & 1 : 0;
+        if (pg >= page_first + NB) {
+            cp_async_wait<NB - 1>();                        // page pg has landed; page pg + 1 may be on its way
             __syncwarp();
         }
         attend_page(pg, buf);
         __syncwarp();                                       // the buffer is free again
-        issue(pg + 2, buf, 0);
+        issue(pg + NB, buf, 0);
     }
     cp_async_wait<0>();
 #pragma unroll
@@ -866,12 +867,12 @@ bool cluster_enabled() {
     return on;
 }
 
-template <int HD, bool CL, bool FQ, bool PROP, bool TR>
+template <int HD, bool CL, bool FQ, bool PROP, bool TR, int NB = 2>
 int launch_variant(dim3 grid, size_t smem, cudaStream_t s, const void* q, int q_stride, const void* k_cache,
                    const void* v_cache, const int* block_table, int max_pages, const int* seq_slot, const int* cu_q,
                    const int* kv_len, int nq, int nkv, float scale, int window, int keep, float sink, int n_chunks, int ppb,
                    float* part_acc, float* part_ml, int* counters, void* out, int o_stride, const Projections& pj, int n_seqs) {
-    auto k = attention_decode_kernel<HD, CL, FQ, PROP, TR>;
+    auto k = attention_decode_kernel<HD, CL, FQ, PROP, TR, NB>;
     static bool attr_done = false;
     if (!attr_done) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -929,6 +930,23 @@ int launch(const void* q, int q_stride, const void* k_cache, const void* v_cache
                                      : launch_variant<HD, CL, FQ, PROP, false>(grid, smem, s, q, q_stride, k_cache, v_cache, block_table, \
                                                          max_pages, seq_slot, cu_q, kv_len, nq, nkv, scale, window, keep, sink, \
                                                          n_chunks, ppb, part_acc, part_ml, counters, out, o_stride, pj, B))
+    // One block a (sequence, head group), and more of them than three a multiprocessor but no more than four: with one page
+    // in flight instead of two all run at once, where a thin second wave took as long as the first (64 sequences of 17 to 57
+    // keys on 8 heads, 512 blocks on 444 places: 16 steps of 36 layers with their prompts 63.4 -> 61.0 ms).  decode_split sends contexts beyond seven pages another way.
+    if constexpr (HD == 128) {
+        const long long blocks = (long long)grid.y * grid.z;
+        if (fused && !proportional && n_chunks == 1 && g <= 8) {
+            static const int sms = [] {
+                int dev = 0, n = 0;
+                return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 0;
+            }();
+            if (blocks > 3 * sms && blocks <= 4 * sms && ppb <= 7)
+                return launch_variant<128, false, true, false, true, 1>(grid, decode_region<128, 1>(), s, q, q_stride, k_cache, v_cache,
+                                                                        block_table, max_pages, seq_slot, cu_q, kv_len, nq, nkv, scale,
+                                                                        window, keep, sink, n_chunks, ppb, part_acc, part_ml, counters,
+                                                                        out, o_stride, pj, B);
+        }
+    }
     if (proportional) return (HD == 128 && fused) ? RB_ADV(false, (HD == 128), true) : RB_ADV(false, false, true);
     if (HD == 128 && fused) return clustered ? RB_ADV(true, (HD == 128), false) : RB_ADV(false, (HD == 128), false);
     return clustered ? RB_ADV(true, false, false) : RB_ADV(false, false, false);

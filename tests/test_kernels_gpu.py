@@ -939,6 +939,13 @@ def test_attention_decode_puts_the_new_row_beside_its_page(lens, window, grid, n
     test_attention_decode_takes_the_projections_itself(lens, nq, nkv, window, S, True, True, grid, 1e-6)
 
 
+@pytest.mark.parametrize("n,nkv,window", [(56, 8, None), (74, 8, 70), (149, 3, None)])
+def test_attention_decode_of_a_few_more_pairs_than_places(n, nkv, window):
+    """445 to 592 (sequence, head group) pairs, a block each: one page in flight a block, and one to five pages long."""
+    lens = [1, 64, 65, 128, 129, 256, 257, 300] + [5 + 37 * i % 310 for i in range(n - 8)]
+    test_attention_decode_takes_the_projections_itself(lens, 2 * nkv, nkv, window, 2, True, True, (5, 1), 1e-6)
+
+
 def test_attention_decode_leaves_wide_groups_to_the_two_kernels():
     """More than 16 query heads a key/value head: several blocks would read the new token's page while
     one of them writes it, so the kernel that takes the projections declines (the caller then writes
