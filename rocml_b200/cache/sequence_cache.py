@@ -46,6 +46,7 @@ class KVGroup:
         shape = (n_entries, n_pages, req.n_kv_heads, PAGE, req.head_dim)
         self.k = torch.zeros(shape, dtype=dtype, device=device)
         self.v = self.k if req.shared_values else torch.zeros(shape, dtype=dtype, device=device)
+        self.k_of, self.v_of = self.k.unbind(0), self.v.unbind(0)      # every layer's part, made once
         self.pool = FreeList(n_pages, "page")
         self.table_host = np.full((max_slots, max_pages_per_seq), -1, dtype=np.int32)
         self.table = torch.full((max_slots, max_pages_per_seq), -1, dtype=torch.int32, device=device)
@@ -202,11 +203,11 @@ class CacheView:
 
     @property
     def k(self):
-        return self.group.k[self.index]
+        return self.group.k_of[self.index]
 
     @property
     def v(self):
-        return self.group.v[self.index]
+        return self.group.v_of[self.index]
 
     @property
     def block_table(self):

@@ -47,12 +47,12 @@ def _ptr(t: Optional[torch.Tensor]):
         return None
     if not t.is_cuda:
         raise KernelError("kernel arguments must live on a CUDA device; there is no CPU path")
-    return _vp(t.data_ptr())
+    return t.data_ptr()
 
 
 def _stream():
     # the raw handle of torch's current stream on the current device, without building a Stream object
-    return _vp(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 launch_count = 0  # kernel launches issued through this module (graph replays are counted by the engine)
@@ -788,7 +788,7 @@ _status = {}
 
 def status_word(device) -> torch.Tensor:
     """One int32 per device where kernels record a bounded wait that ran out (or a bad token id)."""
-    key = torch.device(device).index or 0
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     if key not in _status:
         _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return _status[key]

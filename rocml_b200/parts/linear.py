@@ -33,10 +33,35 @@ GATED_PAIR_MAX_ROWS = 16
 
 
 def _sm_count(device) -> int:
-    key = torch.device(device).index or 0
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     if key not in _SM_COUNT:
         _SM_COUNT[key] = torch.cuda.get_device_properties(device).multi_processor_count
     return _SM_COUNT[key]
+
+
+@functools.lru_cache(maxsize=4096)
+def _split_rule(n: int, k: int, m: int, sms: int) -> int:
+    """``Linear._splits`` on numbers alone (asked several times a layer and step)."""
+    if m > 128:
+        # A few hundred rows: the output has fewer 128 x 256 tiles than the device has
+        # multiprocessors, and each block would stream its share of the weight alone.  The sum over
+        # K is split until the blocks fill one wave (measured at 160 to 1,024 rows: whenever tiles
+        # times splits stays within the multiprocessors the split wins, up to 2.7 times; beyond, it
+        # loses to the kernels for many rows).
+        tiles = ((m + 127) // 128) * ((n + 255) // 256)
+        s = min(sms // max(1, tiles), (k // 64) // 8, 8)
+        return s if s >= 2 else 1
+    tiles = (n + 127) // 128
+    k_blocks = k // 64
+    by_blocks = -(-2 * sms // tiles)
+    by_depth = k_blocks // 5
+    by_bytes = int(0.15 * k / max(m, 1))
+    if m > 64 and tiles >= sms:
+        return 1        # a block a multiprocessor already, and partial sums of many rows cost more than they gain (measured)
+    s = max(1, min(by_blocks, by_depth, by_bytes, 8))
+    if k_blocks // s >= 24 and 4 * s <= by_bytes and 2 * s * tiles <= 4 * sms:
+        s *= 2
+    return s
 
 
 def _labelled(fn):
@@ -248,27 +273,7 @@ class Linear:
         and the device only."""
         if self.k % 8:
             return 1
-        sms = _sm_count(self.env.device)
-        if m > 128:
-            # A few hundred rows: the output has fewer 128 x 256 tiles than the device has
-            # multiprocessors, and each block would stream its share of the weight alone.  The sum over
-            # K is split until the blocks fill one wave (measured at 160 to 1,024 rows: whenever tiles
-            # times splits stays within the multiprocessors the split wins, up to 2.7 times; beyond, it
-            # loses to the kernels for many rows).
-            tiles = ((m + 127) // 128) * ((self.n + 255) // 256)
-            s = min(sms // max(1, tiles), (self.k // 64) // 8, 8)
-            return s if s >= 2 else 1
-        tiles = (self.n + 127) // 128
-        k_blocks = self.k // 64
-        by_blocks = -(-2 * sms // tiles)
-        by_depth = k_blocks // 5
-        by_bytes = int(0.15 * self.k / max(m, 1))
-        if m > 64 and tiles >= sms:
-            return 1        # a block a multiprocessor already, and partial sums of many rows cost more than they gain (measured)
-        s = max(1, min(by_blocks, by_depth, by_bytes, 8))
-        if k_blocks // s >= 24 and 4 * s <= by_bytes and 2 * s * tiles <= 4 * sms:
-            s *= 2
-        return s
+        return _split_rule(self.n, self.k, m, _sm_count(self.env.device))
 
     def _splits_f32(self, x: torch.Tensor, m: int) -> int:
         """The same for the 32-bit product of at most 16 rows, in which a warp streams four weight rows: a
