@@ -150,6 +150,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __shared__ float s_rstd[SCALED ? BN : 1];                // the tokens' 1/RMS
 
     rb::pdl_trigger();
+    if (CS != 0) cluster_arrive_relaxed();   // this block runs: the others may write into its shared memory (waited for below)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int a0 = blockIdx.x * BM;   // first row of the A-side operand in this tile
     const int b0 = blockIdx.y * BN;   // first row of the B-side operand
@@ -253,6 +254,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tc_fence_after();
         const bool aborted = !ok || *(volatile uint32_t*)abort_flag != 0;
         if (!ok && lane == 0) atomicExch(p.status, RB_ERR_TIMEOUT);
+        if (CS != 0) cluster_wait();      // every block of the cluster runs by now: returns at once after a tile's products
         if (SCALED && (CS == 4 || blockIdx.z == 0) && p.row_sumsq != nullptr) {
             // the 1/RMS of this tile's tokens, from the shares the kernel before left
             rb::pdl_wait();
@@ -389,7 +391,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     }
     if (CS != 0) {
-        // every thread of both blocks, whatever happened to it above
+        // every thread of every block, whatever happened to it above (warps 0 and 1 have not waited for the first arrival yet)
+        __syncwarp();
+        if (warp < 2) cluster_wait();
         // what the first round below reads from global memory is requested before the barrier, so that it
         // arrives while the blocks wait for one another (a block is the only writer of its residual rows)
         float first_r = 0.f, first_w = 1.f, first_b = 0.f;

@@ -297,6 +297,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     return r;
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// An arrival that orders no memory: it says only that this CTA runs, which is what a peer has to know before it writes into
+// this CTA's shared memory.  Every thread that arrives waits before it arrives again.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The address of `local` (an address in this CTA's shared memory) in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t local, uint32_t rank) {
