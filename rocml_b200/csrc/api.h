@@ -128,6 +128,7 @@ int rb_rope_table(const int* positions, const float* inv_freq, int T, int half, 
 int rb_gemm_generic(const void* x, int x_dtype, const void* w, int w_dtype, const void* bias, void* out,
                     int out_dtype, int M, int N, int K, long long ldx, long long ldo, int splits,
                     long long split_stride, void* stream);
+int rb_gemm_f32_plan(int M, int N, int K, const int* clusters, int* stretches, int* parts);
 
 // The limit, in clock cycles, of every barrier wait in the tensor-core products (cycles <= 0: the default,
 // about two seconds), and a switch for tests of the give-up path: while it is set a few-token product

@@ -2,19 +2,25 @@
 //
 // 32-bit FMA accumulation, no tensor cores and no reduced-precision mode, for every element
 // type.  It is the matrix product of the true 32-bit path, the fallback for sizes the
-// tcgen05 kernel refuses, and the reference the tcgen05 kernel is tested against.  In the tiled
-// kernel the sum over k runs in ascending order for every output element whatever M is.  It stands
+// tcgen05 kernel refuses, and the reference the tcgen05 kernel is tested against.  It stands
 // where the reference has gemv_f16 / gemm_xwt_f16 (rocml-kernels/kernels/gemv_f16.hip:8-36,
-// gemm_f16.hip:10-41).
+// gemm_f16.hip:10-41).  Three kernels, and in each the order in which a row's products are added
+// depends on the weight's sizes alone: a row's result does not depend on what else is in the batch (up to 16 rows, or 17
+// to any number), so that a prompt in pieces gives the same bits as the whole.
 //
-// Few rows of 32-bit operands (a decode step of the 32-bit path) take a second kernel that is bound
-// by reading the weight once: a warp owns two weight rows and streams them with 16-byte loads, every
-// lane multiplying its slice of k with the same slice of all the step's rows (which a block brings
-// into shared memory tile by tile), and the lanes' sums meet in a shuffle tree.  How k is dealt out over the lanes depends on
-// nothing but k, so a row's result does not depend on what else is in the batch here either.
+// * The tiled kernels take any type, layout and size: k ascending.
+//
+// * Few rows of 32-bit operands (up to 16, a decode step of the 32-bit path) are bound
+//   by reading the weight once: a warp owns two weight rows and streams them with 16-byte loads, every
+//   lane multiplying its slice of k with the same slice of all the step's rows (which a block brings
+//   into shared memory tile by tile), and the lanes' sums meet in a shuffle tree.
+//
+// * More rows of 32-bit operands whose rows start on 16 bytes: tiles in a pipeline, the sum over k in up to eight
+//   stretches that are added as a tree, whether the blocks of a cluster have one each or one block has them all.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "api.h"
+#include <algorithm>
 
 using namespace rb;
 
@@ -179,13 +185,18 @@ gemm_tn_large_kernel(const XT* __restrict__ x, const WT* __restrict__ w, const f
 // large tiles than the device has multiprocessors, and the plain tiles above ran such products at 10 TFLOP/s.
 // So the tiles are lower (32 or 64 rows: 181 rows are 3 x 64, not 2 x 128), and the sum over k is split over the
 // blocks of a thread-block cluster until about two blocks a multiprocessor are at work; the parts meet in shared
-// memory, added in the order of k, so that no partial sums go through global memory and the result is one piece.
+// memory, so that no partial sums go through global memory and the result is one piece.
+// How many parts are best depends on the step's rows, but a row's result must not: k is always cut into the same
+// stretches (`f32_stretches`, by the weight's sizes alone), each is summed from zero, and the sums are added as a balanced tree.  A block
+// has one, two, four or all of them, an aligned subtree; it keeps finished subtrees that wait for their other half in local memory
+// (64 values a thread and level, touched once a stretch).
 // Tiles of 32 k arrive by cp.async in their own layout (rows of 36 floats: eight neighbouring rows' 16-byte groups
 // fall on different banks), three stages deep.  A thread owns 8 x 8 (BM = 64) or 8 x 4 outputs, rows and columns
 // interleaved over the warp so that a warp's 16-byte read is 4 or 8 different groups; a 16-byte group is two
 // pairs of k, and each accumulator is a pair (even k, odd k) fed by the two-FMA instruction, so nothing is
-// packed or transposed anywhere.  At K = 2,048, before and after: 61 x 4,096 162 -> 35 us, 181 x 8,192 372 -> 164 us,
-// 500 x 2,048 304 -> 111 us, 4,096 x 4,096 1,558 -> 1,396 us (49 TFLOP/s); its error against 64 bits falls from 8e-7 to 2..6e-7.
+// packed or transposed anywhere.  At K = 2,048, the plain tiles and these: 64 x 4,096 135 and 34 us, 181 x 8,192 338 and 167,
+// 500 x 2,048 221 and 117, 2,048 x 2,048 398 and 384, 4,096 x 4,096 1,562 and 1,478 (46 TFLOP/s); their error against 64 bits 8e-7 and 2e-7
+// (6e-7 where k is one stretch).  With the order of the additions left to the number of parts the last was 1,397.
 constexpr int FBN = 128, FBK = 32, FLD = FBK + 4, FSTAGES = 3, FTHREADS = 128;
 template <int BM_> struct F32Tile {
     static constexpr int TJ = BM_ == 64 ? 8 : 4;                  // columns a thread
@@ -204,7 +215,7 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 template <int BM_>
 __global__ void __launch_bounds__(FTHREADS, 2)
 gemm_f32_cluster_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
-                        float* __restrict__ out, int M, int N, int K, long long ldx, long long ldo) {
+                        float* __restrict__ out, int M, int N, int K, long long ldx, long long ldo, int stretches) {
     using T = F32Tile<BM_>;
     constexpr int TJ = T::TJ;
     extern __shared__ __align__(16) float fsm[];
@@ -268,44 +279,83 @@ gemm_f32_cluster_kernel(const float* __restrict__ x, const float* __restrict__ w
         for (int j = 0; j < TJ; ++j) acc[i][j] = 0ull;
     wp += (FSTAGES - 1) * FBK; xp += (FSTAGES - 1) * FBK; k_left -= (FSTAGES - 1) * FBK;
     int use = 0, refill = FSTAGES - 1;                            // stages
-    for (int kt = 0; kt < n_kt; ++kt) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
-        __syncthreads();          // tile kt is here, and nobody reads the stage that is refilled next any more
-        if (kt + FSTAGES - 1 < n_kt) {
-            fetch_w(refill, 0);
-            fetch_x(refill, 0);
-            wp += FBK; xp += FBK; k_left -= FBK;
+    const int mine = stretches / parts;                           // stretches of this block: a power of two
+    float4 waiting[3 * 2 * TJ];                                   // finished subtrees of 1, 2 and 4 stretches
+    int local = 0;
+    asm volatile("" : "+r"(local));                               // (an index the compiler cannot see keeps them out of the registers)
+    // The sums of the stretch that just ended with the subtrees that waited for them, 2^levels stretches in all: every load of a
+    // level in flight together, in the registers of the accumulators' other halves.
+    float v[8][TJ];
+    auto join = [&](int levels) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < TJ; ++j)
+                v[i][j] = __uint_as_float((unsigned)acc[i][j]) + __uint_as_float((unsigned)(acc[i][j] >> 32));
+#pragma unroll 1
+        for (int l = 0; l < levels; ++l) {
+            const float4* from = waiting + local + l * 2 * TJ;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TJ; j += 4) {
+                    const float4 f = from[(i * TJ + j) / 4];
+                    v[i][j] = f.x + v[i][j]; v[i][j + 1] = f.y + v[i][j + 1];
+                    v[i][j + 2] = f.z + v[i][j + 2]; v[i][j + 3] = f.w + v[i][j + 3];
+                }
         }
-        commit();                                                 // an empty group at the end keeps the count
-        const float* xs = fsm + use * T::STAGE + (wm + ty) * FLD;
-        const float* ws = fsm + use * T::STAGE + (BM_ + wn + tx) * FLD;
-        use = use + 1 == FSTAGES ? 0 : use + 1;
-        refill = refill + 1 == FSTAGES ? 0 : refill + 1;
+    };
+    int kt = 0;
+    for (int st = 0; ; ++st) {
+        const int kt_end = (int)((long long)(part * mine + st + 1) * kt_total / stretches) - kt0;
+        for (; kt < kt_end; ++kt) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
+            __syncthreads();          // tile kt is here, and nobody reads the stage that is refilled next any more
+            if (kt + FSTAGES - 1 < n_kt) {
+                fetch_w(refill, 0);
+                fetch_x(refill, 0);
+                wp += FBK; xp += FBK; k_left -= FBK;
+            }
+            commit();                                                 // an empty group at the end keeps the count
+            const float* xs = fsm + use * T::STAGE + (wm + ty) * FLD;
+            const float* ws = fsm + use * T::STAGE + (BM_ + wn + tx) * FLD;
+            use = use + 1 == FSTAGES ? 0 : use + 1;
+            refill = refill + 1 == FSTAGES ? 0 : refill + 1;
 #pragma unroll
-        for (int c = 0; c < FBK; c += 4) {
-            ulonglong2 a[8];
+            for (int c = 0; c < FBK; c += 4) {
+                ulonglong2 a[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 4 * FLD + c);
+                for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 4 * FLD + c);
 #pragma unroll
-            for (int j = 0; j < TJ; ++j) {
-                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ws + j * 8 * FLD + c);
+                for (int j = 0; j < TJ; ++j) {
+                    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ws + j * 8 * FLD + c);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i][j] = fma2(a[i].x, b.x, acc[i][j]);
+                    for (int i = 0; i < 8; ++i) acc[i][j] = fma2(a[i].x, b.x, acc[i][j]);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) acc[i][j] = fma2(a[i].y, b.y, acc[i][j]);
+                    for (int i = 0; i < 8; ++i) acc[i][j] = fma2(a[i].y, b.y, acc[i][j]);
+                }
             }
         }
+        if (st == mine - 1) break;
+        const int level = __ffs(~st) - 1;                         // one subtree waits for every trailing one of st
+        join(level);
+        float4* to = waiting + local + level * 2 * TJ;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < TJ; ++j) {
+                if (j % 4 == 0) to[(i * TJ + j) / 4] = make_float4(v[i][j], v[i][j + 1], v[i][j + 2], v[i][j + 3]);
+                acc[i][j] = 0ull;
+            }
     }
     // the finished part goes to this block's shared memory, row by row ...
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
+    join(__ffs(mine) - 1);
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < TJ; ++j) {
-            const float lo = __uint_as_float((unsigned)acc[i][j]), hi = __uint_as_float((unsigned)(acc[i][j] >> 32));
-            fsm[(wm + ty + 4 * i) * FBN + wn + tx + 8 * j] = lo + hi;
-        }
+        for (int j = 0; j < TJ; ++j) fsm[(wm + ty + 4 * i) * FBN + wn + tx + 8 * j] = v[i][j];
     // ... and every block adds and writes its share of the tile, four columns at a time
     if (parts > 1) { sm100::cluster_arrive(); sm100::cluster_wait(); }
     else __syncthreads();
@@ -314,16 +364,20 @@ gemm_f32_cluster_kernel(const float* __restrict__ x, const float* __restrict__ w
         const int r = g / (FBN / 4), c = (g % (FBN / 4)) * 4;
         const int m = m0 + r, n = n0 + c;
         if (m >= M || n >= N) continue;
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        float v[4];
         if (parts > 1) {
             const uint32_t here = (uint32_t)__cvta_generic_to_shared(fsm + g * 4);
-#pragma unroll 1
-            for (int z = 0; z < parts; ++z) {
+            auto of_block = [&](int z) {
                 float4 p;
                 asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
                              : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(sm100::map_to_cta(here, z)) : "memory");
-                v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
-            }
+                return p;
+            };
+            auto add = [](float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); };
+            float4 sum = add(of_block(0), of_block(1));           // the rest of the tree, over the blocks
+            if (parts > 2) sum = add(sum, add(of_block(2), of_block(3)));
+            if (parts > 4) sum = add(sum, add(add(of_block(4), of_block(5)), add(of_block(6), of_block(7))));
+            v[0] = sum.x; v[1] = sum.y; v[2] = sum.z; v[3] = sum.w;
         } else {
             const float4 p = *reinterpret_cast<const float4*>(fsm + g * 4);
             v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w;
@@ -345,24 +399,37 @@ gemm_f32_cluster_kernel(const float* __restrict__ x, const float* __restrict__ w
     if (parts > 1) { sm100::cluster_arrive(); sm100::cluster_wait(); }       // nobody leaves while its part may still be read
 }
 
-// In how many parts the sum over k is split (1 to 8): the cheapest of the parts that leave at least four k tiles each,
-// counted in k tiles: rounds of resident clusters times a part's tiles, with a block's start, end and meeting taken
-// as four tiles.  clusters[p] is asked of the driver: odd sizes leave multiprocessors empty (296 blocks of two,
-// 279 of three, 284 of four, 264 of eight).  A second block on a multiprocessor costs the first nothing (61 x 4,096 on 128
-// blocks and 61 x 8,192 on 256 both take 58 us at K = 2,048), so a round is a round however full it is.
-int f32_parts(long long tiles, int k_tiles, const int* clusters, long long& best_cost) {
+// Into how many stretches k is cut, by the weight alone, each of at least four k tiles (128 k): as many parts as pay where the
+// step's rows are one row of tiles and the weight's column tiles leave the device idle.  61 rows, in 1, 2, 4 and 8 parts:
+// 4,096 x 2,048 124, 84, 59, 34 us; 8,192 x 2,048 125, 106, 62, 66; 12,288 x 2,048 159, 118, 90, 98; 24,576 x 4,096 433, 325, 325, 333;
+// 151,936 x 1,024 469, 466, 510, 572.  A finer cut than the parts costs little: 8,192 x 2,048 and 1,000 rows in one part 725 us with
+// one stretch, 736 with four, 750 with eight.
+int f32_stretches(int N, int k_tiles) {
+    const int columns = (N + FBN - 1) / FBN;
+    int most = columns <= 33 ? 8 : (columns <= 148 ? 4 : (columns <= 296 ? 2 : 1));
+    while (most > 1 && k_tiles / most < 4) most /= 2;
+    return most;
+}
+
+// Over how many blocks the stretches are dealt out: the cheapest of 1, 2, 4, 8, by rounds of resident clusters times a part's k
+// tiles.  clusters[p] is asked of the driver: 296, 148, 71 and 33 on a B200, two blocks a multiprocessor.  A last round that leaves half of
+// the places empty takes 0.6 of a full one, since its blocks have a multiprocessor each; clusters of eight are packed and come
+// closer to their share.  At K = 2,048 in 1, 2, 4 and 8 parts: 2,048 x 2,048 and 2,048 rows (1.7, 3.5, 7.2, 15.5 rounds) 436, 384, 414,
+// 448 us; 2,048 x 2,048 and 320 rows 153, 117, 89, 82; 4,096 x 2,048 and 181 rows 142, 117, 90, 97.
+int f32_parts(long long tiles, int k_tiles, int stretches, const int* clusters) {
     int best = 1;
-    best_cost = -1;
-    for (int p = 1; p <= 8 && (p == 1 || k_tiles / p >= 4); ++p) {
-        if (clusters[p] < 1) continue;
-        const long long cost = (tiles + clusters[p] - 1) / clusters[p] * ((k_tiles + p - 1) / p + 4);
+    long long best_cost = -1;
+    for (int p = 1; p <= stretches; p *= 2) {
+        const long long places = clusters[p];
+        if (places < 1) continue;
+        const long long rest = tiles % places;
+        long long rounds = 10 * (tiles / places);                 // in tenths
+        if (rest > 0) rounds += p < 8 ? (2 * rest <= places ? 6 : 10) : std::min(10ll, 3 + 10 * rest / places);
+        const long long cost = rounds * (4 * ((k_tiles + p - 1) / p) + 4 + p / 8);
         if (best_cost < 0 || cost < best_cost) { best = p; best_cost = cost; }
     }
     return best;
 }
-
-template <typename XT, typename WT, typename OT>
-int launch(const void* x, const void* w, const void* bias, void* out, int M, int N, int K, long long ldx, long long ldo, cudaStream_t s);
 
 template <int BM_>
 int launch_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, long long ldx, long long ldo,
@@ -393,19 +460,13 @@ int launch_f32(const float* x, const float* w, const float* bias, float* out, in
     if (facts.error) return facts.error;
     const long long tiles = (long long)((N + FBN - 1) / FBN) * ((M + BM_ - 1) / BM_);
     const int k_tiles = (K + FBK - 1) / FBK;
-    long long cost;
-    const int parts = f32_parts(tiles, k_tiles, facts.clusters, cost);
-    // The plain 128 x 128 tiles take 1.85 times a round's time; they stay where they need one round and these nearly two
-    // (500 x 8,192 at K = 2,048: 256 tiles against 512; 395 against 410 us).
-    const long long large = (long long)((N + LBN - 1) / LBN) * ((M + LBM - 1) / LBM);
-    if (large <= facts.clusters[1] && 20 * cost > 37ll * k_tiles)
-        return launch<float, float, float>(x, w, bias, out, M, N, K, ldx, ldo, s);
+    const int stretches = f32_stretches(N, k_tiles), parts = f32_parts(tiles, k_tiles, stretches, facts.clusters);
     dim3 grid((N + FBN - 1) / FBN, (M + BM_ - 1) / BM_, parts);
     if (grid.y > 65535) return RB_ERR_BAD_SIZE;
     cudaError_t e = parts > 1 ? launch_clustered(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), dim3(1, 1, parts), F32Tile<BM_>::SMEM, s,
-                                                 x, w, bias, out, M, N, K, ldx, ldo)
+                                                 x, w, bias, out, M, N, K, ldx, ldo, stretches)
                               : rb::launch(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), F32Tile<BM_>::SMEM, s, x, w, bias, out, M, N,
-                                           K, ldx, ldo);
+                                           K, ldx, ldo, stretches);
     if (e != cudaSuccess) return (int)e;
     RB_LAUNCH_CHECK();
     return RB_OK;
@@ -545,6 +606,15 @@ int launch(const void* x, const void* w, const void* bias, void* out, int M, int
     return RB_OK;
 }
 }  // namespace
+
+// How the 32-bit product of more than 16 rows of M x N x K would be cut: into how many stretches of k, over how many blocks, with
+// clusters[p] clusters of p blocks resident at once.  Nothing is launched; for tests and tuning.
+extern "C" int rb_gemm_f32_plan(int M, int N, int K, const int* clusters, int* stretches, int* parts) {
+    const int bm = M <= 32 ? 32 : 64, k_tiles = (K + FBK - 1) / FBK;
+    *stretches = f32_stretches(N, k_tiles);
+    *parts = f32_parts((long long)((N + FBN - 1) / FBN) * ((M + bm - 1) / bm), k_tiles, *stretches, clusters);
+    return RB_OK;
+}
 
 extern "C" int rb_gemm_generic(const void* x, int x_dtype, const void* w, int w_dtype, const void* bias,
                                void* out, int out_dtype, int M, int N, int K, long long ldx, long long ldo,

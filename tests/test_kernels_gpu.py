@@ -345,6 +345,20 @@ def test_gemm_of_more_32_bit_rows_splits_k_over_a_cluster(M, N, K):
         assert torch.isnan(wide[M]).all() and torch.isnan(wide[:M, N:]).all()
 
 
+@pytest.mark.parametrize("N,K", [(66, 4), (130, 260), (4096, 516), (2048, 1024), (8192, 2048), (1000, 4100)])
+def test_a_32_bit_row_does_not_depend_on_the_other_rows(N, K):
+    """From 17 rows on the number of rows decides over how many blocks the sum over k is dealt out, and the tile's height, but
+    not the order in which a row's products are added: the same bits alone, beside others and at another place."""
+    from rocml_b200 import kernels
+    x, w = rnd((2100, K), 1).to(DEV), rnd((N, K), 2).to(DEV)
+    want = torch.empty((2100, N), dtype=torch.float32, device=DEV)
+    kernels.gemm_generic(x, w, want)
+    for first, M in ((0, 17), (5, 32), (300, 33), (64, 61), (1, 181), (1600, 500), (7, 1030)):
+        out = torch.empty((M, N), dtype=torch.float32, device=DEV)
+        kernels.gemm_generic(x[first:first + M], w, out)
+        assert torch.equal(out, want[first:first + M])
+
+
 @pytest.mark.parametrize("M,N,K,S", [(1, 37, 2048, 2), (8, 4096, 4096, 4), (5, 129, 1100, 3), (16, 1001, 12288, 8), (3, 64, 520, 2), (8, 264, 7616, 7)])
 def test_gemm_of_few_32_bit_rows_in_parts_of_k(M, N, K, S):
     """The same product with the sum over K in S parts, each a partial result of its own (the bias in the

@@ -1,5 +1,7 @@
 """How matrix products are split over K and how prompt attention orders its blocks (host-side
 policies; the SM count is given, no GPU)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -61,3 +63,24 @@ def test_prompt_attention_orders_its_blocks_by_what_fits_the_l2_cache():
     assert not kernels.prefill_heads_first(1, 8, 128, 32768)      # 134 MB: one head after another
     assert not kernels.prefill_heads_first(8, 8, 128, 4096)       # eight such sequences: 134 MB
     assert kernels.prefill_heads_first(8, 8, 128, 32768, window=1024)   # a window bounds what a layer reads
+
+
+def f32_plan(m, n, k):
+    clusters = (ctypes.c_int * 9)(0, 296, 148, 93, 71, 55, 46, 39, 33)          # a B200's, for the 64-row tiles
+    out = (ctypes.c_int * 2)()
+    base = ctypes.addressof(out)
+    kernels._lib().rb_gemm_f32_plan(m, n, k, ctypes.addressof(clusters), base, base + 4)
+    return out[0], out[1]
+
+
+@pytest.mark.parametrize("n,most", [(65, 8), (4224, 8), (4225, 4), (18944, 4), (18945, 2), (37888, 2), (37889, 1), (151936, 1)])
+def test_a_32_bit_product_cuts_k_by_the_weight_alone_and_deals_the_stretches_out_by_the_rows(n, most):
+    for k, by_k in ((4, 1), (224, 1), (228, 2), (480, 2), (484, 4), (992, 4), (996, 8), (12288, 8)):
+        plans = [f32_plan(m, n, k) for m in (17, 32, 33, 64, 181, 500, 4096)]
+        assert {stretches for stretches, _ in plans} == {min(most, by_k)}
+        assert all(parts in (1, 2, 4, 8) and parts <= stretches for stretches, parts in plans)
+
+
+def test_a_32_bit_product_takes_as_many_parts_as_its_rounds_ask_for():
+    assert [f32_plan(m, 2048, 2048)[1] for m in (61, 320, 500, 2048)] == [8, 8, 2, 2]
+    assert [f32_plan(m, 8192, 2048)[1] for m in (61, 256, 500, 1000)] == [4, 1, 2, 2]
