@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "sm100.cuh"
 #include "api.h"
+#include "per_device.h"
 #include <algorithm>
 
 using namespace rb;
@@ -434,13 +435,16 @@ int f32_parts(long long tiles, int k_tiles, int stretches, const int* clusters) 
 template <int BM_>
 int launch_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, long long ldx, long long ldo,
                cudaStream_t s) {
-    // what the device holds at once, asked once a process (one kind of device)
-    struct Facts { int error = 0, clusters[9] = {}; };
-    static const Facts facts = [] {
-        Facts f;
+    // the kernel's shared-memory allowance and how many clusters of 1, 2, 4 and 8 blocks run at once, once a device
+    struct Facts { int clusters[9]; };
+    static PerDevice<Facts> known;
+    const Facts* facts = nullptr;
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return (int)e;
+    const int error = known.get(dev, &facts, [](Facts& f) {
         auto k = gemm_f32_cluster_kernel<BM_>;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Tile<BM_>::SMEM);
-        for (int p = 1; p <= 8 && e == cudaSuccess; ++p) {
+        for (int p = 1; p <= 8 && e == cudaSuccess; p *= 2) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(8, 1, p);
             cfg.blockDim = dim3(FTHREADS);
@@ -454,13 +458,12 @@ int launch_f32(const float* x, const float* w, const float* bias, float* out, in
             cfg.numAttrs = 1;
             e = cudaOccupancyMaxActiveClusters(&f.clusters[p], k, &cfg);
         }
-        f.error = (int)e;
-        return f;
-    }();
-    if (facts.error) return facts.error;
+        return (int)e;
+    });
+    if (error) return error;
     const long long tiles = (long long)((N + FBN - 1) / FBN) * ((M + BM_ - 1) / BM_);
     const int k_tiles = (K + FBK - 1) / FBK;
-    const int stretches = f32_stretches(N, k_tiles), parts = f32_parts(tiles, k_tiles, stretches, facts.clusters);
+    const int stretches = f32_stretches(N, k_tiles), parts = f32_parts(tiles, k_tiles, stretches, facts->clusters);
     dim3 grid((N + FBN - 1) / FBN, (M + BM_ - 1) / BM_, parts);
     if (grid.y > 65535) return RB_ERR_BAD_SIZE;
     cudaError_t e = parts > 1 ? launch_clustered(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), dim3(1, 1, parts), F32Tile<BM_>::SMEM, s,

@@ -359,6 +359,20 @@ def test_a_32_bit_row_does_not_depend_on_the_other_rows(N, K):
         assert torch.equal(out, want[first:first + M])
 
 
+def test_gemm_of_more_32_bit_rows_runs_on_every_device():
+    """The shared memory that the kernel asks for is allowed on a device at a time."""
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs a second device")
+    from rocml_b200 import kernels
+    for index in range(2):
+        with torch.cuda.device(index):
+            for M in (20, 40):
+                x, w = rnd((M, 256), 1).to(f"cuda:{index}"), rnd((512, 256), 2).to(f"cuda:{index}")
+                out = torch.empty((M, 512), dtype=torch.float32, device=x.device)
+                kernels.gemm_generic(x, w, out)
+                assert (out.cpu().double() - x.cpu().double() @ w.cpu().double().t()).abs().max().item() < 256 * 2.0 ** -24 * 256
+
+
 @pytest.mark.parametrize("M,N,K,S", [(1, 37, 2048, 2), (8, 4096, 4096, 4), (5, 129, 1100, 3), (16, 1001, 12288, 8), (3, 64, 520, 2), (8, 264, 7616, 7)])
 def test_gemm_of_few_32_bit_rows_in_parts_of_k(M, N, K, S):
     """The same product with the sum over K in S parts, each a partial result of its own (the bias in the
