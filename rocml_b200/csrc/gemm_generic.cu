@@ -222,7 +222,9 @@ gemm_f32_cluster_kernel(const float* __restrict__ x, const float* __restrict__ w
     extern __shared__ __align__(16) float fsm[];
     pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m0 = blockIdx.y * BM_, n0 = blockIdx.x * FBN;
+    // (tiles in one extent of the grid, column tiles first: the others end at 65,535, which 4.2 million rows exceed)
+    const int columns = (N + FBN - 1) / FBN;
+    const int m0 = (int)(blockIdx.x / columns) * BM_, n0 = (int)(blockIdx.x % columns) * FBN;
     const int parts = gridDim.z, part = blockIdx.z;               // the cluster spans the whole of z
     const int kt_total = (K + FBK - 1) / FBK;
     const int kt0 = (int)((long long)part * kt_total / parts);
@@ -464,8 +466,8 @@ int launch_f32(const float* x, const float* w, const float* bias, float* out, in
     const long long tiles = (long long)((N + FBN - 1) / FBN) * ((M + BM_ - 1) / BM_);
     const int k_tiles = (K + FBK - 1) / FBK;
     const int stretches = f32_stretches(N, k_tiles), parts = f32_parts(tiles, k_tiles, stretches, facts->clusters);
-    dim3 grid((N + FBN - 1) / FBN, (M + BM_ - 1) / BM_, parts);
-    if (grid.y > 65535) return RB_ERR_BAD_SIZE;
+    if (tiles > 0x7fffffffll) return RB_ERR_BAD_SIZE;
+    dim3 grid((unsigned)tiles, 1, parts);
     cudaError_t e = parts > 1 ? launch_clustered(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), dim3(1, 1, parts), F32Tile<BM_>::SMEM, s,
                                                  x, w, bias, out, M, N, K, ldx, ldo, stretches)
                               : rb::launch(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), F32Tile<BM_>::SMEM, s, x, w, bias, out, M, N,

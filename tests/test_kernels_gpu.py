@@ -359,6 +359,18 @@ def test_a_32_bit_row_does_not_depend_on_the_other_rows(N, K):
         assert torch.equal(out, want[first:first + M])
 
 
+def test_gemm_of_millions_of_32_bit_rows():
+    """More row tiles than one of the grid's smaller extents holds (65,535 of 64 rows)."""
+    from rocml_b200 import kernels
+    M = 64 * 65535 + 33
+    x, w = rnd((M, 4), 1).to(DEV), rnd((66, 4), 2).to(DEV)
+    out = torch.full((M, 66), float("nan"), dtype=torch.float32, device=DEV)
+    kernels.gemm_generic(x, w, out)
+    for rows in (slice(0, 100), slice(64 * 65535 - 50, M)):
+        assert (out[rows].cpu().double() - x[rows].cpu().double() @ w.cpu().double().t()).abs().max().item() < 4 * 2.0 ** -24 * 4 * 25
+    assert not torch.isnan(out).any()
+
+
 def test_gemm_of_more_32_bit_rows_runs_on_every_device():
     """The shared memory that the kernel asks for is allowed on a device at a time."""
     if torch.cuda.device_count() < 2:
