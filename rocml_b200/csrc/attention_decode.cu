@@ -931,8 +931,11 @@ int launch(const void* q, int q_stride, const void* k_cache, const void* v_cache
                                                          max_pages, seq_slot, cu_q, kv_len, nq, nkv, scale, window, keep, sink, \
                                                          n_chunks, ppb, part_acc, part_ml, counters, out, o_stride, pj, B))
     // One block a (sequence, head group), and more of them than three a multiprocessor but no more than four: with one page
-    // in flight instead of two all run at once, where a thin second wave took as long as the first (64 sequences of 17 to 57
-    // keys on 8 heads, 512 blocks on 444 places: 16 steps of 36 layers with their prompts 63.4 -> 61.0 ms).  decode_split sends contexts beyond seven pages another way.
+    // in flight instead of two all run at once, where a thin second wave took as long as the first.  64 sequences on 8
+    // heads, 512 blocks on 444 places, with 43, 168, 231 and 423 keys (one, three, four, seven pages), two pages in flight and one: a step of 4b sizes
+    // 2,937, 3,137, 3,195, 3,558 and 2,786, 2,962, 3,045, 3,318 us, of 0.6b sizes 1,348, 1,516, 1,612, 1,892 and 1,198, 1,373, 1,451, 1,693.  Blocks
+    // of padding count here but leave at once: up to 444 others would rather keep two pages in flight, so the engine
+    // does not pad such a batch beyond one wave.  From eight pages on decode_split sends them another way.
     if constexpr (HD == 128) {
         const long long blocks = (long long)grid.y * grid.z;
         if (fused && !proportional && n_chunks == 1 && g <= 8) {

@@ -45,6 +45,18 @@ def _bucket(n: int, floor: int = 1) -> int:
     return b
 
 
+def _batch_bucket(n: int, ctx: int, waves: Sequence[int]) -> int:
+    """How many sequences a captured decode graph for ``n`` of them and a context of ``ctx`` is sized for: the next power of two, or
+    one of ``waves`` below it that holds them.  With fewer than eight pages decode attention runs a block a (sequence, head
+    group), and its launch does not know which of them are padding: 33 to 55 sequences on 8 heads, which run as one wave,
+    would be taken for the 64 that do not, whose blocks keep one page in flight instead of two (28 layers of 0.6b sizes, 44
+    sequences of 43, 103, 168 and 231 keys padded to 64: 1,226, 1,293, 1,360 and 1,426 us a step, to 55: 1,185, 1,220, 1,266 and 1,326; 36 layers of 4b sizes 2,773 to 2,994 and 2,678 to 2,859)."""
+    b = _bucket(n)
+    if ctx < 8 * 64:
+        b = min([b] + [w for w in waves if n <= w])
+    return b
+
+
 def _ctx_bucket(n: int) -> int:
     """Context length a captured decode graph is sized for: the next multiple of 256 (of 1024 beyond
     4096).  Fine steps matter: decode attention deals its blocks out over the bucket, and blocks
@@ -77,6 +89,13 @@ class Engine:
             model.cache_requirements(), model.reads_cache_of(), max_tokens, max_slots,
             min(model.spec.max_position, max_seq_len or model.spec.max_position), self.env.act_dtype,
             self.device, self.max_step_tokens)
+        # how many sequences run as one wave of the decode attention that can keep two pages in flight (heads of 128 in
+        # bfloat16), for each of the model's counts of key/value heads
+        self._waves = []
+        if self.use_graphs and self.env.act_dtype == torch.bfloat16:
+            from .. import kernels
+            self._waves = sorted({kernels.decode_wave(g.req.n_kv_heads, self.device) for g in self.cache.kv_groups
+                                  if g.req.head_dim == 128})
         self._eager: Dict[Tuple[int, int], BatchBuffers] = {}
         self._graphs: "OrderedDict[Tuple[int, int], dict]" = OrderedDict()
         self.graphs_captured = 0
@@ -279,8 +298,8 @@ class Engine:
 
     def _run_graph(self, packed, host, T, B, W) -> Optional[torch.Tensor]:
         kv_len = packed[4]
-        b_pad = _bucket(B)
         ctx_pad = _ctx_bucket(max(kv_len))
+        b_pad = _batch_bucket(B, ctx_pad, self._waves)
         key = (b_pad, ctx_pad)
         g = self._graphs.get(key)
         if g is None:

@@ -565,6 +565,19 @@ def attention_prefill(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor,
 _sm_count = {}
 
 
+def _decode_slots(device) -> int:
+    """How many blocks of the decode attention kernel run at once: three a multiprocessor."""
+    key = torch.device(device).index or 0
+    if key not in _sm_count:
+        _sm_count[key] = torch.cuda.get_device_properties(key).multi_processor_count
+    return 3 * _sm_count[key]
+
+
+def decode_wave(n_kv_groups: int, device=0) -> int:
+    """How many sequences decode attention runs at once with a block a (sequence, key/value head group)."""
+    return max(1, _decode_slots(device) // max(1, n_kv_groups))
+
+
 def decode_split(n_seqs: int, n_kv_groups: int, n_pages: int, device=0):
     """(blocks per sequence, pages per block) for decode attention.  Three blocks of the kernel fit a
     multiprocessor; the split is the finest that still runs as ONE wave (blocks per sequence times
@@ -575,10 +588,7 @@ def decode_split(n_seqs: int, n_kv_groups: int, n_pages: int, device=0):
     (sequence, head group): see below.  Up to 16 blocks per sequence form a thread-block cluster and
     merge through shared memory, which is so much quicker than through global memory that a finer
     split is always cut back to 16."""
-    key = torch.device(device).index or 0
-    if key not in _sm_count:
-        _sm_count[key] = torch.cuda.get_device_properties(key).multi_processor_count
-    slots = 3 * _sm_count[key]
+    slots = _decode_slots(device)
     pairs = n_seqs * n_kv_groups
     if (4 <= n_seqs <= 256 and n_pages > 64) or \
             (2 <= n_seqs <= 256 and n_pages >= 8 and slots < pairs <= slots + slots // 3):

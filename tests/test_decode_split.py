@@ -2,6 +2,7 @@
 import pytest
 
 from rocml_b200 import kernels
+from rocml_b200.engine.engine import _batch_bucket, _bucket
 
 
 @pytest.fixture(autouse=True)
@@ -48,3 +49,14 @@ def test_one_long_sequence_and_very_many_sequences_keep_the_equal_split():
     assert kernels.decode_split(1, 8, 128) == (16, 8)
     assert kernels.decode_split(3, 8, 500) == (16, 32)    # up to three long sequences: a cluster each
     assert kernels.decode_split(300, 8, 100)[1] > 0
+
+
+def test_a_batch_that_runs_as_one_wave_is_not_padded_beyond_it():
+    wave = kernels.decode_wave(8)
+    assert wave == 55                                     # 440 blocks of 444
+    for n, want in ((1, 1), (32, 32), (33, 55), (55, 55), (56, 64), (64, 64), (65, 128)):
+        assert _batch_bucket(n, 256, [wave]) == want
+        assert _batch_bucket(n, 512, [wave]) == _bucket(n)          # longer contexts share the pages out, live ones alone
+        assert _batch_bucket(n, 256, []) == _bucket(n)
+    assert _batch_bucket(20, 256, [kernels.decode_wave(16), kernels.decode_wave(4)]) == 27
+    assert _batch_bucket(70, 256, [kernels.decode_wave(16), kernels.decode_wave(4)]) == 111
