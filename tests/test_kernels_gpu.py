@@ -244,16 +244,21 @@ def test_gemm_tcgen05_qkv_projection_rotates_and_caches(M, nq, nkv, K, norm, rop
         assert int((kc.float().abs().sum(-1) > 0).sum()) <= seen * nkv     # nothing written elsewhere
 
 
-@pytest.mark.parametrize("M,N,K", [(257, 256, 64), (289, 288, 72), (300, 352, 520), (513, 1056, 128), (1100, 256, 448)])
+@pytest.mark.parametrize("M,N,K", [(257, 256, 64), (289, 288, 72), (300, 352, 520), (513, 1056, 128), (1100, 256, 448),
+                                   (4100, 2592, 64), (4100, 2592, 72), (4100, 2592, 320)])
 @pytest.mark.parametrize("pad", [0, 8, 1])
 def test_gemm_tcgen05_pair_results_leave_whole(M, N, K, pad):
-    """The kernel of CTA pairs hands its results to the copy engine in pieces of 32 rows (float32 and bfloat16, gated, added
-    into what is there), or stores them itself when the rows are off 16 bytes (pad 1): ragged rows and columns, and nothing
-    outside the matrix is touched.  The bounds: bfloat16 results 2^-8 of their size, float32 ones K 2^-24 of the sum of sizes."""
+    """The kernel of CTA pairs hands its results to the copy engine in pieces of 32 rows (float32 and bfloat16, through an
+    activation, gated, added into what is there), or stores them itself when the rows are off 16 bytes (pad 1): ragged rows
+    and columns, and nothing outside the matrix is touched.  The last sizes have 17 x 11 tiles, so that each of 74 pairs takes two
+    or three: both accumulators come round again, a warp's piece of shared memory is written again, and with one, two and
+    five K blocks a tile the ring's first requests reach into the next tiles.  The bounds: bfloat16 results 2^-8 of their
+    size, float32 ones K 2^-24 of the sum of sizes; an activation's slope is below 1.13."""
     from rocml_b200 import kernels
     x, w = rnd((M, K), 1, torch.bfloat16).to(DEV), rnd((N, K), 2, torch.bfloat16).to(DEV)
     bias = rnd((N,), 3).to(DEV)
-    xd, wd, bd = x.cpu().double(), w.cpu().double(), bias.cpu().double()
+    oracle = "cpu" if M < 2000 else DEV              # float64 either way
+    xd, wd, bd = x.to(oracle).double(), w.to(oracle).double(), bias.to(oracle).double()
     want, sizes = xd @ wd.t() + bd, xd.abs() @ wd.abs().t() + bd.abs()
     slack = sizes * (K * 2.0 ** -24)
 
@@ -264,19 +269,51 @@ def test_gemm_tcgen05_pair_results_leave_whole(M, N, K, pad):
     for dtype, rounding in ((torch.float32, 0.0), (torch.bfloat16, 2.0 ** -8)):
         wide, out = frame(N, dtype, 7.0)
         assert kernels.gemm_tcgen05(x, w, out, bias, M)
-        assert ((out.cpu().double() - want).abs() <= slack + want.abs() * rounding + 1e-30).all()
+        assert ((out.to(oracle).double() - want).abs() <= slack + want.abs() * rounding + 1e-30).all()
+        assert (wide[M:] == 7.0).all() and (wide[:, N:] == 7.0).all()
+    for kind, act in (("gelu", torch.nn.functional.gelu), ("silu", torch.nn.functional.silu),
+                      ("gelu_tanh", lambda t: torch.nn.functional.gelu(t, approximate="tanh"))):
+        wide, out = frame(N, torch.bfloat16, 7.0)
+        assert kernels.gemm_tcgen05_act(x, w, out, kind, bias, M)
+        assert ((out.to(oracle).double() - act(want)).abs() <= 1.13 * slack + act(want).abs() * 2.0 ** -8 + 1e-6).all()
         assert (wide[M:] == 7.0).all() and (wide[:, N:] == 7.0).all()
     wide, out = frame(N, torch.float32, 0.5)
     assert kernels.gemm_tcgen05_add(x, w, out, bias, M)
-    assert ((out.cpu().double() - want - 0.5).abs() <= slack + (want.abs() + 1) * 2.0 ** -22).all()
+    assert ((out.to(oracle).double() - want - 0.5).abs() <= slack + (want.abs() + 1) * 2.0 ** -22).all()
     assert (wide[M:] == 0.5).all() and (wide[:, N:] == 0.5).all()
     g, u = (want.reshape(M, N // 32, 2, 16)[:, :, j].reshape(M, N // 2) for j in (0, 1))
     slack_g, slack_u = (slack.reshape(M, N // 32, 2, 16)[:, :, j].reshape(M, N // 2) for j in (0, 1))
     gated = g / (1 + torch.exp(-g)) * u
     wide, out = frame(N // 2, torch.bfloat16, 7.0)
     assert kernels.gemm_tcgen05(x, w, out, bias, M, gated=True)
-    assert ((out.cpu().double() - gated).abs() <= gated.abs() * 2.0 ** -7.9 + 1.1 * u.abs() * slack_g + g.abs() * slack_u + 1e-6).all()
+    assert ((out.to(oracle).double() - gated).abs() <= gated.abs() * 2.0 ** -7.9 + 1.1 * u.abs() * slack_g + g.abs() * slack_u + 1e-6).all()
     assert (wide[M:] == 7.0).all() and (wide[:, N // 2:] == 7.0).all()
+
+
+@pytest.mark.parametrize("K,norm", [(64, True), (136, True), (320, False)])
+def test_gemm_tcgen05_qkv_projection_of_several_tiles_a_pair(K, norm):
+    """4,100 rows and 24 heads are 17 x 12 tiles for 74 pairs: the same bits, in the queries and in the cache, as in pieces of 512
+    rows and one of 516, which are a tile a pair."""
+    from rocml_b200 import kernels
+    M, nq, nkv = 4100, 16, 4
+    x, w = rnd((M, K), 1, torch.bfloat16).to(DEV), rnd(((nq + 2 * nkv) * 128, K), 2, torch.bfloat16, 0.1).to(DEV)
+    qw, kw = ((1 + 0.1 * rnd((128,), s)).to(DEV) if norm else None for s in (3, 4))
+    pos = torch.arange(M, dtype=torch.int32, device=DEV)
+    slot = torch.zeros(M, dtype=torch.int32, device=DEV)
+    table = torch.randperm(65, generator=torch.Generator().manual_seed(5)).to(torch.int32).reshape(1, 65).to(DEV)
+    inv_freq = (1e4 ** (-torch.arange(0, 64, dtype=torch.float64) * 2 / 128)).float().to(DEV)
+    cs = kernels.rope_table(pos, inv_freq, M)
+    got = []
+    for cuts in ([0, M], [*range(0, 3585, 512), M]):
+        q = torch.zeros((M, nq * 128), dtype=torch.bfloat16, device=DEV)
+        kc, vc = (torch.zeros((65, nkv, 64, 128), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        for lo, hi in zip(cuts, cuts[1:]):
+            assert kernels.gemm_tcgen05_qkv_rope(x[lo:hi], w, q[lo:hi], nq, nkv, qw, kw, 1e-6, cs[lo:hi].contiguous(), pos[lo:hi], slot[lo:hi],
+                                                 table, kc, vc)
+        kernels.check_status(DEV)
+        got.append((q, kc, vc))
+    for whole, pieces in zip(*got):
+        assert whole.abs().sum() > 0 and torch.equal(whole, pieces)
 
 
 def test_gemm_tcgen05_refuses_unaligned_k():
@@ -327,10 +364,12 @@ def test_gemm_of_few_32_bit_rows_reads_the_weight_once(M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(17, 65, 4), (17, 2048, 2048), (32, 130, 36), (33, 129, 2044), (61, 4096, 512), (64, 128, 128),
-                                   (65, 67, 132), (181, 2048, 4096), (226, 1000, 2052), (2049, 66, 260)])
+                                   (65, 67, 132), (181, 2048, 4096), (226, 1000, 2052), (2049, 66, 260),
+                                   (17, 65, 132), (32, 130, 260), (32, 130, 1028), (20, 4300, 516), (2500, 2050, 4), (2500, 2050, 68),
+                                   (1030, 2050, 1028)])
 def test_gemm_of_more_32_bit_rows_splits_k_over_a_cluster(M, N, K):
-    """More than 16 rows of 32-bit operands on 16 bytes: tiles of 32 and 64 rows, k in one part up to eight, ragged rows,
-    columns and k, an output whose rows start off 16 bytes, a strided input; nothing outside the result is written.
+    """More than 16 rows of 32-bit operands on 16 bytes: tiles of 32 and 64 rows, of one k tile and more, k in one stretch up to
+    eight, a block each or several a block (the last), ragged rows, columns and k, an output whose rows start off 16 bytes, a strided input; nothing outside the result is written.
     The bound: K products summed in 32 bits are off by at most K 2^-24 of the sum of their sizes; parts and pairs make it less."""
     from rocml_b200 import kernels
     x = rnd((M, K + 4), 1).to(DEV)[:, :K]
