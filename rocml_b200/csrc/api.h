@@ -127,7 +127,7 @@ int rb_rope_table(const int* positions, const float* inv_freq, int T, int half, 
 
 int rb_gemm_generic(const void* x, int x_dtype, const void* w, int w_dtype, const void* bias, void* out,
                     int out_dtype, int M, int N, int K, long long ldx, long long ldo, int splits,
-                    long long split_stride, void* stream);
+                    long long split_stride, int w_ready, void* stream);
 int rb_gemm_f32_plan(int M, int N, int K, const int* clusters, int* stretches, int* parts);
 
 // The limit, in clock cycles, of every barrier wait in the tensor-core products (cycles <= 0: the default,
@@ -137,7 +137,7 @@ int rb_gemm_f32_plan(int M, int N, int K, const int* clusters, int* stretches, i
 void rb_gemm_tcgen05_set_wait(long long cycles, int withhold_first_stage);
 int rb_gemm_tcgen05(const void* x, const void* w, const float* bias, void* out, int out_dtype, int M, int N,
                     int K, long long ldx, long long ldo, int splits, long long split_stride, int stages,
-                    int gated, int* status, void* stream);
+                    int gated, int w_ready, int* status, void* stream);
 
 int rb_gemm_tcgen05_gated_pair(const void* x, const void* w, const float* bias, void* h, int M, int N, int K,
                                long long ldx, long long ldh, const float* row_sumsq, int row_groups,
@@ -152,7 +152,7 @@ int rb_gemm_tcgen05_qkv_rope(const void* x, const void* w, const float* bias, in
                              void* q_out, long long q_ld, void* k_cache, void* v_cache, const int* positions,
                              const int* slot_of_token, const int* block_table, int max_pages, const void* q_norm_w,
                              const void* k_norm_w, int norm_w_f32, float norm_eps, const float* cos_sin, int nq,
-                             int nkv, int stages, int* status, void* stream);
+                             int nkv, int stages, int w_ready, int* status, void* stream);
 
 // The persistent product over tiles of 128 sorted rows, each with the weight of its group (see the definition).
 int rb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, int out_dtype, int R, int N, int K, int groups,
@@ -160,7 +160,7 @@ int rb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, int out_dty
                             float act_limit, float act_alpha, int* status, void* stream);
 
 int rb_gemm_tcgen05_add(const void* x, const void* w, const float* bias, float* resid, int M, int N, int K,
-                        long long ldx, long long ld_resid, int stages, int* status, void* stream);
+                        long long ldx, long long ld_resid, int stages, int w_ready, int* status, void* stream);
 
 int rb_attention_generic(const void* q, int q_stride, void* out, int o_stride, int dtype, const void* k_cache,
                          const void* v_cache, const int* block_table, int max_pages, const int* seq_slot,

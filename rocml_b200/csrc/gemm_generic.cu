@@ -216,7 +216,7 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 template <int BM_>
 __global__ void __launch_bounds__(FTHREADS, 2)
 gemm_f32_cluster_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
-                        float* __restrict__ out, int M, int N, int K, long long ldx, long long ldo, int stretches) {
+                        float* __restrict__ out, int M, int N, int K, long long ldx, long long ldo, int stretches, int w_ready) {
     using T = F32Tile<BM_>;
     constexpr int TJ = T::TJ;
     extern __shared__ __align__(16) float fsm[];
@@ -265,7 +265,7 @@ gemm_f32_cluster_kernel(const float* __restrict__ x, const float* __restrict__ w
         }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
-    // the weight does not depend on the kernel before this one
+    if (!w_ready) pdl_wait();                                     // (else the weight does not depend on the kernel before this one)
 #pragma unroll
     for (int kt = 0; kt < FSTAGES - 1; ++kt)
         if (kt < n_kt) fetch_w(kt, kt);
@@ -436,7 +436,7 @@ int f32_parts(long long tiles, int k_tiles, int stretches, const int* clusters) 
 
 template <int BM_>
 int launch_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, long long ldx, long long ldo,
-               cudaStream_t s) {
+               int w_ready, cudaStream_t s) {
     // the kernel's shared-memory allowance and how many clusters of 1, 2, 4 and 8 blocks run at once, once a device
     struct Facts { int clusters[9]; };
     static PerDevice<Facts> known;
@@ -469,9 +469,9 @@ int launch_f32(const float* x, const float* w, const float* bias, float* out, in
     if (tiles > 0x7fffffffll) return RB_ERR_BAD_SIZE;
     dim3 grid((unsigned)tiles, 1, parts);
     cudaError_t e = parts > 1 ? launch_clustered(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), dim3(1, 1, parts), F32Tile<BM_>::SMEM, s,
-                                                 x, w, bias, out, M, N, K, ldx, ldo, stretches)
+                                                 x, w, bias, out, M, N, K, ldx, ldo, stretches, w_ready)
                               : rb::launch(gemm_f32_cluster_kernel<BM_>, grid, dim3(FTHREADS), F32Tile<BM_>::SMEM, s, x, w, bias, out, M, N,
-                                           K, ldx, ldo, stretches);
+                                           K, ldx, ldo, stretches, w_ready);
     if (e != cudaSuccess) return (int)e;
     RB_LAUNCH_CHECK();
     return RB_OK;
@@ -497,7 +497,7 @@ template <int MT>
 __global__ void __launch_bounds__(MT <= 8 ? 128 : 256)
 gemm_rows_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ out, int M, int N, int K, long long ldx, long long ldo, int k_per_split,
-                     long long split_stride) {
+                     long long split_stride, int w_ready) {
     constexpr int ROWS_NW = MT <= 8 ? 4 : 2;     // weight rows a warp
     constexpr int ROWS_WARPS = ROWS_PER_BLOCK / ROWS_NW;
     constexpr int KT = 256;                      // floats of k a tile
@@ -539,7 +539,8 @@ gemm_rows_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, c
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // the weights do not depend on the kernel before this one: their first tile is requested at once
+    // weights that do not depend on the kernel before this one: their first tile is requested at once
+    if (!w_ready) pdl_wait();
     float4 wv[U][ROWS_NW];
     load_w(wv, k_lo);
     pdl_wait();
@@ -583,11 +584,11 @@ gemm_rows_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, c
 
 template <int MT>
 int launch_rows(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, long long ldx,
-                long long ldo, int splits, long long split_stride, cudaStream_t s) {
+                long long ldo, int splits, long long split_stride, int w_ready, cudaStream_t s) {
     const int k_per_split = ((K + splits - 1) / splits + 255) / 256 * 256;       // a multiple of the kernel's k tile
     // (a part that lies wholly beyond K, which the rounding to tiles can leave, is written as zeros)
     RB_LAUNCH((gemm_rows_f32_kernel<MT>), dim3((N + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, splits), dim3(MT <= 8 ? 128 : 256), 0, s,
-              x, w, bias, out, M, N, K, ldx, ldo, k_per_split, split_stride);
+              x, w, bias, out, M, N, K, ldx, ldo, k_per_split, split_stride, w_ready);
     RB_LAUNCH_CHECK();
     return RB_OK;
 }
@@ -621,9 +622,11 @@ extern "C" int rb_gemm_f32_plan(int M, int N, int K, const int* clusters, int* s
     return RB_OK;
 }
 
+// w_ready != 0: w is not written by kernels that this one follows in the stream, so that its first tiles may be read before
+// they have ended.
 extern "C" int rb_gemm_generic(const void* x, int x_dtype, const void* w, int w_dtype, const void* bias,
                                void* out, int out_dtype, int M, int N, int K, long long ldx, long long ldo,
-                               int splits, long long split_stride, void* stream) {
+                               int splits, long long split_stride, int w_ready, void* stream) {
     if (M <= 0 || N <= 0) return RB_OK;
     if (K <= 0 || splits < 1) return RB_ERR_BAD_SIZE;
     // splits > 1: float32 partial sums over parts of k at out + z * split_stride (bias in part 0), for the 32-bit
@@ -639,16 +642,16 @@ extern "C" int rb_gemm_generic(const void* x, int x_dtype, const void* w, int w_
         if (M <= 16 && K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
             const float *xf = (const float*)x, *wf = (const float*)w, *bf32 = (const float*)bias;
             float* of = (float*)out;
-            if (M <= 1) return launch_rows<1>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, s);
-            if (M <= 2) return launch_rows<2>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, s);
-            if (M <= 4) return launch_rows<4>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, s);
-            if (M <= 8) return launch_rows<8>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, s);
-            return launch_rows<16>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, s);
+            if (M <= 1) return launch_rows<1>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, w_ready, s);
+            if (M <= 2) return launch_rows<2>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, w_ready, s);
+            if (M <= 4) return launch_rows<4>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, w_ready, s);
+            if (M <= 8) return launch_rows<8>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, w_ready, s);
+            return launch_rows<16>(xf, wf, bf32, of, M, N, K, ldx, ldo, splits, split_stride, w_ready, s);
         }
         // more rows, and enough columns to fill a tile's (the same loads); 32 rows a tile while they hold all of them
         if (M > 16 && N > 64 && K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0)
-            return M <= 32 ? launch_f32<32>((const float*)x, (const float*)w, (const float*)bias, (float*)out, M, N, K, ldx, ldo, s)
-                           : launch_f32<64>((const float*)x, (const float*)w, (const float*)bias, (float*)out, M, N, K, ldx, ldo, s);
+            return M <= 32 ? launch_f32<32>((const float*)x, (const float*)w, (const float*)bias, (float*)out, M, N, K, ldx, ldo, w_ready, s)
+                           : launch_f32<64>((const float*)x, (const float*)w, (const float*)bias, (float*)out, M, N, K, ldx, ldo, w_ready, s);
         RB_G(float, float, float);
     }
     if (x_dtype == RB_F32 && w_dtype == RB_BF16 && out_dtype == RB_F32) RB_G(float, bf, float);

@@ -52,6 +52,7 @@ struct Params {
     int* status;
     int stages;                   // depth of the shared-memory ring actually used (<= Cfg::STAGES)
     long long wait_cycles;        // after this many clock cycles a wait on a barrier gives up
+    int w_ready;                  // the weight is complete already: its first tiles are read before the wait for earlier kernels
     int withhold;                 // tests only: the first stage's copies are never issued, so its barrier never completes
     // CS >= 4 (the product is added into the residual stream, see the kernel):
     float* resid;                 // [tokens][features] float32, updated in place
@@ -179,9 +180,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (lane == 0) {
             tma_prefetch_desc(&map_a);
             tma_prefetch_desc(&map_b);
-            // The weights do not depend on the kernel before this one: their first tiles are
+            // Weights that do not depend on the kernel before this one: their first tiles are
             // requested at once, then the predecessor's results are waited for, then the
             // activations' tiles follow.
+            if (!p.w_ready) rb::pdl_wait();
             const int pre = n_kb < S ? n_kb : S;
             // p.withhold (tests only): nothing is requested for the first stage, so nothing is in flight
             // for it and its barrier never completes: the warp that waits for it must give up
@@ -558,6 +560,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
         if (lane == 0) {
             tma_prefetch_desc(&map_a);
             tma_prefetch_desc(&map_b);
+            if (!p.w_ready) rb::pdl_wait();
             long long it = 0;          // K blocks issued so far, over all tiles: the ring's position
             bool ok = true, waited = tile_group != nullptr;
             for (int tile = blockIdx.x; tile < n_total && ok; tile += gridDim.x) {
@@ -796,6 +799,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         tmem_relinquish_pair();
     }
     if (EPI == 2 && warp >= 2 && warp < 6 && p.q_norm_w != nullptr) {
+        if (!p.w_ready) rb::pdl_wait();
         const int i = threadIdx.x - 64;
         for (int j = 0; j < 2; ++j) {
             const void* w = j == 0 ? p.q_norm_w : p.k_norm_w;
@@ -813,7 +817,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (lane == 0) {
             tma_prefetch_desc(&map_a);
             tma_prefetch_desc(&map_b);
-            // the weight does not depend on the kernel before this one: the ring's first tiles of it are sent for at once
+            // a weight that does not depend on the kernel before this one: the ring's first tiles of it are sent for at once
+            if (!p.w_ready) rb::pdl_wait();
             const long long mine = pair < n_total ? (long long)((n_total - 1 - pair) / n_pairs + 1) * n_kb : 0;
             const int pre = mine < S ? (int)mine : S;
             auto a_row = [&](int tile) { return (tile % m_pairs) * 2 * BM + (int)rank * BM; };
@@ -1313,6 +1318,8 @@ int dispatch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, void* out,
 }  // namespace
 
 // out[M, N] (+ splits) = x[M, K] . w[N, K]^T.  x, w bfloat16; out bfloat16 or float32.
+// w_ready != 0: w (with a norm's weights) is not written by kernels that this one follows in the stream, so its first tiles may
+// be read before they have ended; the products for few rows with a gate or a residual of their own always take it so.
 // splits > 1: float32 partial results at out + z * split_stride, bias in split 0.
 // gated: the weight's rows alternate in blocks of 16 between a gate and an up projection; the output
 // is [M, N / 2] = silu(gate) * up (bfloat16, no split).
@@ -1356,7 +1363,7 @@ static int gemm_entry(const void* x, const void* w, const float* bias, void* out
                       int N, int K, long long ldx, long long ldo, int splits, long long split_stride,
                       int stages, int gated, int* status, void* stream, int cluster_split,
                       const ResidualOut* ro = nullptr, const RowScale* rsc = nullptr, const RopeOut* rope = nullptr,
-                      bool accumulate = false) {
+                      bool accumulate = false, bool w_ready = true) {
     if (M <= 0 || N <= 0) return RB_OK;
     if (K <= 0 || splits < 1) return RB_ERR_BAD_SIZE;
     if (K % 8 || ldx % 8 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return RB_ERR_BAD_ALIGN;
@@ -1383,6 +1390,7 @@ static int gemm_entry(const void* x, const void* w, const float* bias, void* out
     p.stages = stages;   // 0: the default of the mode
     p.wait_cycles = g_wait_cycles;
     p.withhold = g_withhold;
+    p.w_ready = w_ready;
     // gated: 0 no; 1 + the activation's kind otherwise (1: silu, 3: gelu in its tanh form, which the kernels for many
     // tokens apply; the few-token kernels know silu only)
     p.tile_group = nullptr; p.group_rows = 0; p.act_kind = gated > 1 ? gated - 1 : 0; p.act_limit = 0.f; p.act_alpha = 1.f;
@@ -1503,9 +1511,9 @@ static int gemm_entry(const void* x, const void* w, const float* bias, void* out
 
 extern "C" int rb_gemm_tcgen05(const void* x, const void* w, const float* bias, void* out, int out_dtype, int M,
                                int N, int K, long long ldx, long long ldo, int splits, long long split_stride,
-                               int stages, int gated, int* status, void* stream) {
+                               int stages, int gated, int w_ready, int* status, void* stream) {
     return gemm_entry(x, w, bias, out, out_dtype, M, N, K, ldx, ldo, splits, split_stride, stages, gated, status,
-                      stream, 0);
+                      stream, 0, nullptr, nullptr, nullptr, false, w_ready != 0);
 }
 
 // resid[M, N] += x[M, K] . w[N, K]^T (+ bias) for more than 256 rows and N >= 256: the product is added
@@ -1513,9 +1521,9 @@ extern "C" int rb_gemm_tcgen05(const void* x, const void* w, const float* bias, 
 // no delta goes through memory.  RB_ERR_BAD_SIZE for other sizes (the caller writes a delta instead),
 // RB_ERR_BAD_ALIGN as rb_gemm_tcgen05.
 extern "C" int rb_gemm_tcgen05_add(const void* x, const void* w, const float* bias, float* resid, int M, int N, int K,
-                                   long long ldx, long long ld_resid, int stages, int* status, void* stream) {
+                                   long long ldx, long long ld_resid, int stages, int w_ready, int* status, void* stream) {
     return gemm_entry(x, w, bias, resid, RB_F32, M, N, K, ldx, ld_resid, 1, 0, stages, 0, status, stream, 0, nullptr,
-                      nullptr, nullptr, true);
+                      nullptr, nullptr, true, w_ready != 0);
 }
 
 // h[M, N / 2] = silu(gate) * up (bfloat16, row stride ldh) for at most 32 rows and a gate/up weight
@@ -1564,11 +1572,11 @@ extern "C" int rb_gemm_tcgen05_qkv_rope(const void* x, const void* w, const floa
                                         const int* positions, const int* slot_of_token, const int* block_table,
                                         int max_pages, const void* q_norm_w, const void* k_norm_w, int norm_w_f32,
                                         float norm_eps, const float* cos_sin, int nq, int nkv, int stages,
-                                        int* status, void* stream) {
+                                        int w_ready, int* status, void* stream) {
     RopeOut rope{q_out, q_ld, k_cache, v_cache, positions, slot_of_token, block_table, max_pages,
                  q_norm_w, k_norm_w, norm_w_f32, norm_eps, cos_sin, nq, nkv};
     return gemm_entry(x, w, bias, nullptr, RB_BF16, M, N, K, ldx, 0, 1, 0, stages, 0, status, stream, 0, nullptr,
-                      nullptr, &rope);
+                      nullptr, &rope, false, w_ready != 0);
 }
 
 
@@ -1589,7 +1597,7 @@ extern "C" int rb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, 
     const int bn = N >= 256 ? 256 : 128;
     Params p;
     p.K = K; p.splits = 1; p.ldo = ldo; p.split_stride = 0; p.bias = nullptr; p.status = status; p.stages = 0;
-    p.wait_cycles = g_wait_cycles; p.withhold = 0;
+    p.wait_cycles = g_wait_cycles; p.withhold = 0; p.w_ready = 1;
     p.a_rows = R; p.b_rows = N;
     p.tile_group = tile_group; p.group_rows = N; p.act_kind = act_kind; p.act_limit = act_limit; p.act_alpha = act_alpha;
     p.row_sumsq = nullptr; p.row_groups = 0; p.row_sumsq_ld = 0; p.row_eps = 0.f; p.row_inv_width = 0.f;

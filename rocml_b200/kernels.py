@@ -133,7 +133,7 @@ def _lib():
                                               _vp, _i, _vp, _vp, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp, _i, _vp,
                                               _vp, _vp, _f, _f, _i, _vp]
         lib.rb_rope_table.argtypes = [_vp, _vp, _i, _i, _f, _vp, _vp]
-        lib.rb_gemm_generic.argtypes = [_vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _ll, _vp]
+        lib.rb_gemm_generic.argtypes = [_vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _ll, _i, _vp]
         lib.rb_gemm_f32_plan.argtypes = [_i, _i, _i, _vp, _vp, _vp]
         lib.rb_attention_generic.argtypes = [_vp, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _i,
                                              _i, _i, _i, _f, _i, _i, _f, _vp, _f, _i, _i, _vp, _vp, _i, _vp]
@@ -150,11 +150,11 @@ def _lib():
                                                   _vp, _i, _i, _i, _i, _f, _i, _i, _i, _vp, _vp, _vp, _vp, _i,
                                                   _i, _f, _vp, _f, _f, _f, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _ll, _ll, _vp]
         lib.rb_sample.argtypes = [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp]
-        lib.rb_gemm_tcgen05.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _ll, _i, _i, _vp, _vp]
-        lib.rb_gemm_tcgen05_add.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _i, _vp, _vp]
+        lib.rb_gemm_tcgen05.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _ll, _i, _i, _i, _vp, _vp]
+        lib.rb_gemm_tcgen05_add.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _i, _i, _vp, _vp]
         lib.rb_gemm_tcgen05_gated_pair.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _vp, _i, _ll, _f, _i, _i, _vp, _vp]
         lib.rb_gemm_tcgen05_qkv_rope.argtypes = [_vp, _vp, _vp, _i, _i, _i, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _i, _vp,
-                                                 _vp, _i, _f, _vp, _i, _i, _i, _vp, _vp]
+                                                 _vp, _i, _f, _vp, _i, _i, _i, _i, _vp, _vp]
         lib.rb_gemm_tcgen05_residual.argtypes = [_vp, _vp, _vp, _i, _i, _i, _ll, _i, _vp, _ll, _vp, _i, _vp, _ll, _vp,
                                                  _ll, _i, _vp, _vp]
         lib.rb_hold.argtypes = [_ll, _vp]
@@ -414,10 +414,13 @@ def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, n_tokens: int, m
 @_profiled(lambda a, facts: _cost.linear(_rows(a), a["w"].shape[0], a["w"].shape[1], _esz(a["w"]), _esz(a["x"]), _esz(a["out"]),
                                          _n_in(a["out"])))
 def gemm_generic(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                 m: Optional[int] = None):
+                 m: Optional[int] = None, static_w: bool = False):
     """out[M, N] = x[M, K] . w[N, K]^T (+ bias float32 [N]) on the CUDA cores, 32-bit accumulation.
     ``out`` float32 [S, M, N] with S > 1 (32-bit x and w, at most 16 rows): S partial sums over parts of K,
-    to be added in order by the consumer (bias in the first)."""
+    to be added in order by the consumer (bias in the first).
+
+    ``static_w`` (here and in the products below): the weight is a model's, complete before the kernels that are still queued
+    ahead of this one were launched; its first tiles may then be read while those kernels run."""
     M = x.shape[0] if m is None else m
     N, K = w.shape
     splits, split_stride = 1, 0
@@ -435,7 +438,7 @@ def gemm_generic(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Opti
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
         raise KernelError("gemm_generic: bias must be float32 [N]")
     rc = _lib().rb_gemm_generic(_ptr(x), dtype_code(x.dtype), _ptr(w), dtype_code(w.dtype), _ptr(bias), _ptr(out),
-                                dtype_code(out.dtype), M, N, K, x.stride(0), ldo, splits, split_stride, _stream())
+                                dtype_code(out.dtype), M, N, K, x.stride(0), ldo, splits, split_stride, 1 if static_w else 0, _stream())
     _check(rc, "gemm_generic")
 
 
@@ -844,7 +847,7 @@ def set_wait_limit(cycles: int = 0, withhold_first_stage: bool = False) -> None:
 @_profiled(lambda a, facts: (_cost.gated_linear(_rows(a), a["w"].shape[0], a["w"].shape[1], 2, 2, _esz(a["out"])) if a["gated"] else
                          _cost.linear(_rows(a), a["w"].shape[0], a["w"].shape[1], 2, 2, _esz(a["out"]), _n_in(a["out"]))))
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                 m: Optional[int] = None, stages: int = 0, gated: bool = False, act: str = "silu") -> bool:
+                 m: Optional[int] = None, stages: int = 0, gated: bool = False, act: str = "silu", static_w: bool = False) -> bool:
     """out = x . w^T on the tensor cores; x, w bfloat16, out bfloat16 [M, N] or float32 [M, N] or
     float32 [S, M, N] (S partial sums over K, to be added by the consumer).  Returns False when the
     kernel refuses the layout (K or a row stride not a multiple of 8, a pointer off 16 bytes);
@@ -871,7 +874,7 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Opti
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
         raise KernelError("gemm_tcgen05: bias must be float32 [N]")
     rc = _lib().rb_gemm_tcgen05(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), dtype_code(out.dtype), M, N, K, x.stride(0),
-                                ldo, splits, split_stride, stages, (1 + GATED_ACTS[act]) if gated else 0,
+                                ldo, splits, split_stride, stages, (1 + GATED_ACTS[act]) if gated else 0, 1 if static_w else 0,
                                 _ptr(status_word(x.device)), _stream())
     if rc == 10003:
         return False
@@ -891,7 +894,7 @@ def _row_scale(rowscale, m: int, what: str):
 
 @_profiled(lambda a, facts: (a["w"].numel() * 2 + _rows(a) * (a["w"].shape[1] + a["w"].shape[0]) * 2, 2 * _rows(a) * a["w"].numel()))
 def gemm_tcgen05_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: str, bias: Optional[torch.Tensor] = None,
-                     m: Optional[int] = None) -> bool:
+                     m: Optional[int] = None, static_w: bool = False) -> bool:
     """out bfloat16 [M, N] = act(x . w^T (+ bias)) for more than 256 rows and at least 256 features, the activation (see ``unary_act``)
     in the product's epilogue.  False when the kernel does not take the sizes or the layout (use the two kernels)."""
     M = x.shape[0] if m is None else m
@@ -900,7 +903,7 @@ def gemm_tcgen05_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: s
             not w.is_contiguous() or x.shape[1] != K or out.shape[1] != N or out.stride(1) != 1:
         return False
     rc = _lib().rb_gemm_tcgen05(_ptr(x), _ptr(w), _f32vec(bias, N, "gemm_tcgen05_act: bias"), _ptr(out), BF16, M, N, K, x.stride(0),
-                                out.stride(0), 1, 0, 0, -1 - PLAIN_ACTS[act], _ptr(status_word(x.device)), _stream())
+                                out.stride(0), 1, 0, 0, -1 - PLAIN_ACTS[act], 1 if static_w else 0, _ptr(status_word(x.device)), _stream())
     if rc in (10001, 10003):
         return False
     _check(rc, "gemm_tcgen05_act")
@@ -910,13 +913,13 @@ def gemm_tcgen05_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: s
 @_profiled(lambda a, facts: _cost.gated_linear(_rows(a), a["w"].shape[0], a["w"].shape[1], 2, 2, 2))
 def gemm_tcgen05_gated_pair(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor, bias: Optional[torch.Tensor] = None,
                             m: Optional[int] = None, rowscale=None, parts: int = 2) -> bool:
-    """h = silu(gate) * up for at most 32 rows, w's rows alternating in blocks of 16 between gate and
-    up, with the sum over K done in two halves by two blocks that form a thread-block cluster: the
-    second hands its half to the first through shared memory, so no partial sums go through global
-    memory.  h is bfloat16 [M, N / 2].  ``rowscale`` = (sumsq float32 [G, >= M], eps): x's rows are
+    """h = silu(gate) * up for a few rows, w's rows alternating in blocks of 16 between gate and up, the sum over K done by the
+    blocks of a thread-block cluster, which hand their parts over through shared memory, so that no partial sums go
+    through global memory: in two halves (at most 32 rows; the second block hands its half to the first), or with
+    ``parts`` = 4 in four (at most 16 rows; every block finishes a quarter of the outputs).  w is a model's weight, as with
+    ``static_w`` elsewhere.  h is bfloat16 [M, N / 2].  ``rowscale`` = (sumsq float32 [G, >= M], eps): x's rows are
     residual * norm weight, not yet divided by their RMS; column m of sumsq sums to row m's sum of
     squares over K values, and the product is scaled by rsqrt(sum / K + eps) before the bias.
-    ``parts`` = 4 (at most 16 rows): the sum in four parts by clusters of four blocks.
     Returns False when the kernel refuses the sizes or the layout."""
     M = x.shape[0] if m is None else m
     N, K = w.shape
@@ -940,7 +943,7 @@ def gemm_tcgen05_gated_pair(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor, b
 
 @_profiled(lambda a, facts: _cost.linear(_rows(a), a["w"].shape[0], a["w"].shape[1], 2, 2, 4, 1, True))
 def gemm_tcgen05_add(x: torch.Tensor, w: torch.Tensor, resid: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                     m: Optional[int] = None) -> bool:
+                     m: Optional[int] = None, static_w: bool = False) -> bool:
     """resid += x . w^T (+ bias) for many rows (more than 256, N at least 256): the product is added into
     the float32 residual stream in its own epilogue, so no delta goes through memory.  Returns False
     when the kernel refuses the sizes or the layout (write a delta instead)."""
@@ -955,7 +958,7 @@ def gemm_tcgen05_add(x: torch.Tensor, w: torch.Tensor, resid: torch.Tensor, bias
         raise KernelError("gemm_tcgen05_add: bias must be float32 [N]")
     if M <= 256 or N < 256:
         return False
-    rc = _lib().rb_gemm_tcgen05_add(_ptr(x), _ptr(w), _ptr(bias), _ptr(resid), M, N, K, x.stride(0), resid.stride(0), 0,
+    rc = _lib().rb_gemm_tcgen05_add(_ptr(x), _ptr(w), _ptr(bias), _ptr(resid), M, N, K, x.stride(0), resid.stride(0), 0, 1 if static_w else 0,
                                     _ptr(status_word(x.device)), _stream())
     if rc in (10001, 10003):
         return False
@@ -971,7 +974,7 @@ def gemm_tcgen05_residual(x: torch.Tensor, w: torch.Tensor, resid: torch.Tensor,
                           m: Optional[int] = None) -> bool:
     """resid += x . w^T (+ bias) for at most 64 rows, the sum over K in ``splits`` (4, 8, 16) parts by
     the blocks of a thread-block cluster that exchange their parts through shared memory.  For the
-    norm that follows: ``xhat`` bfloat16 [M, N] = resid * next_w (the row's 1/RMS is applied by the
+    norm that follows (w is a model's weight, as with ``static_w`` elsewhere): ``xhat`` bfloat16 [M, N] = resid * next_w (the row's 1/RMS is applied by the
     consumer) and ``sumsq`` float32 [ceil(N / 128) * splits, >= M], whose column m sums to the sum of
     squares of row m.  Returns False when the kernel refuses the sizes or the layout."""
     M = x.shape[0] if m is None else m
@@ -1010,7 +1013,7 @@ def gemm_tcgen05_qkv_rope(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor,
                           cos_sin: Optional[torch.Tensor], positions: torch.Tensor, slot_of_token: torch.Tensor,
                           block_table: Optional[torch.Tensor], k_cache: Optional[torch.Tensor],
                           v_cache: Optional[torch.Tensor], bias: Optional[torch.Tensor] = None,
-                          m: Optional[int] = None) -> bool:
+                          m: Optional[int] = None, static_w: bool = False) -> bool:
     """A prompt's q | k | v projection (more than 256 rows, heads of 128) with the per-head norm, the
     rotation and the cache write done in the product's epilogue: q_out bfloat16 [M, nq * 128] receives the
     queries, the keys and values go into their pages.  w is [(nq + 2 nkv) * 128, K], or [nq * 128, K] for
@@ -1049,7 +1052,7 @@ def gemm_tcgen05_qkv_rope(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor,
         _i32(positions, "positions"), _i32(slot_of_token, "slot_of_token"),
         None if block_table is None else _i32(block_table, "block_table"),
         block_table.shape[1] if block_table is not None else 0, _ptr(q_norm_w), _ptr(k_norm_w), w_f32, float(eps),
-        _ptr(cos_sin), nq, nkv, 0, _ptr(status_word(x.device)), _stream())
+        _ptr(cos_sin), nq, nkv, 0, 1 if static_w else 0, _ptr(status_word(x.device)), _stream())
     if rc in (10001, 10003):
         return False
     _check(rc, "gemm_tcgen05_qkv_rope")

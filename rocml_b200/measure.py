@@ -251,7 +251,7 @@ def micro(which, model=None):
                     out = torch.empty((S, M, N), dtype=torch.float32, device=dev)
                     for stages in (3, 5):
                         it = iter(range(10 ** 9))
-                        us = in_graph(lambda: kernels.gemm_tcgen05(x, ws[next(it) % copies], out, None, M, stages), 4 * copies)
+                        us = in_graph(lambda: kernels.gemm_tcgen05(x, ws[next(it) % copies], out, None, M, stages, static_w=True), 4 * copies)
                         print(f"gemm decode M={M} {name} N={N} K={K} splits={S} stages={stages}: {us:.1f} us "
                               f"{N * K * 2 / us / 1e6:.2f} TB/s", flush=True)
                 del ws
@@ -261,7 +261,7 @@ def micro(which, model=None):
             x = torch.randn(PREFILL_TOKENS, K, device=dev).bfloat16()
             for od in (torch.bfloat16, torch.float32):
                 out = torch.empty((PREFILL_TOKENS, N), dtype=od, device=dev)
-                us = in_graph(lambda: kernels.gemm_tcgen05(x, w, out, None, PREFILL_TOKENS), 10)
+                us = in_graph(lambda: kernels.gemm_tcgen05(x, w, out, None, PREFILL_TOKENS, static_w=True), 10)
                 print(f"gemm prefill M={PREFILL_TOKENS} {name} N={N} K={K} out={str(od)[6:]}: {us:.1f} us "
                       f"{2 * PREFILL_TOKENS * N * K / us / 1e6:.0f} TFLOP/s", flush=True)
         x = torch.randn(PREFILL_TOKENS, H, device=dev).bfloat16()

@@ -478,7 +478,7 @@ class Attention(Mixer):
             if not kernels.gemm_tcgen05_qkv_rope(
                     xn, self.qkv.weight, q, self.nq, self.nkv, self.q_norm_w, self.k_norm_w, self.qk_norm_eps,
                     cos_sin, batch.positions, batch.slot_of_token,
-                    view.block_table, view.k, view.v, self.qkv.bias, T):
+                    view.block_table, view.k, view.v, self.qkv.bias, T, static_w=True):
                 return False
         self.attend(q, out, batch, view, window)
         return True

@@ -167,7 +167,7 @@ class Linear:
         """[M, N / 2] = act(gate(x)) * up(x) in one kernel (needs ``interleave_pairs``; "gelu_tanh" needs more than
         128 rows)."""
         out = torch.empty((m, self.n // 2), dtype=torch.bfloat16, device=x.device)
-        if not kernels.gemm_tcgen05(x, self.weight, out, self.bias, m, gated=True, act=act):
+        if not kernels.gemm_tcgen05(x, self.weight, out, self.bias, m, gated=True, act=act, static_w=True):
             raise KernelError("the gated matrix product refused a layout that interleave_pairs accepted")
         return out
 
@@ -177,7 +177,7 @@ class Linear:
         if not self._tensor_core(x) or self._splits(m) != 1:
             return None
         out = torch.empty((m, self.n), dtype=torch.bfloat16, device=x.device)
-        return out if kernels.gemm_tcgen05_act(x, self.weight, out, act, self.bias, m) else None
+        return out if kernels.gemm_tcgen05_act(x, self.weight, out, act, self.bias, m, static_w=True) else None
 
     @_labelled
     def forward_gated_pair(self, x: torch.Tensor, m: int, rowscale=None) -> Optional[torch.Tensor]:
@@ -231,7 +231,7 @@ class Linear:
         product cannot be done that way (use ``forward_delta``)."""
         if not self._tensor_core(x) or self._splits(m) != 1:
             return False
-        return kernels.gemm_tcgen05_add(x, self.weight, resid, self.bias, m)
+        return kernels.gemm_tcgen05_add(x, self.weight, resid, self.bias, m, static_w=True)
 
     def adopt(self, weight: torch.Tensor) -> None:
         """Use an existing tensor as the weight (a tied head reads the embedding table)."""
@@ -254,9 +254,9 @@ class Linear:
     @_labelled
     def forward(self, x: torch.Tensor, out: torch.Tensor, m: Optional[int] = None) -> torch.Tensor:
         """out[:M] = x[:M] . W^T (+ bias); ``out`` is [M, N] float32 or of x's type."""
-        if self._tensor_core(x) and kernels.gemm_tcgen05(x, self.weight, out, self.bias, m):
+        if self._tensor_core(x) and kernels.gemm_tcgen05(x, self.weight, out, self.bias, m, static_w=True):
             return out
-        kernels.gemm_generic(x, self.weight, out, self.bias, m)
+        kernels.gemm_generic(x, self.weight, out, self.bias, m, static_w=True)
         return out
 
     def _splits(self, m: int) -> int:
@@ -292,14 +292,14 @@ class Linear:
         tc = self._tensor_core(x)
         S = self._splits(m) if tc else self._splits_f32(x, m)
         out = torch.empty((S, m, self.n), dtype=torch.float32, device=x.device)
-        if tc and kernels.gemm_tcgen05(x, self.weight, out, self.bias, m):
+        if tc and kernels.gemm_tcgen05(x, self.weight, out, self.bias, m, static_w=True):
             return out
         if not tc and S > 1:
-            kernels.gemm_generic(x, self.weight, out, self.bias, m)
+            kernels.gemm_generic(x, self.weight, out, self.bias, m, static_w=True)
             return out
         if S > 1:
             out = out[:1]
-        kernels.gemm_generic(x, self.weight, out[0], self.bias, m)
+        kernels.gemm_generic(x, self.weight, out[0], self.bias, m, static_w=True)
         return out
 
     def forward_auto(self, x: torch.Tensor, m: int) -> torch.Tensor:
