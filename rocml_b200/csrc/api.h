@@ -195,7 +195,7 @@ int rb_attention_decode_fused(const float* proj, int n_in, long long in_stride, 
                               int* counters, void* out, int o_stride, int keep, float sink, const float* sinks, float softcap, float temp_coef,
                               float temp_every, int rot_dim, int post_norm,
                               const float* v_first, const float* v_lambda, float* v_keep, const void* gate, int gate_f32,
-                              int gate_n_in, long long gate_in_stride, long long gate_row_stride, void* stream);
+                              int gate_n_in, long long gate_in_stride, long long gate_row_stride, int rows_ready, void* stream);
 
 int rb_attention_merge(const float* part_acc, const float* part_ml, void* out, int o_stride, int dtype,
                        const int* positions, const int* slot_of_token, int T, int nq, int hd, int chunk,

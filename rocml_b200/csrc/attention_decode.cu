@@ -8,9 +8,10 @@
 // keys and 16 values into shared memory with cp.async (16-byte chunks, XOR-swizzled for ldmatrix),
 // computes S = Q K^T, the softmax statistics of its keys and P V, and the warps' results are merged
 // through shared memory.  Then the blocks of one (sequence, head group) merge their partial results,
-// in ascending order of the keys.  Up to 16 of them are launched as one thread-block cluster: each
-// keeps its part in its own shared memory, and after a cluster barrier each merges one slice of the
-// head size, reading the others' parts through distributed shared memory.  More blocks than that
+// in ascending order of the keys.  Up to 16 of them are launched as one thread-block cluster, and each
+// merges one slice of the head size: with up to 8 heads a group the blocks push their parts of it into its shared
+// memory and meet at one cluster barrier; wider groups keep their parts and read one another's between two.  A
+// sequence that one block of the cluster covers needs no merge.  More blocks than that
 // write unnormalised partial results to global memory; a counter per (sequence, head group) tells
 // the last block to arrive, which merges all chunks and writes the output (the counter is left at
 // zero for the next launch).  Softmax is float32, base 2 (exp(x) = exp2(x log2 e)).
@@ -108,6 +109,7 @@ struct Projections {
     // after everything else that happens to it
     float temp_coef, temp_every;
     float softcap;            // > 0: scores become softcap * tanh(score / softcap)
+    int rows_ready;           // the new token's page is complete up to it: those rows are read before the wait
 };
 
 // One head of 128 values by half a warp, so that a block's four warps make eight heads at once: lane i (0 to 15) holds the
@@ -285,8 +287,8 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     pdl_trigger();
     // Everything up to pdl_wait() below may run while the kernels before this one in the stream are
     // still running.  It reads the step's integers (copied to the device before the step's first
-    // kernel) and pages of keys and values that EARLIER steps wrote; the one page of a sequence that
-    // receives this step's token, and the queries, are read after the wait.
+    // kernel) and keys and values that EARLIER steps wrote: the pages below the one that receives this step's token and, with
+    // rows_ready, that page's older rows.  The queries and this step's own key and value come after the wait.
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);        // [16][HD]
     __nv_bfloat16* KVs = Qs + ROWS * HD;                                    // per warp: K [32][HD], V [32][HD]
@@ -397,11 +399,11 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     };
     // Two pages in flight per warp.  A page below the one that holds position `pos` was complete
     // before this step began, so its copies start at once.  So do those of the page that holds `pos` when this
-    // block itself makes the new token's key and value (FQ): its other rows are as old, and the new row is put into
-    // shared memory beside them when it is ready.  Any other page waits for the kernels before this one.
+    // block itself makes the new token's key and value (FQ) and the caller says that the page's other rows are as old
+    // (rows_ready): the new row is put into shared memory beside them when it is ready.  Any other page waits for the kernels before this one.
     const int new_page = pos / CHUNK;
     const bool owner = FQ && pj.write_kv && hc == 0 && page_first <= new_page && new_page <= page_last;
-    const bool patch = owner && new_page < page_first + NB;    // (a block's later pages are copied after their rows were written)
+    const bool patch = owner && pj.rows_ready && new_page < page_first + NB;   // (later pages are copied after their rows were written)
     const bool early0 = page_first < new_page || (patch && page_first == new_page);
     const bool early1 = NB == 1 || page_first + 1 < new_page || (patch && page_first + 1 == new_page);
     const bool idle = CL && page_first > page_last;            // a block of the cluster beyond the sequence
@@ -490,7 +492,9 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
             }
             __syncwarp();
         }
-        // (a page that is neither early nor patched is copied in the loop below, after the barrier that follows)
+        // a page that waited for the kernels before this one and for the new row; a block's later pages are copied in the loop
+        // below, after the barrier that follows
+        if (owner && !pj.rows_ready) __syncthreads();
         if (!early0) issue(page_first, 0, 0);
         if (!early1) issue(page_first + 1, 1, 0);           // commits an empty group beyond page_last
     } else {
@@ -1016,7 +1020,9 @@ extern "C" int rb_attention_decode(const void* q, int q_stride, const void* k_ca
 // With row_sumsq (shares [row_groups][>= T] of the sums of squares of the rows the projection was made
 // from, over row_width values each) the sums are first scaled by rsqrt(sum / row_width + row_eps).
 // keep, sink and gate as in rb_attention_decode; rot_dim, post_norm, v_first, v_lambda, v_keep: see Projections (the rows
-// may be wider than the heads they hold: gate columns follow the values).
+// may be wider than the heads they hold: gate columns follow the values).  rows_ready != 0: the rows below the new token's in its
+// page were not written by kernels that this one follows in the stream, so that they may be read before those have ended
+// (pages below it always are).
 // Returns RB_ERR_BAD_SIZE for other head sizes, RB_ERR_BAD_ALIGN for partial sums off 16 bytes.
 extern "C" int rb_attention_decode_fused(const float* proj, int n_in, long long in_stride, int row_stride,
                                          const void* q_norm_w, const void* k_norm_w, int w_f32, float eps,
@@ -1029,7 +1035,7 @@ extern "C" int rb_attention_decode_fused(const float* proj, int n_in, long long 
                                          int* counters, void* out, int o_stride, int keep, float sink, const float* sinks, float softcap,
                                          float temp_coef, float temp_every, int rot_dim, int post_norm, const float* v_first, const float* v_lambda, float* v_keep,
                                          const void* gate, int gate_f32, int gate_n_in, long long gate_in_stride,
-                                         long long gate_row_stride, void* stream) {
+                                         long long gate_row_stride, int rows_ready, void* stream) {
     if (hd != 128 || proj == nullptr || n_in < 1) return RB_ERR_BAD_SIZE;
     if (((uintptr_t)proj & 15) || (in_stride % 4) || (row_stride % 4) || ((uintptr_t)cos_sin & 15)) return RB_ERR_BAD_ALIGN;
     if (temp_coef != 0.f && !(temp_every > 0.f)) return RB_ERR_BAD_SIZE;
@@ -1050,6 +1056,7 @@ extern "C" int rb_attention_decode_fused(const float* proj, int n_in, long long 
     if (row_sumsq != nullptr && (row_groups < 1 || row_width < 1)) return RB_ERR_BAD_SIZE;
     pj.rot_dim = rot_dim; pj.post_norm = post_norm;
     pj.softcap = softcap;
+    pj.rows_ready = rows_ready;
     pj.sinks = sinks; pj.temp_coef = temp_coef; pj.temp_every = temp_every;
     pj.v_first = v_first; pj.v_lambda = v_lambda; pj.v_keep = v_keep;
     if (gate != nullptr) pj.gate = GateCols{gate, gate_f32, gate_n_in, gate_in_stride, gate_row_stride};

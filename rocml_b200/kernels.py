@@ -148,7 +148,7 @@ def _lib():
         lib.rb_attention_decode_fused.argtypes = [_vp, _i, _ll, _i, _vp, _vp, _i, _f, _vp, _i, _vp, _i, _ll, _f, _i,
                                                   _vp, _vp, _vp, _i, _vp, _vp,
                                                   _vp, _i, _i, _i, _i, _f, _i, _i, _i, _vp, _vp, _vp, _vp, _i,
-                                                  _i, _f, _vp, _f, _f, _f, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _ll, _ll, _vp]
+                                                  _i, _f, _vp, _f, _f, _f, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _ll, _ll, _i, _vp]
         lib.rb_sample.argtypes = [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp]
         lib.rb_gemm_tcgen05.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _ll, _i, _i, _i, _vp, _vp]
         lib.rb_gemm_tcgen05_add.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _i, _i, _vp, _vp]
@@ -687,7 +687,8 @@ def attention_decode_fused(proj: torch.Tensor, out: torch.Tensor, k_cache: torch
                            pages_per_block: int = 1, rowscale=None, row_width: int = 0, keep: int = 0,
                            sink=None, rot_dim: int = 0, post_norm: bool = False,
                            v_first: Optional[torch.Tensor] = None, v_lambda: Optional[torch.Tensor] = None,
-                           v_keep: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, q_temp=None, softcap: float = 0.0) -> bool:
+                           v_keep: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, q_temp=None, softcap: float = 0.0,
+                           static_rows: bool = False) -> bool:
     """attention_decode for head size 128 that takes the step's projections as the matrix product left
     them: ``proj`` float32 [S, T, (nq + 2 nkv) * 128] partial sums (or [T, ...]; only the nq query heads
     when ``write_kv`` is off).  The kernel adds them, applies the per-head norm and the rotation
@@ -700,7 +701,9 @@ def attention_decode_fused(proj: torch.Tensor, out: torch.Tensor, k_cache: torch
     by their root mean square after the rotation; ``v_keep``: float32 [T, nkv * 128], receives the new values as projected;
     ``v_first`` and ``v_lambda`` (float32 [1]): such rows of an earlier layer, blended into what is cached; ``q_temp``
     (coef, every): queries times 1 + coef ln(floor((p + 1) / every) + 1) at position p.  With any
-    of these the rows may hold further columns after the heads.
+    of these the rows may hold further columns after the heads.  ``static_rows``: the cache's rows below the new token's, in
+    its own page too, were complete before the kernels that are still queued ahead of this one were launched, and may be read
+    while those run (the pages below it always are).
     Returns False when the kernel does not take the sizes (use the two kernels)."""
     if hd != 128 or proj.dtype != torch.float32 or k_cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 \
             or out.stride(-1) != 1 or n_seqs * nq > _COUNTER_INTS:
@@ -743,7 +746,7 @@ def attention_decode_fused(proj: torch.Tensor, out: torch.Tensor, k_cache: torch
         int(window), int(n_chunks), int(pages_per_block), _ptr(part_acc), _ptr(part_ml),
         _ptr(decode_counters(out.device)), _ptr(out), out.stride(0), int(keep), *_sink(sink, nq), float(softcap), *_temperature(q_temp), rot, 1 if post_norm else 0,
         _ptr(v_first), _ptr(v_lambda), _ptr(v_keep), _ptr(gate), 1 if gate is not None and gate.dtype == torch.float32 else 0,
-        g_n, g_in, g_row, _stream())
+        g_n, g_in, g_row, 1 if static_rows else 0, _stream())
     if rc in (10001, 10003):
         return False
     _check(rc, "attention_decode_fused")

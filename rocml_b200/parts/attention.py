@@ -513,7 +513,7 @@ class Attention(Mixer):
             self.position.cos_sin(batch) if rot else None, writes, self.scale, window, n_blocks, acc, ml, ppb,
             rowscale=rowscale, row_width=row_width, keep=self.keep_first, sink=self.sink, rot_dim=rot,
             post_norm=self.qk_unit_norm, v_first=v_first, v_lambda=self.v_lambda if v_first is not None else None,
-            v_keep=v_keep, gate=gate, q_temp=self.q_temp, softcap=self.softcap)
+            v_keep=v_keep, gate=gate, q_temp=self.q_temp, softcap=self.softcap, static_rows=True)
 
     def attend(self, q, out, batch, view, window):
         """Softmax attention of the step's queries over the cache (see ``paged_attention``)."""

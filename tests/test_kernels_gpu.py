@@ -965,7 +965,7 @@ def test_attention_decode_takes_the_projections_itself(lens, nq, nkv, window, S,
     ppb, shared_blocks = grid
     n_chunks = shared_blocks if ppb == 0 else ((max(lens) + 63) // 64 + ppb - 1) // ppb
     outs, caches = [], []
-    for fused in (False, True):
+    for fused in (False, True, "rows complete"):
         k2, v2 = kc.clone().to(DEV), vc.clone().to(DEV)
         out = torch.full((B, nq * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
         acc = torch.empty((B, nq, n_chunks, hd), dtype=torch.float32, device=DEV)
@@ -973,7 +973,7 @@ def test_attention_decode_takes_the_projections_itself(lens, nq, nkv, window, S,
         if fused:
             assert kernels.attention_decode_fused(proj, out, k2, v2, d["table"], d["seq_slot"], d["cu_q"], d["kv_len"],
                                                   B, nq, nkv, hd, qw, kw, eps, cs, True, scale, window or 0,
-                                                  n_chunks, acc, ml, ppb)
+                                                  n_chunks, acc, ml, ppb, static_rows=fused == "rows complete")
         else:
             q = torch.empty((B, nq * hd), dtype=torch.bfloat16, device=DEV)
             kernels.qk_norm_rope_cache(proj, q, B, nq, nkv, hd, qw, kw, eps, inv_freq, hd if rope else 0, pos,
@@ -986,6 +986,8 @@ def test_attention_decode_takes_the_projections_itself(lens, nq, nkv, window, S,
     assert torch.isfinite(outs[1]).all()
     assert torch.equal(caches[0][0], caches[1][0]) and torch.equal(caches[0][1], caches[1][1])
     assert (outs[0] - outs[1]).abs().max().item() < 1e-2
+    # the new token's page read before the wait, its new row put beside it, or read after it: the same bits
+    assert torch.equal(outs[1], outs[2]) and torch.equal(caches[1][0], caches[2][0]) and torch.equal(caches[1][1], caches[2][1])
     # float64: the new token's key and value from the summed projections, the other keys from the cache
     import plain_qwen3 as P
     summed = proj.double().sum(0).cpu().reshape(B, nq + 2 * nkv, hd)
