@@ -63,7 +63,8 @@ struct Params {
     long long xhat_ld;
     float* sumsq;                 // [feature groups][tokens]: sums of squares of the new residual rows
     long long sumsq_ld;
-    // CS == 2: the input rows still lack the norm's 1/RMS; it is applied to the product instead
+    // gate/up in a cluster (CS == 2, or CS == 4 with the gate): the input rows still lack the norm's 1/RMS; it is applied to the
+    // product instead
     const float* row_sumsq;       // [row_groups][tokens] shares of the input rows' sums of squares, or null
     int row_groups;
     long long row_sumsq_ld;
@@ -100,13 +101,6 @@ __device__ __forceinline__ void store16(float* dst, const float* v) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
         reinterpret_cast<float4*>(dst)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-}
-__device__ __forceinline__ void load16(const float* src, float* v) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float4 f = reinterpret_cast<const float4*>(src)[i];
-        v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
-    }
 }
 __device__ __forceinline__ void store16(__nv_bfloat16* dst, const float* v) {
     uint32_t w[8];
@@ -972,7 +966,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             };
             if (EPI == 2) {
                 rb::pdl_wait();   // these threads read what an earlier kernel wrote (the angles' table): returns at once by now
-                int slot = -1, pos = 0, page = -1;
+                int slot = -1, pos = 0;
                 if (ar < p.a_rows) { slot = p.slot_of_token[ar]; pos = p.positions[ar]; }
                 const int head = b0 >> 7;                // this half of the tile is one head
                 const int kind = head < p.nq ? 0 : (head < p.nq + p.nkv ? 1 : 2);

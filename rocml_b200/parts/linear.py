@@ -26,9 +26,9 @@ from .base import BuildEnv, DeferredNorm
 
 _SM_COUNT = {}
 
-# The gated pair product (two K halves as a cluster, SiLU where they meet) beats the plain product
-# followed by the activation kernel up to this many rows; its 32-row tiles are slower than the two
-# kernels (51-57 us against 38-40 for a 24,576 x 4,096 weight).
+# The gated product in parts (two or four K parts as a cluster, SiLU where they meet) beats the plain product
+# followed by the activation kernel up to this many rows; in two halves its 32-row tiles are slower than the two
+# kernels (51-57 us against 38-40 for a 24,576 x 4,096 weight), in four it has none.
 GATED_PAIR_MAX_ROWS = 16
 
 
@@ -191,9 +191,12 @@ class Linear:
         return out if kernels.gemm_tcgen05_gated_pair(x, self.weight, out, self.bias, m, rowscale=rowscale, parts=parts) else None
 
     def gated_parts(self, m: int) -> int:
-        """In how many parts ``forward_gated_pair`` would take the sum over K for m rows: two, or four where more would be
-        in flight otherwise (a step of 8 rows and 28 layers with 12,288 x 2,048 weights: 1.42 ms with four partial sums and
-        the activation's kernel, 1.48 in two parts, which are half the blocks, 1.31 in four); 0: not at all."""
+        """In how many parts ``forward_gated_pair`` would take the sum over K for m rows: two, or four where ``_splits`` says three
+        to sixteen; 0: not at all.  Where it says more than four, fewer blocks are in flight than with partial sums, but the norm's and
+        the activation's kernels are gone.  A layer of a captured decode step, 16 layers, one row and sixteen, before (partial
+        sums) and so: 6,144 x 1,024 (three) 29.5 and 31.9 -> 26.6 and 29.2 us, 12,288 x 2,048 (four) 43.0 and 42.8 -> 36.9 and 39.7, 8,704 x
+        2,048 (five) 38.7 and 39.3 -> 33.1 and 36.1, 6,656 x 2,560 (six) 39.0 and 42.5 -> 35.0 and 39.0, 5,760 x 2,560 (seven) 38.1 and 41.3 -> 34.1
+        and 38.3, 2,048 x 5,120 (eight) 57.8 and 60.8 -> 56.1 and 58.9; 5,120 x 4,096 (eight) 47.3 -> 44.4 with one row and even with sixteen."""
         s = self._splits(m)
         if s < 2 or m > GATED_PAIR_MAX_ROWS or self.k <= 64:
             return 0
@@ -205,7 +208,9 @@ class Linear:
         if m > 64 or self.weight is None or self.weight.dtype != torch.bfloat16 or self.k % 8:
             return 0
         # clusters of 8: larger ones leave too few of them resident at once (a cluster needs all its
-        # blocks on neighbouring multiprocessors)
+        # blocks on neighbouring multiprocessors).  Six and seven parts become eight, which keeps the step free of partial sums: a layer
+        # with an output product of 2,048 x 2,048 (six), one row and sixteen, 38.9 and 42.3 -> 36.9 and 39.7 us; with a down product of
+        # 3,072 x 2,048 (six) 38.0 and 42.1 -> 35.3 and 39.5.
         s = self._splits(m)
         s = 8 if s >= 6 else (4 if s >= 4 else 0)
         return s if s and self.k // 64 >= s else 0

@@ -70,8 +70,8 @@ class GatedMLP(FeedForward):
     can_sink = True        # forward() accepts sink=ResidualSink (see parts.base)
 
     def takes_deferred(self, batch) -> bool:
-        """Whether forward() can be handed a DeferredNorm for this step: only the product of two blocks
-        that applies the activation itself also applies the rows' 1/RMS."""
+        """Whether forward() can be handed a DeferredNorm for this step: only the product whose blocks form clusters and
+        apply the activation where their parts meet also applies the rows' 1/RMS."""
         T = batch.n_tokens
         return (self.act == "silu" and self.gate_up.paired and self.gate_up.weight.dtype == torch.bfloat16
                 and self.gate_up.gated_parts(T) > 0)
@@ -90,7 +90,7 @@ class GatedMLP(FeedForward):
             # many tokens: the activation happens in the product's epilogue, hidden behind the next tile
             h = self.gate_up.forward_gated(xn, T, self.act)
         elif h is None and self.gate_up.paired and self.act == "silu":
-            # few tokens, the sum over K in two halves: the activation happens where the halves meet
+            # few tokens, the sum over K in two or four parts: the activation happens where the parts meet
             h = self.gate_up.forward_gated_pair(xn, T)
         if h is None:
             # the product is split over K some other way, so the activation waits for the partial sums
