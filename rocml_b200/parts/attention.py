@@ -52,8 +52,10 @@ from .linear import Linear
 
 # From this many tokens in a step the q | k | v projection normalises, rotates and caches in its own
 # epilogue; from eight times as many if its sum over K is split for want of tiles (the partial sums go to the rotation kernel).
-# Product and rotation kernel against one: 37 and 37 us at 760 tokens of a 4,096 wide model, 87 and 78 at 2,048; 65 and 56 at
-# 2,048 of a 2,560 wide one, 80 and 65 at 4,096 of a 2,048 wide one.
+# Product and rotation kernel against one, microseconds in a graph: 36 and 36 at 760 tokens of a 4,096 wide model, 90 and 80 at 2,048; 62 and 54 at
+# 2,048 of a 2,560 wide one, 70 and 57 at 4,000 of a 2,048 wide one.  Where the tiles are one round or less nothing hides the
+# epilogue (640 tokens of a 1,024 wide model 16 and 19, of a 2,048 wide one 21 and 24), but such a prompt waits for its launches, of which
+# there is one less a layer: whole prompts of 640 tokens, 0.6b sizes 3.9 and 3.5 ms, 1.7b 3.9 and 3.7, 4b 7.3 and 7.2, 8b 11.0 and 10.9.
 PROMPT_FUSED_MIN_TOKENS = 512
 
 # Tensor-name stems by role, unless the spec's ``names`` says otherwise (the defaults are those of
