@@ -281,6 +281,28 @@ def test_prompts_add_into_the_residual_inside_the_products(tmp_path, monkeypatch
     kernels.check_status("cuda:0")
 
 
+def test_a_decode_graph_of_one_wave(tmp_path):
+    """20 sequences on 16 key/value heads of 128 run as one wave of decode attention, 32 would not: their graph is sized for the
+    wave (an odd number of rows, the last ones padding), and its logits are the plain implementation's."""
+    from plain_qwen3 import PlainQwen3
+    from rocml_b200 import Engine, StepEntry, kernels
+    config = {**CONFIGS["E"], "num_attention_heads": 16, "num_key_value_heads": 16}
+    folder = str(tmp_path / "m")
+    write_model(folder, config, seed=71, std=0.05)
+    plain = PlainQwen3(folder, dtype=torch.float64)
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=4096, max_slots=32)
+    ids = [prompt(400 + i, 6 + 11 * i, config["vocab_size"]) for i in range(20)]
+    slots = [eng.new_sequence() for _ in ids]
+    eng.step([StepEntry(s, p[:-4], []) for s, p in zip(slots, ids)])
+    for t in range(-4, 0):
+        got = eng.step([StepEntry(s, [p[t]], [0]) for s, p in zip(slots, ids)])
+        for row, p in zip(got, ids):
+            assert rel_err(row, plain.logits(p)[t]) < TOL["bfloat16"]
+    wave = kernels.decode_wave(16, eng.device)
+    assert list(eng._graphs) == [(wave if 20 <= wave < 32 else 32, 256)]
+    kernels.check_status(eng.device)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_captured_decode_graphs_are_bounded(tmp_path, monkeypatch, dtype):
     """Decode graphs are kept per context bucket; only ``max_graphs`` of them stay, the least recently
