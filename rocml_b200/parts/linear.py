@@ -196,11 +196,18 @@ class Linear:
         the activation's kernels are gone.  A layer of a captured decode step, 16 layers, one row and sixteen, before (partial
         sums) and so: 6,144 x 1,024 (three) 29.5 and 31.9 -> 26.6 and 29.2 us, 12,288 x 2,048 (four) 43.0 and 42.8 -> 36.9 and 39.7, 8,704 x
         2,048 (five) 38.7 and 39.3 -> 33.1 and 36.1, 6,656 x 2,560 (six) 39.0 and 42.5 -> 35.0 and 39.0, 5,760 x 2,560 (seven) 38.1 and 41.3 -> 34.1
-        and 38.3, 2,048 x 5,120 (eight) 57.8 and 60.8 -> 56.1 and 58.9; 5,120 x 4,096 (eight) 47.3 -> 44.4 with one row and even with sixteen."""
+        and 38.3, 2,048 x 5,120 (eight) 57.8 and 60.8 -> 56.1 and 58.9; 5,120 x 4,096 (eight) 47.3 -> 44.4 with one row and even with sixteen.  Behind a norm of its own
+        kernel four parts win less: norm, gate/up and down with one row 2,048 x 4,096 16.4 -> 16.1, 2,048 x 5,120 18.5 -> 18.6, 4,096 x 8,192 28.8 ->
+        28.7; and where fewer than half of the multiprocessors would have a block, each with 24 K blocks or more, partial sums stay:
+        2,048 x 6,144 19.7 against 20.5, 2,048 x 8,192 22.2 against 23.5."""
         s = self._splits(m)
         if s < 2 or m > GATED_PAIR_MAX_ROWS or self.k <= 64:
             return 0
-        return 2 if s == 2 else (4 if self.k // 64 >= 8 else 0)
+        if s == 2:
+            return 2
+        blocks, depth = 4 * ((self.n + 127) // 128), self.k // 64
+        thin = 2 * blocks < _sm_count(self.env.device) and depth >= 4 * 24
+        return 4 if depth >= 8 and not thin else 0
 
     def residual_splits(self, m: int) -> int:
         """In how many parts ``forward_residual`` would split the sum over K for m rows (0: it would not

@@ -67,7 +67,7 @@ def test_prompt_attention_orders_its_blocks_by_what_fits_the_l2_cache():
 
 def test_gate_and_up_meet_in_clusters_of_two_or_four():
     for (n, k), want in (((24576, 4096), 2), ((12288, 2048), 4), ((6144, 1024), 4), ((8704, 2048), 4), ((4096, 2560), 4),
-                         ((24576, 512), 0)):
+                         ((2048, 5120), 4), ((4096, 8192), 4), ((24576, 512), 0), ((2048, 6144), 0), ((2048, 8192), 0)):
         assert [product(n, k).gated_parts(m) for m in (1, 16, 17)] == [want, want, 0]
     assert product(6144, 448).gated_parts(1) == 0          # fewer than two K blocks a part
 
