@@ -24,6 +24,7 @@ from ..cache import SequenceCache
 from ..config import load_model_spec
 from ..errors import CacheError, ConfigError, KernelError, RocmlError
 from ..parts import BuildEnv
+from ..parts.plain import plain_layer
 from ..profile import profiler as _profiler
 from .batch import BatchBuffers, HostBatch, StepBatch, pack_entries
 from .model import Model
@@ -65,12 +66,26 @@ def _ctx_bucket(n: int) -> int:
     return max(step, -(-n // step) * step)
 
 
+# Prompts of at most this many tokens (all sequences of a piece together) are replayed from captured graphs too: their kernels
+# take less time than the host takes to launch them one by one (61 tokens, 28 layers of 1.7b sizes: 256 launches, 4.0 ms on the host, 2.0
+# as a graph).
+PROMPT_GRAPH_TOKENS = 256
+PROMPT_GRAPHS = 4          # how many are kept
+
+
+def _prompt_bucket(n: int) -> int:
+    """How many tokens a captured prompt graph for ``n`` is sized for: the next multiple of 16, of 32 beyond 64, of 64 beyond 128."""
+    step = 16 if n <= 64 else (32 if n <= 128 else 64)
+    return -(-n // step) * step
+
+
 class Engine:
     def __init__(self, model: Model, max_tokens: int, max_slots: Optional[int] = None,
                  max_step_tokens: int = 4096, use_graphs: bool = True, max_seq_len: Optional[int] = None,
                  max_graphs: int = 8):
         """``max_graphs``: how many captured decode graphs are kept (one per batch bucket and context
-        bucket, least recently used dropped first); each holds its own activations and logits."""
+        bucket, least recently used dropped first); each holds its own activations and logits.  (A few graphs of short prompts
+        are kept beside them.)"""
         self.model = model
         self.env = model.env
         self.device = model.env.device
@@ -98,6 +113,9 @@ class Engine:
                                   if g.req.head_dim == 128})
         self._eager: Dict[Tuple[int, int], BatchBuffers] = {}
         self._graphs: "OrderedDict[Tuple[int, int], dict]" = OrderedDict()
+        self._prompt_graphs: "OrderedDict[Tuple[int, ...], dict]" = OrderedDict()
+        # (layers whose prompt kernels take nothing from the host but the step's sizes)
+        self._graph_prompts = self.use_graphs and self.env.act_dtype == torch.bfloat16 and all(plain_layer(b) for b in model.blocks)
         self.graphs_captured = 0
         self._pool = None
         self.launches = 0          # steps issued (sub-steps counted)
@@ -225,7 +243,8 @@ class Engine:
                 for (i, a, b) in piece:
                     self.cache.commit(entries[i].slot, b - a)
                 if logits is not None:
-                    outs.append(logits)
+                    # (a replayed graph's logits live until its next replay, which may be the next piece)
+                    outs.append(logits if len(pieces) == 1 else logits.clone())
             if not outs:
                 return None
             result = outs[0] if len(outs) == 1 else torch.cat(outs, dim=0)
@@ -272,7 +291,12 @@ class Engine:
             with prof.step("decode" if is_decode else "prefill", q_lens, kv_len):
                 return self._run_eager(packed, host, slots, q_lens, T, B, W, is_decode)
         if is_decode and self.use_graphs:
-            return self._run_graph(packed, host, T, B, W)
+            ctx_pad = _ctx_bucket(max(kv_len))
+            b_pad = _batch_bucket(B, ctx_pad, self._waves)
+            return self._run_graph(self._graphs, self.max_graphs, (b_pad, ctx_pad), packed, host, W, (b_pad, b_pad, b_pad, 1, ctx_pad, True))
+        if not is_decode and self._graph_prompts and T <= PROMPT_GRAPH_TOKENS:
+            pads = (_prompt_bucket(T), _bucket(B), _bucket(W) if W else 0, _bucket(max(q_lens), 16), _ctx_bucket(max(kv_len)), False)
+            return self._run_graph(self._prompt_graphs, PROMPT_GRAPHS, pads[:5], packed, host, W, pads)
         return self._run_eager(packed, host, slots, q_lens, T, B, W, is_decode)
 
     def _run_eager(self, packed, host, slots, q_lens, T, B, W, is_decode) -> Optional[torch.Tensor]:
@@ -296,38 +320,39 @@ class Engine:
             seq_slot=buf.seq_slot, cu_q=buf.cu_q, kv_len=buf.kv_len, want_rows=buf.want_rows, host=host,
             capturing=capturing)
 
-    def _run_graph(self, packed, host, T, B, W) -> Optional[torch.Tensor]:
-        kv_len = packed[4]
-        ctx_pad = _ctx_bucket(max(kv_len))
-        b_pad = _batch_bucket(B, ctx_pad, self._waves)
-        key = (b_pad, ctx_pad)
-        g = self._graphs.get(key)
+    def _run_graph(self, graphs, kept: int, key, packed, host, W, pads) -> Optional[torch.Tensor]:
+        """Replay the graph of ``key`` among ``graphs``, of which ``kept`` are kept, after capturing it if need be.  ``pads``: the
+        tokens, sequences and wanted rows that it is sized for, the longest piece of a sequence, the longest sequence, whether it is
+        a step of single tokens."""
+        t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode = pads
+        B = len(host.seq_slots)
+        g = graphs.get(key)
         if g is None:
-            while len(self._graphs) >= self.max_graphs:
+            while len(graphs) >= kept:
                 # the least recently used bucket goes; its memory returns to the graphs' pool.  Work that
                 # is still queued may read it: wait before it is released.
-                _, old = self._graphs.popitem(last=False)
+                _, old = graphs.popitem(last=False)
                 torch.cuda.current_stream().synchronize()
                 if old["graph"] is not None:
                     old["graph"].reset()
                 old.clear()
-            g = {"buffers": BatchBuffers(b_pad, b_pad, b_pad, self.device), "graph": None, "logits": None}
-            self._graphs[key] = g
+            g = {"buffers": BatchBuffers(t_pad, b_pad, w_pad, self.device), "graph": None, "logits": None}
+            graphs[key] = g
         else:
-            self._graphs.move_to_end(key)
+            graphs.move_to_end(key)
         buf: BatchBuffers = g["buffers"]
-        buf.fill(*packed, host.seq_slots, pad_tokens=b_pad, pad_seqs=b_pad, pad_want=b_pad)
+        buf.fill(*packed, host.seq_slots, pad_tokens=t_pad, pad_seqs=b_pad, pad_want=w_pad)
         if self._device_tokens is not None:
             buf.token_ids[:B].copy_(self._device_tokens[:B], non_blocking=True)
         self.last_h2d_bytes = buf.h2d_bytes
         if g["graph"] is None:
             # First use of this bucket: run it plainly (this also loads every kernel), then
             # capture the same launches for the next time.  Capturing executes nothing.
-            batch = self._batch(buf, b_pad, b_pad, b_pad, 1, ctx_pad, True, host)
+            batch = self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, host)
             out = self.model.forward(batch, self.cache)
             torch.cuda.current_stream().synchronize()
             graph = torch.cuda.CUDAGraph()
-            cap = self._batch(buf, b_pad, b_pad, b_pad, 1, ctx_pad, True, None, capturing=True)
+            cap = self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, None, capturing=True)
             from .. import kernels
             before = kernels.launch_count
             with torch.cuda.graph(graph, pool=self._pool):
@@ -337,7 +362,7 @@ class Engine:
             if self._pool is None:
                 self._pool = graph.pool()
             g["graph"] = graph
-            self.graphs_captured += 1
+            self.graphs_captured += is_decode
             return out[:W] if W else None
         g["graph"].replay()
         self.graph_kernel_launches += g["kernels"]
