@@ -16,7 +16,7 @@ from ..cache.requirements import BundleRequirement, KVRequirement
 from ..profile import scope
 from ..config.specs import MixerSpec, ModelSpec
 from ..errors import ConfigError
-from ..parts import BuildEnv, build_block, build_norm, build_position
+from ..parts import BuildEnv, build_block, build_norm, build_position, decode_layers
 from ..parts.linear import Linear
 from ..weights.decl import TensorDecl
 from ..weights.loader import load_tensors
@@ -209,6 +209,9 @@ class Model:
                     x0.copy_(resid)
         pending = None
         sched = self.spec.schedule
+        if decode_layers.takes(self, batch, cache):
+            decode_layers.forward(self, resid, batch, cache)
+            sched = ()
         for i, e in enumerate(sched):
             block = self.blocks[e.layer]
             if e.add_input or e.add_row is not None:

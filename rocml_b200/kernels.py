@@ -134,6 +134,7 @@ def _lib():
                                               _vp, _vp, _f, _f, _i, _vp]
         lib.rb_rope_table.argtypes = [_vp, _vp, _i, _i, _f, _vp, _vp]
         lib.rb_gemm_generic.argtypes = [_vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _ll, _i, _vp]
+        lib.rb_decode_layers.argtypes = [_vp, _vp]
         lib.rb_gemm_f32_plan.argtypes = [_i, _i, _i, _vp, _vp, _vp]
         lib.rb_attention_generic.argtypes = [_vp, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _i,
                                              _i, _i, _i, _f, _i, _i, _f, _vp, _f, _i, _i, _vp, _vp, _i, _vp]
@@ -751,6 +752,88 @@ def attention_decode_fused(proj: torch.Tensor, out: torch.Tensor, k_cache: torch
         return False
     _check(rc, "attention_decode_fused")
     return True
+
+
+class _DecodeLayer(ctypes.Structure):
+    _fields_ = [(n, _vp) for n in ("qkv", "o", "gate_up", "down", "ff_norm", "next_norm", "q_norm", "k_norm", "k", "v")] + \
+        [("ff_eps", _f), ("in_eps", _f)]
+
+
+class _DecodeStep(ctypes.Structure):
+    _fields_ = [(n, _i) for n in ("T", "H", "I", "nq", "nkv", "layers", "splits", "max_pages", "norm_f32", "head_norm_f32", "n_pages")] + \
+        [("head_eps", _f), ("scale", _f)] + \
+        [(n, _vp) for n in ("cos_sin", "seq_slot", "kv_len", "block_table", "first_norm", "resid", "xhat", "sumsq", "qkv", "attn", "h", "part_o",
+                            "part_ml", "counters", "status")] + [("wait_limit", _ll), ("layer", _c.POINTER(_DecodeLayer))]
+
+
+def decode_layers_splits(pairs: int, max_kv_len: int, device) -> int:
+    """In how many parts ``decode_layers`` takes the pages of each of ``pairs`` (sequence, key/value head) pairs: as many as there are
+    blocks for, but at least four pages each (parts are merged through global memory, which costs about what four pages do)."""
+    pages = max(1, -(-max_kv_len // PAGE))
+    sms = torch.cuda.get_device_properties(device).multi_processor_count
+    return max(1, min(sms // pairs, -(-pages // 4)))
+
+
+def decode_layers(resid: torch.Tensor, first_norm: torch.Tensor, layers, nq: int, nkv: int, inter: int, head_eps: float, scale: float,
+                  cos_sin: Optional[torch.Tensor], seq_slot: torch.Tensor, kv_len: torch.Tensor, block_table: torch.Tensor,
+                  splits: int = 1, wait_limit: int = 0) -> None:
+    """All layers of a decode step of at most 16 tokens, one of each sequence, in one persistent kernel (bfloat16 weights and cache,
+    heads of 128).  ``resid`` [T, H] float32 is the residual stream and receives the result; ``first_norm`` [H] the weight of the
+    first layer's first norm.  ``layers``: for each layer (qkv [(nq + 2 nkv) * 128, H], o [H, nq * 128], gate_up [2 * inter, H] (blocks
+    of 16 gate rows and the 16 up rows of the same outputs), down [H, inter], norm behind the mixer, next layer's first norm (None: no
+    such), q norm, k norm (None: no norm), key pages, value pages [pages, nkv, 64, 128], eps of the norm behind the mixer, eps of the norm that
+    made the layer's input).  Row t of the step belongs to sequence t: ``seq_slot`` (-1: nobody's, its stream is left without meaning),
+    ``kv_len`` with the new token, ``block_table`` [slots, pages].  The new keys and values are written to their pages.  ``splits``: parts of
+    a sequence's pages that blocks take.  ``wait_limit``: clock cycles after which a wait gives up and the device's status word says so
+    (0: about two seconds)."""
+    T, H = resid.shape
+    dev = resid.device
+    if not 1 <= T <= 16 or not layers or nkv < 1 or nq % nkv or nq // nkv > 8 or H % 64 or inter % 64:
+        raise KernelError(f"decode_layers: {T} tokens, {len(layers)} layers, {nq} heads on {nkv}, {H} and {inter} wide are not taken")
+    if resid.dtype != torch.float32 or not resid.is_contiguous():
+        raise KernelError("decode_layers: the stream must be contiguous float32 [T, H]")
+    if first_norm.dtype != layers[0][4].dtype or first_norm.numel() != H or not first_norm.is_contiguous():
+        raise KernelError("decode_layers: the first norm's weight must be [H], of the other norms' type")
+    if seq_slot.numel() < T or kv_len.numel() < T or splits < 1:
+        raise KernelError("decode_layers: a slot and a length for every token, and at least one part")
+    if cos_sin is not None and (cos_sin.dtype != torch.float32 or not cos_sin.is_contiguous() or cos_sin.numel() < T * 128):
+        raise KernelError("decode_layers: cos_sin must be float32 [T, 64, 2]")
+    shapes = (((nq + 2 * nkv) * 128, H), (H, nq * 128), (2 * inter, H), (H, inter))
+    p = _DecodeStep()
+    rows = (_DecodeLayer * len(layers))()
+    n_pages = layers[0][8].shape[0]
+    for i, (qkv, o, gate_up, down, ff_norm, next_norm, q_norm, k_norm, k, v, ff_eps, in_eps) in enumerate(layers):
+        for w, shape in zip((qkv, o, gate_up, down), shapes):
+            if w.dtype != torch.bfloat16 or not w.is_contiguous() or tuple(w.shape) != shape:
+                raise KernelError(f"decode_layers: layer {i}: a weight is not contiguous bfloat16 {shape}")
+        for w, n, like in ((ff_norm, H, layers[0][4]), (next_norm, H, layers[0][4]), (q_norm, 128, layers[0][6]), (k_norm, 128, layers[0][6])):
+            if w is not None and (like is None or w.dtype != like.dtype or w.numel() != n or not w.is_contiguous()):
+                raise KernelError(f"decode_layers: layer {i}: a norm weight is not contiguous [{n}] of the first layer's type")
+        if (q_norm is None) != (k_norm is None) or ff_norm is None or (next_norm is None) != (i + 1 == len(layers)):
+            raise KernelError(f"decode_layers: layer {i}: norm weights are missing")
+        for c in (k, v):
+            if c.dtype != torch.bfloat16 or not c.is_contiguous() or tuple(c.shape) != (n_pages, nkv, PAGE, 128):
+                raise KernelError(f"decode_layers: layer {i}: cache must be contiguous bfloat16 [pages, nkv, 64, 128]")
+        L = rows[i]
+        L.qkv, L.o, L.gate_up, L.down, L.ff_norm, L.next_norm = (_ptr(t) for t in (qkv, o, gate_up, down, ff_norm, next_norm))
+        L.q_norm, L.k_norm, L.k, L.v, L.ff_eps, L.in_eps = _ptr(q_norm), _ptr(k_norm), _ptr(k), _ptr(v), ff_eps, in_eps
+    f32, bf16 = dict(dtype=torch.float32, device=dev), dict(dtype=torch.bfloat16, device=dev)
+    xhat, attn, h = torch.empty((T, H), **bf16), torch.empty((T, nq * 128), **bf16), torch.empty((T, inter), **bf16)
+    sumsq, qkv_rows = torch.empty((T, H // 16), **f32), torch.empty((T, (nq + 2 * nkv) * 128), **f32)
+    part_o = part_ml = None
+    if splits > 1:
+        part_o, part_ml = torch.empty((T, nq, splits, 128), **f32), torch.empty((T, nq, splits, 2), **f32)
+    counters = torch.empty(1 + T * nkv, dtype=torch.int32, device=dev)
+    q_norm = layers[0][6]
+    p.T, p.H, p.I, p.nq, p.nkv, p.layers, p.splits, p.max_pages = T, H, inter, nq, nkv, len(layers), splits, block_table.shape[1]
+    p.norm_f32 = 1 if dtype_code(layers[0][4].dtype) == F32 else 0
+    p.head_norm_f32 = 1 if q_norm is not None and dtype_code(q_norm.dtype) == F32 else 0
+    p.n_pages, p.head_eps, p.scale, p.cos_sin = n_pages, head_eps, scale, _ptr(cos_sin)
+    p.seq_slot, p.kv_len, p.block_table = _i32(seq_slot, "seq_slot"), _i32(kv_len, "kv_len"), _i32(block_table, "block_table")
+    p.first_norm, p.resid, p.xhat, p.sumsq, p.qkv, p.attn, p.h = (_ptr(t) for t in (first_norm, resid, xhat, sumsq, qkv_rows, attn, h))
+    p.part_o, p.part_ml, p.counters, p.status = _ptr(part_o), _ptr(part_ml), _ptr(counters), _ptr(status_word(dev))
+    p.wait_limit, p.layer = int(wait_limit), rows
+    _check(_lib().rb_decode_layers(ctypes.byref(p), _stream()), "decode_layers")
 
 
 @_profiled(lambda a, facts: (a["part_acc"].numel() * 4 + a["part_ml"].numel() * 4 + a["n_tokens"] * a["nq"] * a["hd"] * _esz(a["out"]), 0))

@@ -20,6 +20,7 @@ from .mlstm import MatrixLSTM
 from .rglru import RealGatedLRU
 from .side_by_side import SideBySide
 from .block import OutputNormBlock, ParallelBlock, PostNormBlock, PreNormBlock, SandwichNormBlock
+from . import decode_layers  # noqa: F401
 
 __all__ = [
     "BuildEnv", "DeferredNorm", "ResidualSink", "FeedForward", "Mixer", "Norm", "Part", "PositionEncoding", "build_block",
