@@ -43,7 +43,7 @@ using mma_tiles::tile_addr;
 namespace {
 constexpr int CW = 8;                         // warps that compute
 constexpr int CTHREADS = CW * 32;
-constexpr int THREADS = CTHREADS + 32;        // and the producer's
+constexpr int THREADS = CTHREADS + 128;       // and the producer's warpgroup, of which one thread works
 constexpr int UR = 16;                        // weight rows of a unit
 constexpr int KC = 256;                       // values of k of a stage
 constexpr int KB = 64;                        // values of k of a row of 128 bytes, the swizzle's width
@@ -59,8 +59,7 @@ constexpr int MAX_LAYERS = 38;                // of a launch: what its parameter
 constexpr float NEG_BIG = -1e30f;
 constexpr float LOG2E = 1.4426950408889634f;
 static_assert(STAGE == 2 * SK * HD * 2 && STAGES % CW == 0, "a stage holds 16 keys and 16 values");
-template <int NT>
-constexpr int CPW = NT == 1 ? 2 : 1;          // stages a warp takes of a unit: what it holds activations for (64 registers)
+constexpr int CPW = 2;                        // stages a warp takes of a unit: what it holds activations for (64 registers a tile of tokens)
 
 struct LayerPtrs {
     const void *ff_norm, *next_norm;                     // the norm behind the mixer, and the next layer's first (null: none)
@@ -73,11 +72,11 @@ struct LayerPtrs {
 // code once a layer, and what does not fit the instruction caches is fetched anew each time.
 enum { QKV, ATTENTION, OUT, GATED, DOWN, PHASES };
 
-// A phase's shape, worked out by the host.  Its units (items of attention) go to the blocks in turn: `each` to every one and one
+// A phase's shape, worked out by the host.  Its units go to the blocks in turn: `each` to every one and one
 // more to `rest` of them.  A unit's sum over k is taken in `passes` of at most `per` stages, as few as the warps' registers allow; in a
 // pass `warps` warps share a unit, and `units` units are in work at a time (one where there are several passes).
 struct Plan {
-    int each, rest;
+    int each, rest;                           // (attention: its items stay with the same blocks in every layer, see Item)
     int K, stages, passes, per, warps, units;
 };
 
@@ -130,12 +129,14 @@ __device__ __forceinline__ void load_rows(uint32_t dst, const CUtensorMap* map, 
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %3}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(row) : "memory");
 }
+// (Neither these nor what goes between them clobbers memory: the step's facts, which lie in shared memory, are then read once and not
+// again for every load.  They are volatile, as the barriers are, and stay between them.)
 __device__ __forceinline__ void load_if(bool yes, uint4& v, const void* p) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
-                 : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(p), "r"((int)yes) : "memory");
+                 : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(p), "r"((int)yes));
 }
 __device__ __forceinline__ void load_if(bool yes, float& v, const void* p) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.cg.f32 %0, [%1];\n\t}" : "+f"(v) : "l"(p), "r"((int)yes) : "memory");
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.cg.f32 %0, [%1];\n\t}" : "+f"(v) : "l"(p), "r"((int)yes));
 }
 // Where value k of a row of activations lies.  A product's lane (gq, tq) needs words tq (two values) of the eight 16-byte chunks of 64 values
 // as the B operands of four MMAs (the A operands come from ldmatrix, in the weight's own order); stored together, they are two loads.
@@ -181,7 +182,7 @@ static_assert(SMEM<2> <= 227 * 1024, "a block's shared memory");
 struct Walk {
     int stage = 0;
     uint32_t phase = 0;
-    int unit = 0;                             // units and items of the phases so far, modulo the grid
+    int unit = 0;                             // units of the phases so far, modulo the grid
     __device__ void skip(int n) {             // n < STAGES
         stage += n;
         if (stage >= STAGES) { stage -= STAGES; phase ^= 1; }
@@ -227,18 +228,24 @@ struct Waits {
 // The first row of unit u.  Gate | up alternate in blocks of 16 rows: its other eight rows lie 16 further down, in place of 8.
 __device__ __forceinline__ int weight_row(int phase, int u) { return phase == GATED ? (u >> 1) * 32 + (u & 1) * 8 : u * UR; }
 
-// The sequence, key/value head and part of an item of attention (a whole number below 2^20 over a small one: exact in 32-bit)
-__device__ __forceinline__ void decode(const Step& p, int item, int& b, int& head, int& part) {
-    const int pair = (int)(((float)item + 0.5f) * p.inv_T);
-    b = item - pair * p.T;
-    part = p.splits == 1 ? 0 : (int)(((float)pair + 0.5f) * p.inv_nkv);
-    head = pair - part * p.nkv;
-}
-// The pages of a part of a sequence
-__device__ __forceinline__ void part_pages(const Step& p, int pages, int part, int& p0, int& p1) {
-    p0 = 0; p1 = pages;
-    if (p.splits > 1) { p0 = part * pages / p.splits; p1 = (part + 1) * pages / p.splits; }
-}
+// An item of attention: block b has items b, b + grid, .. in every layer.  Sequence, key/value head and part (a whole number below 2^20
+// over a small one: exact in 32-bit), the keys of earlier steps (below 0: nobody's place), and of those this item's: its pages and keys.
+struct Item {
+    int b, head, part, old, p0, p1, key1;
+    template <class S>
+    __device__ void find(const S& s, int item) {
+        const Step& p = s.step;
+        const int pair = (int)(((float)item + 0.5f) * p.inv_T);
+        b = item - pair * p.T;
+        part = p.splits == 1 ? 0 : (int)(((float)pair + 0.5f) * p.inv_nkv);
+        head = pair - part * p.nkv;
+        old = s.slot[b] < 0 ? -1 : s.old[b];
+        const int pages = (max(old, 0) + RB_PAGE - 1) / RB_PAGE;
+        p0 = 0; p1 = pages;
+        if (p.splits > 1) { p0 = part * pages / p.splits; p1 = (part + 1) * pages / p.splits; }
+        key1 = min(max(old, 0), p1 * RB_PAGE);
+    }
+};
 
 // ---- the producer ------------------------------------------------------------------------------------------
 // One thread walks, so that a stage costs a few instructions (a warp in step, with an arrival each: 340 to 460 cycles a stage, which set the
@@ -288,28 +295,24 @@ struct Producer {
                 }
     }
 
-    __device__ void keys(const Step& p, const CUtensorMap* maps, const LayerPtrs& L) {
-        int first;
-        const int mine = w.share(p.plan[ATTENTION], first);
-        if (L.q_norm != nullptr && mine > 0) {
+    __device__ void keys(const Step& p, const CUtensorMap* maps, const LayerPtrs& L, const Item& mine) {
+        const int items = p.T * p.nkv * p.splits;
+        if (L.q_norm != nullptr && (int)blockIdx.x < items) {
             const int half = p.head_norm_f32 ? 256 : 128;
             prefetch(L.q_norm, 0); prefetch(L.q_norm, half); prefetch(L.k_norm, 0); prefetch(L.k_norm, half);
         }
+        Item it = mine;
 #pragma unroll 1
-        for (int n = 0; n < mine; ++n) {
-            int b, head, part;
-            decode(p, first + n * (int)gridDim.x, b, head, part);
-            const int slot = s.slot[b], old = s.old[b];
-            if (slot < 0 || old <= 0) continue;
-            int p0, p1;
-            part_pages(p, (old + RB_PAGE - 1) / RB_PAGE, part, p0, p1);
-            const int* table = p.block_table + (size_t)slot * p.max_pages;
-            int next = p0 < p1 ? table[p0] : 0;
+        for (int item = blockIdx.x; item < items; item += gridDim.x) {
+            if (item != (int)blockIdx.x) it.find(s, item);
+            if (it.old <= 0) continue;
+            const int* table = p.block_table + (size_t)s.slot[it.b] * p.max_pages;
+            int next = it.p0 < it.p1 ? table[it.p0] : 0;
 #pragma unroll 1
-            for (int pg = p0; pg < p1; ++pg) {
-                const int row = (max(next, 0) * p.nkv + head) * RB_PAGE;
-                next = table[min(pg + 1, p1 - 1)];                       // (a page ahead of its use)
-                const int rows = min(RB_PAGE, old - pg * RB_PAGE);
+            for (int pg = it.p0; pg < it.p1; ++pg) {
+                const int row = (max(next, 0) * p.nkv + it.head) * RB_PAGE;
+                next = table[min(pg + 1, it.p1 - 1)];                    // (a page ahead of its use)
+                const int rows = min(RB_PAGE, it.old - pg * RB_PAGE);
 #pragma unroll 1
                 for (int r = 0; r < rows; r += SK) {
                     if (!room()) return;
@@ -323,12 +326,14 @@ struct Producer {
     }
 
     __device__ void run(const Step& p, const Params& params) {
+        Item first;
+        first.find(s, blockIdx.x);
 #pragma unroll 1
         for (int i = 0; i < p.layers * PHASES && !waits.gave_up(); ++i) {
             const LayerPtrs& L = p.layer[i / PHASES];
             const CUtensorMap* maps = params.map[i / PHASES];
             const int phase = i % PHASES;
-            if (phase == ATTENTION) keys(p, maps, L);
+            if (phase == ATTENTION) keys(p, maps, L, first);
             else product(p, maps + phase, L, phase);
         }
         // The last copies land before the block's memory goes, whatever the warps that compute have waited for (a limit of its own:
@@ -370,13 +375,14 @@ struct Compute {
     // go out ahead of the first unit's products, the sums follow behind them.
     struct Squares { float v[NT][8]; };
     __device__ void ask_squares(Squares& q) {
-        const int n = p.H / UR;
+        const int n = p.H / UR, T = p.T;
+        const float* from = p.sumsq + (warp * n + lane);
 #pragma unroll
         for (int i = 0; i < NT; ++i)
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 q.v[i][j] = 0.f;
-                load_if(warp + i * CW < p.T && j * 32 + lane < n, q.v[i][j], p.sumsq + ((warp + i * CW) * n + j * 32 + lane));
+                load_if(warp + i * CW < T && j * 32 + lane < n, q.v[i][j], from + (i * CW * n + j * 32));
             }
     }
     __device__ void row_scales(const Squares& q, float eps) {
@@ -396,54 +402,73 @@ struct Compute {
         }
     }
 
-    // What a unit's sums become.  begin(): by the threads that will have them, ahead of the unit's last stages; finish(): with the sum
-    // of row r and token t, by whole warps (16 rows of two tokens each).
-    struct Epilogue { float before; uint32_t weight; };
-    __device__ void begin(int phase, const void* norm, int u, int t, int r, Epilogue& e) {
-        if (phase != OUT && phase != DOWN) return;
-        e.before = t < p.T ? __ldcg(p.resid + (t * p.H + u * UR + r)) : 0.f;
-        e.weight = norm != nullptr ? bits_any(norm, p.norm_f32, u * UR + r) : 0u;
+    // What a unit's sums become: what the thread of row r and token t needs for that, looked up once a phase.
+    struct Out {
+        int phase, H;
+        bool live, next;           // the token exists; a norm follows
+        const void* norm;          // its weights
+        float* f32;                // QKV: the token's row of the projections, otherwise of the stream
+        __nv_bfloat16* bf16;       // GATED: the token's row of h, otherwise of xhat
+        float* sumsq;
+        float before;
+        uint32_t weight;
+    };
+    __device__ Out output(int phase, const void* norm, int t) {
+        Out o;
+        o.phase = phase; o.H = p.H; o.live = t < p.T; o.next = norm != nullptr; o.norm = norm;
+        o.f32 = phase == QKV ? p.qkv + t * ((p.nq + 2 * p.nkv) * HD) : p.resid + t * p.H;
+        o.bf16 = phase == GATED ? p.h + t * p.I : p.xhat + t * p.H;
+        o.sumsq = p.sumsq + t * (p.H / UR);
+        o.before = 0.f; o.weight = 0u;
+        return o;
     }
-    // x: the stream's new value at row t, column u * 16 + r: kept, and the next norm's rows and sums of squares
-    __device__ void to_stream(const void* norm, int u, int t, int r, float x, float weight, bool keep) {
-        float sq = t < p.T ? x * x : 0.f;
+    // ahead of the unit's last stages
+    __device__ void begin(Out& o, int u, int r) {
+        if (o.phase != OUT && o.phase != DOWN) return;
+        load_if(o.live, o.before, o.f32 + (u * UR + r));
+        if (o.next) o.weight = bits_any(o.norm, p.norm_f32, u * UR + r);
+    }
+    // x: the stream's new value at column u * 16 + r: kept, and the next norm's rows and sums of squares
+    __device__ void to_stream(const Out& o, int u, int r, float x, bool keep) {
+        float sq = x * x;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (t < p.T) {
-            const int at = t * p.H + u * UR + r;
-            if (keep) p.resid[at] = x;
-            if (norm != nullptr) {
-                p.xhat[t * p.H + ordered(u * UR + r)] = __float2bfloat16_rn(x * weight);
-                if (r == 0) p.sumsq[t * (p.H / UR) + u] = sq;
+        for (int d = 8; d > 0; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
+        if (o.live) {
+            if (keep) o.f32[u * UR + r] = x;
+            if (o.next) {
+                o.bf16[ordered(u * UR + r)] = __float2bfloat16_rn(x * value_any(o.weight, p.norm_f32));
+                if (r == 0) o.sumsq[u] = sq;
             }
         }
     }
-    __device__ void finish(int phase, const void* norm, int u, int t, int r, float sum, const Epilogue& e) {
-        if (phase == OUT || phase == DOWN) {
-            to_stream(norm, u, t, r, e.before + sum, value_any(e.weight, p.norm_f32), true);
+    // the sum is there (whole warps: 16 rows of two tokens each)
+    __device__ void finish(const Out& o, int u, int t, int r, float sum) {
+        if (o.phase == OUT || o.phase == DOWN) {
+            to_stream(o, u, r, o.before + sum, true);
             return;
         }
-        const float v = t < p.T ? sum * s.rstd[t] : 0.f;
-        if (phase == QKV) {
-            if (t < p.T) p.qkv[t * ((p.nq + 2 * p.nkv) * HD) + u * UR + r] = v;
+        const float v = sum * s.rstd[t];
+        if (o.phase == QKV) {
+            if (o.live) o.f32[u * UR + r] = v;
         } else {                              // SiLU(gate) * up: rows 0..7 and 8..15 of the unit
             const float up = __shfl_down_sync(0xffffffffu, v, 8, 16);
-            if (r < 8 && t < p.T) p.h[t * p.I + ordered(u * 8 + r)] = __float2bfloat16_rn(silu(v) * up);
+            if (r < 8 && o.live) o.bf16[ordered(u * 8 + r)] = __float2bfloat16_rn(silu(v) * up);
         }
     }
     // The first layer's first norm: the stream's rows times its weight, and their sums of squares
     __device__ void first_rows() {
         const int t = threadIdx.x >> 4, r = threadIdx.x & 15;
+        Out o = output(DOWN, p.first_norm, t);
 #pragma unroll 1
         for (int u = blockIdx.x; u < p.H / UR; u += gridDim.x) {
-            const float x = t < p.T ? p.resid[t * p.H + u * UR + r] : 0.f;
-            to_stream(p.first_norm, u, t, r, x, value_any(bits_any(p.first_norm, p.norm_f32, u * UR + r), p.norm_f32), false);
+            begin(o, u, r);
+            to_stream(o, u, r, o.before, false);
         }
     }
 
     // A product of the step's rows x [T][K] with this block's units.
     __device__ void product(int phase, const __nv_bfloat16* x, float eps, const void* norm) {
-        constexpr int C = CPW<NT>, OUTS = UR * 8 * NT;
+        constexpr int C = CPW, OUTS = UR * 8 * NT, A = NT == 1 ? 4 : 2;
         int first;
         const Plan& ps = p.plan[phase];
         const int mine = w.share(ps, first), K = ps.K;
@@ -451,6 +476,9 @@ struct Compute {
         const int my_unit = warp / ps.warps, my_stage = (warp - my_unit * ps.warps) * C;      // of those in work
         // the lane's row of the four 8 x 8 matrices of a 16 x 16 A operand: rows 0..7 and 8..15 of two neighbouring chunks
         const uint32_t lane_ring = sm100::smem_u32(s.ring[0]) + (lane & 15) * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
+        // who sums what: a thread row r of token t of one of the units in work, and (short sums) of the next but one
+        const int r = threadIdx.x & 15, t = threadIdx.x / UR % (8 * NT);
+        Out out = output(phase, norm, t);
 #pragma unroll 1
         for (int g0 = 0; g0 < mine; g0 += group)
 #pragma unroll 1
@@ -480,16 +508,13 @@ struct Compute {
 #pragma unroll 1
                 for (int i = g0; i < end; i += ps.units) {
                     const int units = min(ps.units, end - i);
-                    // who sums what: a thread row r of token t of one of the units in work, and (short sums) of the next but one
-                    const int r = threadIdx.x & 15, t = threadIdx.x / UR % (8 * NT);
                     int unit = threadIdx.x / OUTS;
-                    Epilogue e;
-                    if (last && unit < units) begin(phase, norm, first + (i + unit) * (int)gridDim.x, t, r, e);
-                    float acc[NT][2][4];
+                    if (last && unit < units) begin(out, first + (i + unit) * (int)gridDim.x, r);
+                    float acc[NT][A][4];                      // A chains of MMAs, added at the end
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) acc[nt][k >> 2][k & 3] = 0.f;
+                        for (int k = 0; k < A * 4; ++k) acc[nt][k >> 2][k & 3] = 0.f;
                     if (my_unit < units) {
                         Walk at = w;
                         at.skip(my_unit * nc + my_stage);
@@ -512,7 +537,7 @@ struct Compute {
 #pragma unroll
                                             for (int nt = 0; nt < NT; ++nt) {
                                                 const uint4 b = B[c * (KC / KB) + (j > 0 ? j - 1 : 0)][nt][k >> 1];
-                                                mma_tiles::mma_bf16(acc[nt][k & 1], m[(j & 1) ^ 1][k], k & 1 ? b.z : b.x, k & 1 ? b.w : b.y);
+                                                mma_tiles::mma_bf16(acc[nt][k % A], m[(j & 1) ^ 1][k], k & 1 ? b.z : b.x, k & 1 ? b.w : b.y);
                                             }
                                 }
                                 __syncwarp();
@@ -523,6 +548,10 @@ struct Compute {
 #pragma unroll
                         for (int nt = 0; nt < NT; ++nt) {
                             float* to = &s.part[turn & 1][warp][nt * 8 + tq * 2][gq];
+#pragma unroll
+                            for (int a = 2; a < A; ++a)
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) acc[nt][a & 1][k] += acc[nt][a][k];
                             to[0] = acc[nt][0][0] + acc[nt][1][0];
                             to[TOK] = acc[nt][0][1] + acc[nt][1][1];
                             to[8] = acc[nt][0][2] + acc[nt][1][2];
@@ -549,8 +578,8 @@ struct Compute {
                         }
                         if (last) {
                             const int u = first + (i + unit) * (int)gridDim.x;
-                            if (unit >= CTHREADS / OUTS) begin(phase, norm, u, t, r, e);
-                            finish(phase, norm, u, t, r, sum, e);
+                            if (unit >= CTHREADS / OUTS) begin(out, u, r);
+                            finish(out, u, t, r, sum);
                         }
                     }
                     ++turn;
@@ -600,25 +629,21 @@ struct Compute {
 
     __device__ static uint2 pack4(const float* v) { return make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3])); }
 
-    __device__ void attention(const LayerPtrs& L) {
-        int first;
-        const int mine = w.share(p.plan[ATTENTION], first);
-        const int g = p.nq / p.nkv, width = (p.nq + 2 * p.nkv) * HD;
+    __device__ void attention(const LayerPtrs& L, const Item& mine, int g) {
+        const int items = p.T * p.nkv * p.splits, width = (p.nq + 2 * p.nkv) * HD;
+        Item it = mine;
 #pragma unroll 1
-        for (int n = 0; n < mine; ++n) {
-            int b, kvh, part;
-            decode(p, first + n * (int)gridDim.x, b, kvh, part);
-            const int slot = s.slot[b], old = s.old[b];                 // keys of earlier steps
-            if (slot < 0 || old < 0) {
+        for (int item = blockIdx.x; item < items; item += gridDim.x) {
+            if (item != (int)blockIdx.x) it.find(s, item);
+            const int b = it.b, kvh = it.head, part = it.part, old = it.old;
+            if (old < 0) {
                 // a place without a sequence: zeros, so that the products behind it stay finite
                 if (part == 0)
 #pragma unroll 1
                     for (int i = threadIdx.x; i < g * HD; i += CTHREADS) p.attn[(b * p.nq + kvh * g) * HD + i] = __float2bfloat16_rn(0.f);
                 continue;
             }
-            int p0, p1;
-            part_pages(p, (old + RB_PAGE - 1) / RB_PAGE, part, p0, p1);
-            const int key0 = p0 * RB_PAGE, key1 = min(old, p1 * RB_PAGE);
+            const int key0 = it.p0 * RB_PAGE, key1 = it.key1;
             const bool owner = part == p.splits - 1;                     // makes the new key and value
             compute_sync();                                             // the item before is done with s.q and s.o
             {
@@ -828,6 +853,9 @@ struct Compute {
     }
 
     __device__ void run() {
+        Item mine;
+        mine.find(s, blockIdx.x);
+        const int g = p.nq / p.nkv;
         if (p.first_norm != nullptr) {
             first_rows();
             meet();
@@ -837,7 +865,7 @@ struct Compute {
             const LayerPtrs& L = p.layer[i / PHASES];
             const int phase = i % PHASES;
             if (phase == ATTENTION) {
-                attention(L);
+                attention(L, mine, g);
             } else {
                 const __nv_bfloat16* x = phase == OUT ? p.attn : (phase == DOWN ? p.h : p.xhat);
                 product(phase, x, phase == QKV ? L.in_eps : L.ff_eps, phase == OUT ? L.ff_norm : L.next_norm);
@@ -875,12 +903,15 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
     for (int i = threadIdx.x; i < (int)sizeof(s.q) / 16; i += THREADS) reinterpret_cast<uint4*>(s.q)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     const Waits waits{&s.abort, s.step.status, s.step.wait_limit};
+    // Registers move to the warps that compute: 12 warps of 168 at launch, 4 of 40 and 8 of 232 from here on.
     if (threadIdx.x >= CTHREADS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (threadIdx.x == CTHREADS) {
             Producer<NT> producer(s, waits);
             producer.run(s.step, params);
         }
     } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
         Compute<NT> compute(s, waits);
         compute.run();
     }
@@ -986,16 +1017,15 @@ extern "C" int rb_decode_layers(const void* step, void* stream) {
     p.attn = static_cast<__nv_bfloat16*>(q.attn); p.h = static_cast<__nv_bfloat16*>(q.h);
     p.part_o = q.part_o; p.part_ml = q.part_ml; p.counters = q.counters; p.status = q.status;
     p.wait_limit = (unsigned)(q.wait_limit > 0 && q.wait_limit < sm100::RB_WAIT_CYCLES ? q.wait_limit : sm100::RB_WAIT_CYCLES);
-    const int work[PHASES] = {(q.nq + 2 * q.nkv) * HD / UR, q.T * q.nkv * q.splits, q.H / UR, 2 * q.I / UR, q.H / UR};
+    const int work[PHASES] = {(q.nq + 2 * q.nkv) * HD / UR, 0, q.H / UR, 2 * q.I / UR, q.H / UR};
     const int inputs[PHASES] = {q.H, KC, q.nq * HD, q.H, q.I};
-    const int a_warp = q.T <= 8 ? CPW<1> : CPW<2>;
     for (int i = 0; i < PHASES; ++i) {
         Plan& a = p.plan[i];
         a.each = work[i] / ready->sms; a.rest = work[i] % ready->sms;
         a.K = inputs[i]; a.stages = (a.K + KC - 1) / KC;
-        a.passes = (a.stages + CW * a_warp - 1) / (CW * a_warp);
+        a.passes = (a.stages + CW * CPW - 1) / (CW * CPW);
         a.per = (a.stages + a.passes - 1) / a.passes;
-        a.warps = (a.per + a_warp - 1) / a_warp;
+        a.warps = (a.per + CPW - 1) / CPW;
         a.units = a.warps > 4 ? 1 : (a.warps > 2 ? 2 : (q.T <= 8 ? 4 : 2));
     }
     const unsigned long long cached = (unsigned long long)q.n_pages * q.nkv * RB_PAGE;

@@ -2,7 +2,7 @@
 
 The kernel stands for the layers of a plain dense decoder: pre-norm blocks of grouped-query attention (heads of 128 with or
 without per-head norm and rotation, every earlier key visible) and a SiLU-gated feed-forward, RMS norms, bfloat16 weights
-without biases, all layers alike.  Any other layer, wider models, several tokens and a step under the profiler (which times the
+without biases, all layers alike.  Any other layer, more than eight tokens and a step under the profiler (which times the
 kernels of a layer one by one) run layer by layer as always.
 """
 from __future__ import annotations
@@ -18,9 +18,11 @@ from .block import _defer_enabled
 from .norm import RMSNorm
 from .plain import plain_layer
 
-# Where the one kernel is the faster one: narrow models, one token (28 layers of 1,024, a step 758 -> 673 us; with 16 tokens 884 and 899).
-MAX_TOKENS = 1
-MAX_HIDDEN = 1024
+# Up to one tile of tokens the one kernel is the faster one: a step before and now, microseconds, 28 layers of 0.6b sizes with 1, 2 and 8
+# sequences 758, 853, 856 -> 677, 791, 769; 1.7b with 1 and 4 1,131, 1,159 -> 942, 1,012, with 8 of 700 to 1,300 tokens 1,281 -> 1,279;
+# 4b with 1 (900 tokens) and 4 2,075, 2,100 -> 2,005, 1,981; 8b with 1 and 8 2,961, 3,099 -> 2,778, 3,083.  A second tile of tokens: 0.6b with 16
+# 884 -> 1,051, 8b 3,537 -> 3,802.
+MAX_TOKENS = 8
 
 
 def enabled() -> bool:
@@ -65,7 +67,7 @@ def _block_fits(block, first, hidden: int) -> bool:
 
 def takes(model, batch, cache) -> bool:
     """Whether this step's layers run as the one kernel."""
-    if not batch.is_decode or model.env.act_dtype != torch.bfloat16 or _profiler.ACTIVE is not None \
+    if not batch.is_decode or batch.n_tokens > MAX_TOKENS or model.env.act_dtype != torch.bfloat16 or _profiler.ACTIVE is not None \
             or not enabled():
         return False
     first = None
@@ -78,8 +80,6 @@ def takes(model, batch, cache) -> bool:
                 or view.group is not cache.views[0].group or view.k.dtype != torch.bfloat16:
             return False
     if first is None:
-        return False
-    if model.hidden > MAX_HIDDEN or batch.n_tokens > MAX_TOKENS:
         return False
     # every block should have a unit (16 rows) of the first product and of gate | up
     sms = torch.cuda.get_device_properties(model.env.device).multi_processor_count

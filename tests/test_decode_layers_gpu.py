@@ -168,7 +168,6 @@ def test_decode_through_the_engine(tmp_path, monkeypatch, graphs):
     narrow for the one kernel always takes."""
     from plain_qwen3 import PlainQwen3
     from rocml_b200 import Engine, StepEntry, kernels
-    from rocml_b200.parts import decode_layers
     config = {**CONFIGS["E"], "use_sliding_window": False, "layer_types": ["full_attention"] * 2, "num_attention_heads": 16,
               "num_key_value_heads": 2, "intermediate_size": 1216}
     folder = str(tmp_path / "m")
@@ -177,7 +176,6 @@ def test_decode_through_the_engine(tmp_path, monkeypatch, graphs):
     calls = []
     real = kernels.decode_layers
     monkeypatch.setattr(kernels, "decode_layers", lambda *a, **k: calls.append(a[0].shape[0]) or real(*a, **k))
-    monkeypatch.setattr(decode_layers, "MAX_TOKENS", 16)
     ids = [prompt(70 + i, n, config["vocab_size"]) for i, n in enumerate((400, 50, 40))]
     starts = [340, 20, 1]
     for on in ("1", "0"):
