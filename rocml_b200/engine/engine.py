@@ -351,12 +351,17 @@ class Engine:
             batch = self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, host)
             out = self.model.forward(batch, self.cache)
             torch.cuda.current_stream().synchronize()
-            graph = torch.cuda.CUDAGraph()
+            graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream(self.device)
             cap = self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, None, capturing=True)
             from .. import kernels
             before = kernels.launch_count
-            with torch.cuda.graph(graph, pool=self._pool):
-                g["logits"] = self.model.forward(cap, self.cache)
+            # (torch.cuda.graph collects garbage and empties the allocator's cache first, which takes longer than all the rest)
+            with torch.cuda.stream(side):
+                graph.capture_begin(*([] if self._pool is None else [self._pool]))
+                try:
+                    g["logits"] = self.model.forward(cap, self.cache)
+                finally:
+                    graph.capture_end()
             g["kernels"] = kernels.launch_count - before
             kernels.launch_count = before  # captured, not launched
             if self._pool is None:
