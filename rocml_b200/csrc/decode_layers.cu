@@ -24,6 +24,11 @@
 // Norms are deferred as in the kernels that this one stands for: a product that adds into the 32-bit residual stream also
 // writes residual * weight in bfloat16 and the units' sums of squares; 1/RMS is applied to the next product's sums.
 //
+// What it costs: a meeting of the blocks is a release, a poll and the next operands, a round trip to the L2 cache each (0.5 us), and the chain of
+// a unit's sums, 4 us in all; under it the weights' stream goes on.  A step, with the layers' own kernels and so, microseconds: 28 layers of 1,024
+// (31 MB) with one token 758 -> 667, 28 of 2,048 with one 1,131 -> 937, 36 of 2,560 with four 2,114 -> 1,947, 36 of 4,096 (386 MB, 6.0 TB/s in gate | up) with one 2,961 ->
+// 2,761, with eight 3,096 -> 3,058.
+//
 // Every wait is bounded.  A warp that gives up raises the block's flag and records RB_ERR_TIMEOUT; from then on no wait of
 // the block waits, and everything else runs on as always (garbage, at addresses that do not depend on data), so that no barrier is ever
 // short of a warp and no block of a partner.  The launch is cooperative: all blocks are resident or none is.
@@ -59,7 +64,8 @@ constexpr int MAX_LAYERS = 38;                // of a launch: what its parameter
 constexpr float NEG_BIG = -1e30f;
 constexpr float LOG2E = 1.4426950408889634f;
 static_assert(STAGE == 2 * SK * HD * 2 && STAGES % CW == 0, "a stage holds 16 keys and 16 values");
-constexpr int CPW = 2;                        // stages a warp takes of a unit: what it holds activations for (64 registers a tile of tokens)
+template <int NT>
+constexpr int CPW = NT == 1 ? 2 : 1;          // stages a warp takes of a unit: what it holds activations for (64 registers)
 
 struct LayerPtrs {
     const void *ff_norm, *next_norm;                     // the norm behind the mixer, and the next layer's first (null: none)
@@ -68,8 +74,7 @@ struct LayerPtrs {
     float ff_eps, in_eps;                                // of ff_norm, and of the norm whose rows this layer's first product reads
 };
 
-// A layer's phases in order.  One loop runs through them, and every product is the same code: a step goes through all of the kernel's
-// code once a layer, and what does not fit the instruction caches is fetched anew each time.
+// A layer's phases in order.  One loop runs through them, and every product is the same code (54 KB in all, 131 with a copy for each phase).
 enum { QKV, ATTENTION, OUT, GATED, DOWN, PHASES };
 
 // A phase's shape, worked out by the host.  Its units go to the blocks in turn: `each` to every one and one
@@ -359,12 +364,15 @@ struct Compute {
 
     __device__ Compute(Smem<NT>& s, Waits waits) : s(s), waits(waits), p(s.step) {}
 
-    // Every block has come this far, and what it wrote is visible (read it past the L1 cache).
-    __device__ void meet() {
+    // Every block has come this far, and what it wrote is visible (read it past the L1 cache).  In two halves: what the next phase needs to
+    // know of itself is worked out between them.
+    __device__ void arrive() {
         compute_sync();
         met += gridDim.x;
+        if (threadIdx.x == 0) add_release(p.counters);
+    }
+    __device__ void wait() {
         if (threadIdx.x == 0) {
-            add_release(p.counters);
             const unsigned t0 = (unsigned)clock();
             while ((int)(load_acquire(p.counters) - met) < 0 && !waits.over(t0)) {}
         }
@@ -466,19 +474,42 @@ struct Compute {
         }
     }
 
-    // A product of the step's rows x [T][K] with this block's units.
-    __device__ void product(int phase, const __nv_bfloat16* x, float eps, const void* norm) {
-        constexpr int C = CPW, OUTS = UR * 8 * NT, A = NT == 1 ? 4 : 2;
-        int first;
+    // A product of the step's rows [T][K] with this block's units: which, and where this thread's share of everything is.  (The plan stays in
+    // shared memory: a copy in registers made steps of 2,560 wide layers 4 % slower.)
+    struct Job {
+        int phase;
+        int first, mine, group, my_unit, my_stage;      // (unit and stage of those in work)
+        bool scaled;
+        float eps;
+        const __nv_bfloat16* row[NT];
+        Out out;
+    };
+    __device__ void prepare(Job& job, int i) {
+        const LayerPtrs& L = p.layer[i / PHASES];
+        const int phase = i % PHASES, T = p.T;
         const Plan& ps = p.plan[phase];
-        const int mine = w.share(ps, first), K = ps.K;
-        const int group = ps.passes == 1 ? mine : GROUP;
-        const int my_unit = warp / ps.warps, my_stage = (warp - my_unit * ps.warps) * C;      // of those in work
+        job.phase = phase;
+        job.mine = w.share(ps, job.first);
+        job.group = ps.passes == 1 ? job.mine : GROUP;
+        job.my_unit = warp / ps.warps;
+        job.my_stage = (warp - job.my_unit * ps.warps) * CPW<NT>;
+        job.scaled = phase == QKV || phase == GATED;
+        job.eps = phase == QKV ? L.in_eps : L.ff_eps;
+        const __nv_bfloat16* x = phase == OUT ? p.attn : (phase == DOWN ? p.h : p.xhat);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) job.row[nt] = x + (min(nt * 8 + gq, T - 1) * ps.K + job.my_stage * KC + tq * 16);
+        job.out = output(phase, phase == OUT ? L.ff_norm : L.next_norm, threadIdx.x / UR % (8 * NT));
+    }
+
+    __device__ void product(Job& job) {
+        constexpr int C = CPW<NT>, OUTS = UR * 8 * NT, A = NT == 1 ? 4 : 2;
+        const Plan& ps = p.plan[job.phase];
+        const int first = job.first, mine = job.mine, group = job.group, my_unit = job.my_unit, my_stage = job.my_stage, K = ps.K;
         // the lane's row of the four 8 x 8 matrices of a 16 x 16 A operand: rows 0..7 and 8..15 of two neighbouring chunks
         const uint32_t lane_ring = sm100::smem_u32(s.ring[0]) + (lane & 15) * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
         // who sums what: a thread row r of token t of one of the units in work, and (short sums) of the next but one
         const int r = threadIdx.x & 15, t = threadIdx.x / UR % (8 * NT);
-        Out out = output(phase, norm, t);
+        Out& out = job.out;
 #pragma unroll 1
         for (int g0 = 0; g0 < mine; g0 += group)
 #pragma unroll 1
@@ -491,7 +522,7 @@ struct Compute {
                 uint4 B[C * (KC / KB)][NT][2];
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
-                    const __nv_bfloat16* row = x + (min(nt * 8 + gq, p.T - 1) * K + (c0 + my_stage) * KC + tq * 16);
+                    const __nv_bfloat16* row = job.row[nt] + c0 * KC;
 #pragma unroll
                     for (int j = 0; j < C * (KC / KB); ++j)
 #pragma unroll
@@ -500,7 +531,7 @@ struct Compute {
                             load_if(j < nb, B[j][nt][half], row + j * KB + half * 8);
                         }
                 }
-                bool scales = (phase == QKV || phase == GATED) && g0 == 0 && pass == 0;
+                bool scales = job.scaled && g0 == 0 && pass == 0;
                 Squares squares;
                 if (scales) ask_squares(squares);
                 const bool last = pass == ps.passes - 1;
@@ -558,7 +589,7 @@ struct Compute {
                             to[TOK + 8] = acc[nt][0][3] + acc[nt][1][3];
                         }
                     }
-                    if (scales) row_scales(squares, eps);
+                    if (scales) row_scales(squares, job.eps);
                     scales = false;
                     // (behind this barrier every warp has left the stages of the round, which are fewer than the ring's: what a warp waits
                     // for next is at most one use of a stage away, so that its parity says which)
@@ -811,10 +842,9 @@ struct Compute {
             if (p.splits > 1) {
                 compute_sync();
                 if (threadIdx.x == 0) {
-                    __threadfence();
-                    const unsigned before = atomicAdd(p.counters + 1 + b * p.nkv + kvh, 1u);
+                    unsigned before;
+                    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(p.counters + 1 + b * p.nkv + kvh) : "memory");
                     s.last = (before + 1) % (unsigned)p.splits == 0;      // (every layer adds `splits`)
-                    __threadfence();
                 }
                 compute_sync();
                 if (s.last)
@@ -856,21 +886,25 @@ struct Compute {
         Item mine;
         mine.find(s, blockIdx.x);
         const int g = p.nq / p.nkv;
+        Job job;
         if (p.first_norm != nullptr) {
             first_rows();
-            meet();
+            arrive();
+            prepare(job, 0);
+            wait();
+        } else {
+            prepare(job, 0);
         }
+        const int n = p.layers * PHASES;
 #pragma unroll 1
-        for (int i = 0; i < p.layers * PHASES; ++i) {
-            const LayerPtrs& L = p.layer[i / PHASES];
-            const int phase = i % PHASES;
-            if (phase == ATTENTION) {
-                attention(L, mine, g);
-            } else {
-                const __nv_bfloat16* x = phase == OUT ? p.attn : (phase == DOWN ? p.h : p.xhat);
-                product(phase, x, phase == QKV ? L.in_eps : L.ff_eps, phase == OUT ? L.ff_norm : L.next_norm);
+        for (int i = 0; i < n; ++i) {
+            if (i % PHASES == ATTENTION) attention(p.layer[i / PHASES], mine, g);
+            else product(job);
+            if (i + 1 < n) {
+                arrive();
+                if ((i + 1) % PHASES != ATTENTION) prepare(job, i + 1);
+                wait();
             }
-            if (i + 1 < p.layers * PHASES) meet();
         }
     }
 };
@@ -1019,13 +1053,14 @@ extern "C" int rb_decode_layers(const void* step, void* stream) {
     p.wait_limit = (unsigned)(q.wait_limit > 0 && q.wait_limit < sm100::RB_WAIT_CYCLES ? q.wait_limit : sm100::RB_WAIT_CYCLES);
     const int work[PHASES] = {(q.nq + 2 * q.nkv) * HD / UR, 0, q.H / UR, 2 * q.I / UR, q.H / UR};
     const int inputs[PHASES] = {q.H, KC, q.nq * HD, q.H, q.I};
+    const int a_warp = q.T <= 8 ? CPW<1> : CPW<2>;
     for (int i = 0; i < PHASES; ++i) {
         Plan& a = p.plan[i];
         a.each = work[i] / ready->sms; a.rest = work[i] % ready->sms;
         a.K = inputs[i]; a.stages = (a.K + KC - 1) / KC;
-        a.passes = (a.stages + CW * CPW - 1) / (CW * CPW);
+        a.passes = (a.stages + CW * a_warp - 1) / (CW * a_warp);
         a.per = (a.stages + a.passes - 1) / a.passes;
-        a.warps = (a.per + CPW - 1) / CPW;
+        a.warps = (a.per + a_warp - 1) / a_warp;
         a.units = a.warps > 4 ? 1 : (a.warps > 2 ? 2 : (q.T <= 8 ? 4 : 2));
     }
     const unsigned long long cached = (unsigned long long)q.n_pages * q.nkv * RB_PAGE;

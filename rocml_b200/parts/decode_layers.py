@@ -19,9 +19,9 @@ from .norm import RMSNorm
 from .plain import plain_layer
 
 # Up to one tile of tokens the one kernel is the faster one: a step before and now, microseconds, 28 layers of 0.6b sizes with 1, 2 and 8
-# sequences 758, 853, 856 -> 677, 791, 769; 1.7b with 1 and 4 1,131, 1,159 -> 942, 1,012, with 8 of 700 to 1,300 tokens 1,281 -> 1,279;
-# 4b with 1 (900 tokens) and 4 2,075, 2,100 -> 2,005, 1,981; 8b with 1 and 8 2,961, 3,099 -> 2,778, 3,083.  A second tile of tokens: 0.6b with 16
-# 884 -> 1,051, 8b 3,537 -> 3,802.
+# sequences 758, 853, 856 -> 667, 769, 764; 1.7b with 1 and 4 1,131, 1,159 -> 937, 1,006, with 8 of 700 to 1,300 tokens 1,280 -> 1,248;
+# 4b with 1 (900 tokens), 4 and 8 2,080, 2,114, 2,227 -> 1,971, 1,947, 2,068; 8b with 1 and 8 2,961, 3,096 -> 2,761, 3,058.  A second tile of
+# tokens: 0.6b with 16 884 -> 880, 8b 3,537 -> 4,000.
 MAX_TOKENS = 8
 
 
