@@ -264,9 +264,11 @@ struct Producer {
 
     __device__ Producer(Smem<NT>& s, Waits waits) : s(s), waits(waits) {}
 
-    // The next stage is free, and its barrier knows what will land in it; false: given up.
+    // The next stage is free, and its barrier knows what will land in it; false: given up.  A warp that gave up on a stage hands it back
+    // all the same, perhaps while the copy into it is still on its way; it has read or raised the flag before, which is therefore
+    // seen here behind the wait: such a stage is not armed a second time, and the drain at the end finds each copy's own phase.
     __device__ bool room() {
-        if (!waits.barrier(&s.empty[w.stage], w.phase ^ 1)) return false;
+        if (!waits.barrier(&s.empty[w.stage], w.phase ^ 1) || waits.gave_up()) return false;
         sm100::mbar_arrive_expect_tx(&s.full[w.stage], STAGE);         // (beyond K and beyond the cache's rows zeros arrive)
         ++issued;
         return true;
