@@ -193,7 +193,6 @@ class Engine:
         ``device_tokens`` (int32 on the device, one per entry) replaces the entries' token ids
         for a step of one token per sequence: the ids a sampling kernel has just written are
         fed back without passing through the host."""
-        self._device_tokens = device_tokens
         if device_tokens is not None and any(len(e.tokens) != 1 for e in entries if isinstance(e, StepEntry)):
             raise RocmlError("device_tokens needs exactly one token per entry")
         entries = [e if isinstance(e, StepEntry) else StepEntry(*e) for e in entries]
@@ -239,6 +238,8 @@ class Engine:
                     w_here = sorted(w for w in set(e.want) if a <= w < b)
                     wants.append([w - a for w in w_here])
                     order.extend((i, w) for w in w_here)
+                # (one token per entry: a piece's entries are a run of them)
+                self._device_tokens = None if device_tokens is None else device_tokens[piece[0][0]:piece[-1][0] + 1]
                 logits = self._run(slots, olds, toks, wants)
                 for (i, a, b) in piece:
                     self.cache.commit(entries[i].slot, b - a)
@@ -307,7 +308,7 @@ class Engine:
         buf = self._eager[key]
         buf.fill(*packed, slots, pad_tokens=T, pad_seqs=B, pad_want=W)
         if self._device_tokens is not None:
-            buf.token_ids[:B].copy_(self._device_tokens[:B], non_blocking=True)
+            buf.token_ids[:B].copy_(self._device_tokens, non_blocking=True)
         self.last_h2d_bytes = buf.h2d_bytes
         batch = self._batch(buf, T, B, W, max(q_lens), max(kv_len), is_decode, host)
         return self.model.forward(batch, self.cache)
@@ -343,7 +344,7 @@ class Engine:
         buf: BatchBuffers = g["buffers"]
         buf.fill(*packed, host.seq_slots, pad_tokens=t_pad, pad_seqs=b_pad, pad_want=w_pad)
         if self._device_tokens is not None:
-            buf.token_ids[:B].copy_(self._device_tokens[:B], non_blocking=True)
+            buf.token_ids[:B].copy_(self._device_tokens, non_blocking=True)
         self.last_h2d_bytes = buf.h2d_bytes
         if g["graph"] is None:
             # First use of this bucket: run it plainly (this also loads every kernel), then

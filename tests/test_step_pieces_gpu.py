@@ -143,3 +143,24 @@ def test_a_step_that_cannot_fit_takes_nothing(model_folder):
     assert eng.launches == before and eng.length(a) == 0 and eng.length(b) == 0
     assert all(g.pool.n_held == 0 for g in eng.cache.kv_groups)
     eng.cache.check_invariants()
+
+
+@pytest.mark.parametrize("use_graphs", [True, False])
+def test_tokens_fed_back_on_the_device_reach_their_piece(tmp_path, use_graphs):
+    """A batch larger than a piece, each sequence's next token taken from where the sampling kernel wrote it: every piece gets its own
+    sequences' tokens, with and without graphs, and a tensor with more entries than the step is read from its beginning."""
+    from plain_qwen3 import PlainQwen3
+    from rocml_b200 import Engine, StepEntry
+    folder = str(tmp_path / "m")
+    write_model(folder, CONFIGS["A"], seed=5, std=0.05)
+    plain = PlainQwen3(folder, dtype=torch.float64)
+    vocab = CONFIGS["A"]["vocab_size"]
+    ids = [prompt(900 + i, 9 + i, vocab) for i in range(5)]
+    eng = Engine.from_folder(folder, dtype="float32", max_tokens=1024, max_step_tokens=2, use_graphs=use_graphs)
+    done = eng.generate(ids, max_new_tokens=6, stop_tokens=[], ignore_eos=True)
+    assert [c.tokens for c in done] == [plain.greedy(x, 6) for x in ids]
+    slots = [eng.new_sequence() for _ in ids]
+    eng.step([StepEntry(s, x[:-1], []) for s, x in zip(slots, ids)])
+    fed = torch.tensor([x[-1] for x in ids] + [0, 0], dtype=torch.int32, device="cuda:0")
+    got = eng.step([StepEntry(s, [0], [0]) for s in slots], device_tokens=fed)
+    assert rel_err(got, torch.stack([plain.logits(x)[-1] for x in ids])) < TOL["float32"]
