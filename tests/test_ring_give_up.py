@@ -1,5 +1,5 @@
-"""A ring of stages whose waits may run out: warps that give up hand their stages back though the copies may still be on their way, so the
-producer looks at the flag behind every wait for a free stage, before it arms the stage's barrier.  Read off the source; no GPU is needed."""
+"""A ring of stages whose waits may run out: a warp that gave up must not hand its stage back, since the copy into it may still be on its way
+and the producer would arm the stage's barrier a second time.  Read off the source; no GPU is needed."""
 import os
 import re
 
@@ -19,13 +19,19 @@ def body(text, head):
             return text[at:end]
 
 
-def test_no_stage_is_armed_once_a_wait_has_run_out():
+def test_no_stage_is_handed_back_once_a_wait_has_run_out():
     with open(PATH) as f:
         text = re.sub(r"//[^\n]*", "", f.read())
-    room = body(text, "bool room()")
-    waited, armed = room.index("waits.barrier("), room.index("mbar_arrive_expect_tx(")
-    looked = [m.start() for m in re.finditer(r"waits\.gave_up\(\)", room)]
-    assert any(waited < at < armed for at in looked)
-    assert text.count("mbar_arrive_expect_tx(") == 1          # nothing else arms a stage
-    # and the warps that compute raise or read the flag before they hand a stage back without success
+    # what is handed back was looked at behind the wait for its copy
+    taken, back = body(text, "bool taken("), body(text, "void give_back(")
+    assert taken.index("waits.barrier(&s.full[") < taken.index("return !waits.gave_up()")
+    assert "if (lane == 0 && whole) sm100::mbar_arrive(&s.empty[" in back
+    compute = body(text, "struct Compute ")
+    assert compute.count("&s.full[") == taken.count("&s.full[") == 1 and compute.count("&s.empty[") == 1
+    uses = re.findall(r"const bool whole = taken\(at\);|give_back\(at, whole\);", compute)
+    assert uses == ["const bool whole = taken(at);", "give_back(at, whole);"] * 2
+    # a warp that leaves a wait without success has raised the flag or seen it
     assert "return false" in body(text, "bool barrier(") and "gave_up()) return true" in body(text, "bool over(")
+    # and one place arms a stage, behind the wait for it
+    room = body(text, "bool room()")
+    assert room.index("waits.barrier(&s.empty[") < room.index("mbar_arrive_expect_tx(") and text.count("mbar_arrive_expect_tx(") == 1
