@@ -122,6 +122,7 @@ class Engine:
         self.last_h2d_bytes = 0
         self._sampler = None
         self._device_tokens = None
+        self._replayed = False     # the last piece's logits are a graph's
         self.graph_kernel_launches = 0  # kernels run by graph replays
 
     # After the weights are resident: does the cache fit what is left, with head room for a step's
@@ -244,8 +245,8 @@ class Engine:
                 for (i, a, b) in piece:
                     self.cache.commit(entries[i].slot, b - a)
                 if logits is not None:
-                    # (a replayed graph's logits live until its next replay, which may be the next piece)
-                    outs.append(logits if len(pieces) == 1 else logits.clone())
+                    # (a replayed graph's logits live until the next replay, which may be the next piece's)
+                    outs.append(logits.clone() if self._replayed and len(pieces) > 1 else logits)
             if not outs:
                 return None
             result = outs[0] if len(outs) == 1 else torch.cat(outs, dim=0)
@@ -286,6 +287,7 @@ class Engine:
         host = HostBatch(list(slots), q_lens, list(kv_len), list(want_rows))
         self.cache.flush()
         self.launches += 1
+        self._replayed = False
         prof = _profiler.ACTIVE
         if prof is not None:
             # a profiled step runs its kernels one by one, without a graph (rocml_b200.profile.profiler)
@@ -371,6 +373,7 @@ class Engine:
             self.graphs_captured += is_decode
             return out[:W] if W else None
         g["graph"].replay()
+        self._replayed = True
         self.graph_kernel_launches += g["kernels"]
         return g["logits"][:W] if W else None
 

@@ -164,3 +164,27 @@ def test_tokens_fed_back_on_the_device_reach_their_piece(tmp_path, use_graphs):
     fed = torch.tensor([x[-1] for x in ids] + [0, 0], dtype=torch.int32, device="cuda:0")
     got = eng.step([StepEntry(s, [0], [0]) for s in slots], device_tokens=fed)
     assert rel_err(got, torch.stack([plain.logits(x)[-1] for x in ids])) < TOL["float32"]
+
+
+def test_only_a_replayed_graphs_logits_are_copied(tmp_path, monkeypatch):
+    """The pieces of a step that run without a graph own their logits: they are joined as they are, not copied first."""
+    from rocml_b200 import Engine, StepEntry
+    from rocml_b200.engine import engine as module
+    folder = str(tmp_path / "m")
+    write_model(folder, CONFIGS["A"], seed=6, std=0.05)
+    ids = prompt(77, 120, CONFIGS["A"]["vocab_size"])
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=1024, max_step_tokens=32, use_graphs=False)
+    made, joined = [], []
+    run, cat = eng._run, torch.cat
+
+    def piece(*a):
+        made.append(run(*a))
+        return made[-1]
+
+    def join(tensors, **kw):
+        joined.extend(t.data_ptr() for t in tensors)
+        return cat(tensors, **kw)
+    monkeypatch.setattr(eng, "_run", piece)
+    monkeypatch.setattr(module.torch, "cat", join)
+    eng.step([StepEntry(eng.new_sequence(), ids, list(range(120)))])
+    assert len(made) == 4 and joined[-4:] == [t.data_ptr() for t in made]
