@@ -117,7 +117,6 @@ class Engine:
         # (layers whose prompt kernels take nothing from the host but the step's sizes)
         self._graph_prompts = self.use_graphs and self.env.act_dtype == torch.bfloat16 and all(plain_layer(b) for b in model.blocks)
         self.graphs_captured = 0
-        self._pool = None
         self.launches = 0          # steps issued (sub-steps counted)
         self.last_h2d_bytes = 0
         self._sampler = None
@@ -360,15 +359,15 @@ class Engine:
             before = kernels.launch_count
             # (torch.cuda.graph collects garbage and empties the allocator's cache first, which takes longer than all the rest)
             with torch.cuda.stream(side):
-                graph.capture_begin(*([] if self._pool is None else [self._pool]))
+                # (graphs share their memory, as no two run side by side; it goes with the last of them)
+                pool = next((x["graph"].pool() for t in (self._graphs, self._prompt_graphs) for x in t.values() if x["graph"] is not None), None)
+                graph.capture_begin(pool)
                 try:
                     g["logits"] = self.model.forward(cap, self.cache)
                 finally:
                     graph.capture_end()
             g["kernels"] = kernels.launch_count - before
             kernels.launch_count = before  # captured, not launched
-            if self._pool is None:
-                self._pool = graph.pool()
             g["graph"] = graph
             self.graphs_captured += is_decode
             return out[:W] if W else None

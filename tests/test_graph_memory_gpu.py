@@ -1,0 +1,46 @@
+"""The memory of captured graphs: shared while there is a graph, given back, and bounded over many captures."""
+import pytest
+import torch
+
+from tiny_models import CONFIGS, prompt, write_model
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2.5e-2        # as the other tests of bfloat16 layers
+
+
+def rel_err(got, want):
+    want = want.to(torch.float64)
+    return float(((got.double().cpu() - want).abs() / want.abs().amax(dim=-1, keepdim=True).clamp_min(1e-30)).max())
+
+
+@pytest.fixture(scope="module")
+def model(tmp_path_factory):
+    from plain_qwen3 import PlainQwen3
+    config = {**CONFIGS["E"], "use_sliding_window": False, "layer_types": ["full_attention"] * 2}
+    folder = str(tmp_path_factory.mktemp("graph_memory"))
+    write_model(folder, config, seed=23, std=0.05)
+    return config, folder, PlainQwen3(folder, dtype=torch.float64)
+
+
+def decode(eng, ids, steps=3):
+    """The logits of ``steps`` single tokens behind the rest of each of ``ids``, [sequences][steps, vocab]."""
+    from rocml_b200 import StepEntry
+    slots = [eng.new_sequence() for _ in ids]
+    eng.step([StepEntry(s, x[:-steps], []) for s, x in zip(slots, ids)])
+    rows = [eng.step([StepEntry(s, [x[t - steps]], [0]) for s, x in zip(slots, ids)]).clone() for t in range(steps)]
+    for s in slots:
+        eng.release(s)
+    return torch.stack(rows, dim=1)
+
+
+def test_one_graph_is_kept_and_another_size_takes_its_place(model):
+    """max_graphs=1: with the only graph goes the memory that it shared, and the next size's graph begins anew."""
+    from rocml_b200 import Engine
+    config, folder, plain = model
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=2048, max_slots=4, max_graphs=1)
+    for n in (1, 3, 1, 2, 1):
+        ids = [prompt(40 + n + i, 300 + i, config["vocab_size"]) for i in range(n)]
+        got = decode(eng, ids)
+        for i, x in enumerate(ids):
+            assert rel_err(got[i], plain.logits(x)[-3:]) < TOL
