@@ -116,6 +116,7 @@ class Engine:
         self._prompt_graphs: "OrderedDict[Tuple[int, ...], dict]" = OrderedDict()
         # (layers whose prompt kernels take nothing from the host but the step's sizes)
         self._graph_prompts = self.use_graphs and self.env.act_dtype == torch.bfloat16 and all(plain_layer(b) for b in model.blocks)
+        self._capture_stream = None
         self.graphs_captured = 0
         self.launches = 0          # steps issued (sub-steps counted)
         self.last_h2d_bytes = 0
@@ -353,12 +354,15 @@ class Engine:
             batch = self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, host)
             out = self.model.forward(batch, self.cache)
             torch.cuda.current_stream().synchronize()
-            graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream(self.device)
+            graph = torch.cuda.CUDAGraph()
+            if self._capture_stream is None:
+                # (one for all captures: the allocator hands a block out again only on the stream that it was made for)
+                self._capture_stream = torch.cuda.Stream(self.device)
             cap = self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, None, capturing=True)
             from .. import kernels
             before = kernels.launch_count
             # (torch.cuda.graph collects garbage and empties the allocator's cache first, which takes longer than all the rest)
-            with torch.cuda.stream(side):
+            with torch.cuda.stream(self._capture_stream):
                 # (graphs share their memory, as no two run side by side; it goes with the last of them)
                 pool = next((x["graph"].pool() for t in (self._graphs, self._prompt_graphs) for x in t.values() if x["graph"] is not None), None)
                 graph.capture_begin(pool)

@@ -44,3 +44,18 @@ def test_one_graph_is_kept_and_another_size_takes_its_place(model):
         got = decode(eng, ids)
         for i, x in enumerate(ids):
             assert rel_err(got[i], plain.logits(x)[-3:]) < TOL
+
+
+def test_memory_stops_growing_over_many_captures(model):
+    """More sizes than are kept, over and over: what earlier graphs held is used again."""
+    from rocml_b200 import Engine
+    config, folder, _ = model
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=4096, max_slots=8, max_graphs=2)
+    batches = [[prompt(60 + i, 300 * k + i, config["vocab_size"]) for i in range(n)] for n in (1, 2, 4, 8) for k in (1, 2) if n * k <= 8]
+    held = []
+    for _ in range(8):
+        for ids in batches:
+            decode(eng, ids)
+        torch.cuda.synchronize()
+        held.append(torch.cuda.memory_reserved())
+    assert eng.graphs_captured >= 8 * 6 and held[-1] == held[2], held
