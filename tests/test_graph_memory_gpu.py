@@ -59,3 +59,27 @@ def test_memory_stops_growing_over_many_captures(model):
         torch.cuda.synchronize()
         held.append(torch.cuda.memory_reserved())
     assert eng.graphs_captured >= 8 * 6 and held[-1] == held[2], held
+
+
+@pytest.mark.parametrize("failures", [1, 2])
+def test_a_capture_that_runs_out_of_memory_loses_no_step(model, monkeypatch, failures):
+    """The memory that the allocator holds goes back and the capture is tried again; if that does not help, the size runs without a
+    graph.  Every step gives its logits."""
+    from rocml_b200 import Engine
+    config, folder, plain = model
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=2048, max_slots=4)
+    forward, left, emptied = eng.model.forward, [failures], []
+
+    def short_of_memory(batch, cache):
+        if batch.capturing and left[0] > 0:
+            left[0] -= 1
+            raise torch.OutOfMemoryError("out of memory (made up)")
+        return forward(batch, cache)
+    monkeypatch.setattr(eng.model, "forward", short_of_memory)
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: emptied.append(1))
+    ids = [prompt(90 + i, 310 + i, config["vocab_size"]) for i in range(2)]
+    for _ in range(2):
+        got = decode(eng, ids)
+        for i, x in enumerate(ids):
+            assert rel_err(got[i], plain.logits(x)[-3:]) < TOL
+    assert left == [0] and len(emptied) == failures and eng.graphs_captured == 2 - failures
