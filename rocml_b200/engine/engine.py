@@ -378,7 +378,8 @@ class Engine:
             graph = torch.cuda.CUDAGraph()
             try:
                 with torch.cuda.stream(self._capture_stream):
-                    graph.capture_begin(pool)
+                    # (only this thread's calls are watched: others may allocate meanwhile)
+                    graph.capture_begin(pool, "thread_local")
                     try:
                         logits = self.model.forward(batch, self.cache)
                     finally:

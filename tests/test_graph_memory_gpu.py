@@ -83,3 +83,35 @@ def test_a_capture_that_runs_out_of_memory_loses_no_step(model, monkeypatch, fai
         for i, x in enumerate(ids):
             assert rel_err(got[i], plain.logits(x)[-3:]) < TOL
     assert left == [0] and len(emptied) == failures and eng.graphs_captured == 2 - failures
+
+
+def test_another_thread_may_allocate_during_captures(model):
+    """Fresh device memory for another thread while sizes are captured: neither disturbs the other."""
+    import threading
+    import time
+    from rocml_b200 import Engine
+    config, folder, plain = model
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=4096, max_slots=8, max_graphs=1)
+    stop, failed, held = threading.Event(), [], []
+
+    def allocate():
+        try:
+            while not stop.is_set() and len(held) < 500:
+                held.append(torch.empty(32 << 20, dtype=torch.uint8, device="cuda:0"))       # (more than is cached: from the device each time)
+                time.sleep(0.001)
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+    other = threading.Thread(target=allocate)
+    other.start()
+    try:
+        for n in (1, 2, 4, 8) * 4:
+            ids = [prompt(120 + n + i, 300 + i, config["vocab_size"]) for i in range(n)]
+            got = decode(eng, ids)
+            for i, x in enumerate(ids[:1]):
+                assert rel_err(got[i], plain.logits(x)[-3:]) < TOL
+    finally:
+        stop.set()
+        other.join()
+    assert not failed and len(held) > 50, failed
+    held.clear()
+    torch.cuda.empty_cache()
