@@ -66,17 +66,62 @@ def _ctx_bucket(n: int) -> int:
     return max(step, -(-n // step) * step)
 
 
-# Prompts of at most this many tokens (all sequences of a piece together) are replayed from captured graphs too: their kernels
-# take less time than the host takes to launch them one by one (61 tokens, 28 layers of 1.7b sizes: 256 launches, 4.0 ms on the host, 2.0
-# as a graph).
-PROMPT_GRAPH_TOKENS = 256
-PROMPT_GRAPHS = 4          # how many are kept
+# Prompts of few tokens (all sequences of a piece together) are replayed from captured graphs too, where their kernels take less time than the host
+# takes to launch them one by one (9 launches a layer): the layers' weights decide that.  Milliseconds of a step alone, launched and replayed, at 61,
+# 128 and 256 tokens: 28 layers of 0.6b sizes (31 MB a layer) 4.1, 4.0, 3.8 and 1.7, 2.3, 2.5; 28 of 1.7b (101 MB) 4.2, 4.3, 3.9 and 2.1, 2.8, 3.1; 36 of 4b
+# (202 MB) 5.3, 5.3, 6.1 and 3.4, 4.4, 5.6, but with 129 tokens 5.7 for 5.5; 36 of 8b (386 MB) 5.4, 5.4, 7.2 and 4.5, 5.1, 6.9, with 129 tokens 6.5 for 7.0.
+# A capture takes 3 to 6 ms more than the step that it stands for (at times 30 to 190), which a few replays pay for: a size is captured the fourth time
+# that it comes.  (Streams of prompts on new engines, ms a prompt, launched, captured the first time with four kept as they came, and by these rules: 64 lengths
+# at random up to 256, 0.6b 3.96, 5.87, 3.49, 4b 5.58, 9.05, 5.58; five lengths in turn 4.03, 9.47, 2.89 and 5.36, 21.1, 4.98; one length 4.15, 2.03, 2.22 and 5.37, 3.67,
+# 4.01; the prompts of ten turns of a chat 4.26, 8.53, 4.24 and 6.44, 64.9, 6.03.)
+PROMPT_GRAPH_RULES = ((128 << 20, 256), (400 << 20, 128))      # (bytes of a layer at most, tokens at most)
+PROMPT_GRAPH_TIMES = 4
+PROMPT_GRAPHS = 8                                              # how many are kept at most
 
 
-def _prompt_bucket(n: int) -> int:
-    """How many tokens a captured prompt graph for ``n`` is sized for: the next multiple of 16, of 32 beyond 64, of 64 beyond 128."""
-    step = 16 if n <= 64 else (32 if n <= 128 else 64)
-    return -(-n // step) * step
+def _prompt_graph_tokens(layer_bytes: int) -> int:
+    return next((tokens for most, tokens in PROMPT_GRAPH_RULES if layer_bytes <= most), 0)
+
+
+def _prompt_pads(n_tokens: int, n_seqs: int, n_want: int, longest: int):
+    """What a captured prompt graph is sized for, tokens, sequences, wanted rows, longest piece, longest sequence (which decides the order of
+    blocks only), or None where the step has no graph: more wanted places than sequences.  Powers of two, few of them: padding 33
+    tokens to 64 costs 4 % of a replay, a size more a capture."""
+    t, b = _bucket(n_tokens, 16), _bucket(n_seqs)
+    return (t, b, b if n_want else 0, t, _bucket(longest, 4096), False) if n_want <= b else None
+
+
+class GraphSizes:
+    """Which sizes of short prompts are worth a captured graph.  The first steps of a size are launched kernel by kernel; the ``times``-th is captured
+    while there is room, and later only if the size has come more often than the rarest of those kept by as many times:
+    sizes that take turns do not drive one another out.  Counts are halved now and then, so that what was common long ago gives way."""
+
+    def __init__(self, kept: int, times: int = PROMPT_GRAPH_TIMES):
+        self.kept, self.times = kept, times
+        self.seen: Dict[tuple, int] = {}
+        self._total = 0
+
+    def due(self, size, graphs: "OrderedDict") -> bool:
+        """Whether a step of this size runs as a graph, of which ``graphs`` are there; the one that has to go for it is then the first of them."""
+        if size in graphs:
+            return True
+        n = self.seen.get(size, 0) + 1
+        if n < self.times or self.kept < 1:
+            return False
+        if len(graphs) >= self.kept:
+            rarest = min(graphs, key=lambda k: self.seen.get(k, 0))
+            if n < self.seen.get(rarest, 0) + self.times:
+                return False
+            graphs.move_to_end(rarest, last=False)
+        return True
+
+    def note(self, size) -> None:
+        """A step of this size has run."""
+        self.seen[size] = self.seen.get(size, 0) + 1
+        self._total += 1
+        if self._total >= 256:
+            self.seen = {k: n // 2 for k, n in self.seen.items() if n > 1}
+            self._total = sum(self.seen.values())
 
 
 class Engine:
@@ -84,8 +129,8 @@ class Engine:
                  max_step_tokens: int = 4096, use_graphs: bool = True, max_seq_len: Optional[int] = None,
                  max_graphs: int = 8):
         """``max_graphs``: how many captured decode graphs are kept (one per batch bucket and context
-        bucket, least recently used dropped first); each holds its own activations and logits.  (A few graphs of short prompts
-        are kept beside them.)"""
+        bucket, least recently used dropped first); each holds its own activations and logits.  As many graphs of short prompts, up to
+        ``PROMPT_GRAPHS`` and as the memory left over allows, are kept beside them."""
         self.model = model
         self.env = model.env
         self.device = model.env.device
@@ -99,7 +144,11 @@ class Engine:
             # of the block table and, where a layer keeps fixed-size state, its state)
             max_slots = max(1, min((max_tokens + 63) // 64, 4096))
         self.use_graphs = bool(use_graphs) and model.graph_safe and self.device.type == "cuda"
-        self._check_budget(max_tokens, max_slots)
+        # (layers whose prompt kernels take nothing from the host but the step's sizes)
+        self._prompt_graph_tokens = 0
+        if self.use_graphs and self.env.act_dtype == torch.bfloat16 and all(plain_layer(b) for b in model.blocks):
+            self._prompt_graph_tokens = _prompt_graph_tokens(max(b.weight_bytes() for b in model.blocks))
+        self._prompt_sizes = GraphSizes(self._check_budget(max_tokens, max_slots))
         self.cache = SequenceCache(
             model.cache_requirements(), model.reads_cache_of(), max_tokens, max_slots,
             min(model.spec.max_position, max_seq_len or model.spec.max_position), self.env.act_dtype,
@@ -114,8 +163,6 @@ class Engine:
         self._eager: Dict[Tuple[int, int], BatchBuffers] = {}
         self._graphs: "OrderedDict[Tuple[int, int], dict]" = OrderedDict()
         self._prompt_graphs: "OrderedDict[Tuple[int, ...], dict]" = OrderedDict()
-        # (layers whose prompt kernels take nothing from the host but the step's sizes)
-        self._graph_prompts = self.use_graphs and self.env.act_dtype == torch.bfloat16 and all(plain_layer(b) for b in model.blocks)
         self._capture_stream = None
         self.graphs_captured = 0
         self.launches = 0          # steps issued (sub-steps counted)
@@ -129,10 +176,11 @@ class Engine:
     # activations?  (The reference's check: rocml/src/forward/mod.rs:145-168, 768 MiB of head room,
     # rocml/src/budget/mod.rs:37.)  What a step needs is asked of the parts, so it holds for any
     # arrangement: the widest step's buffers, one more set and its logits for every captured decode
-    # graph that may be kept, and the groups of fixed-size state.
-    def _check_budget(self, max_tokens: int, max_slots: int) -> None:
+    # graph that may be kept, and the groups of fixed-size state.  Returns how many graphs of short prompts
+    # fit beside all that.
+    def _check_budget(self, max_tokens: int, max_slots: int) -> int:
         if self.device.type != "cuda":
-            return
+            return 0
         esz = 4 if self.env.act_dtype == torch.float32 else 2
         per_token = state = 0
         from ..cache.requirements import simple_requirements
@@ -160,6 +208,10 @@ class Engine:
                 f"{headroom / 2**30:.1f} GiB head room (a step of {self.max_step_tokens} tokens: {step / 2**30:.2f}, "
                 f"{self.max_graphs if self.use_graphs else 0} decode graphs: {graphs / 2**30:.2f}) against "
                 f"{free / 2**30:.1f} GiB free of {total / 2**30:.1f} GiB"))
+        if not self._prompt_graph_tokens:
+            return 0
+        each = self.model.workspace_bytes(self._prompt_graph_tokens, min(_bucket(max_slots), self._prompt_graph_tokens))
+        return min(PROMPT_GRAPHS, self.max_graphs, (free - need - headroom) // each)
 
     # ---- construction ----------------------------------------------------------------------------
     @staticmethod
@@ -297,23 +349,30 @@ class Engine:
             ctx_pad = _ctx_bucket(max(kv_len))
             b_pad = _batch_bucket(B, ctx_pad, self._waves)
             return self._run_graph(self._graphs, self.max_graphs, (b_pad, ctx_pad), packed, host, W, (b_pad, b_pad, b_pad, 1, ctx_pad, True))
-        if not is_decode and self._graph_prompts and T <= PROMPT_GRAPH_TOKENS:
-            pads = (_prompt_bucket(T), _bucket(B), _bucket(W) if W else 0, _bucket(max(q_lens), 16), _ctx_bucket(max(kv_len)), False)
-            return self._run_graph(self._prompt_graphs, PROMPT_GRAPHS, pads[:5], packed, host, W, pads)
+        pads = _prompt_pads(T, B, W, max(kv_len)) if not is_decode and T <= self._prompt_graph_tokens and self._prompt_sizes.kept else None
+        if pads is not None:
+            if self._prompt_sizes.due(pads, self._prompt_graphs):
+                out = self._run_graph(self._prompt_graphs, self._prompt_sizes.kept, pads, packed, host, W, pads)
+            else:
+                # (padded as the graph will be: an answer does not depend on how often its size has come)
+                out = self._run_eager(packed, host, slots, q_lens, T, B, W, is_decode, pads)
+            self._prompt_sizes.note(pads)
+            return out
         return self._run_eager(packed, host, slots, q_lens, T, B, W, is_decode)
 
-    def _run_eager(self, packed, host, slots, q_lens, T, B, W, is_decode) -> Optional[torch.Tensor]:
+    def _run_eager(self, packed, host, slots, q_lens, T, B, W, is_decode, pads=None) -> Optional[torch.Tensor]:
         kv_len = packed[4]
         key = (_bucket(T, 64), _bucket(B, 8))
         if key not in self._eager:
             self._eager[key] = BatchBuffers(key[0], key[1], key[0], self.device)
         buf = self._eager[key]
-        buf.fill(*packed, slots, pad_tokens=T, pad_seqs=B, pad_want=W)
+        t_pad, b_pad, w_pad, max_q, max_kv, _ = pads or (T, B, W, max(q_lens), max(kv_len), is_decode)
+        buf.fill(*packed, slots, pad_tokens=t_pad, pad_seqs=b_pad, pad_want=w_pad)
         if self._device_tokens is not None:
             buf.token_ids[:B].copy_(self._device_tokens, non_blocking=True)
         self.last_h2d_bytes = buf.h2d_bytes
-        batch = self._batch(buf, T, B, W, max(q_lens), max(kv_len), is_decode, host)
-        return self.model.forward(batch, self.cache)
+        out = self.model.forward(self._batch(buf, t_pad, b_pad, w_pad, max_q, max_kv, is_decode, host), self.cache)
+        return out[:W] if W else None
 
     @staticmethod
     def _batch(buf: BatchBuffers, T, B, W, max_q, max_kv, is_decode, host, capturing=False) -> StepBatch:
@@ -348,15 +407,18 @@ class Engine:
         if self._device_tokens is not None:
             buf.token_ids[:B].copy_(self._device_tokens, non_blocking=True)
         self.last_h2d_bytes = buf.h2d_bytes
+        def batch(capturing=False):
+            return self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, None if capturing else host, capturing=capturing)
+        if g["graph"] is None and not is_decode and not g["plain"]:
+            self._capture(g, batch(capturing=True))              # (a prompt of this size has run before)
         if g["graph"] is None:
-            # First use of this bucket: run it plainly (this also loads every kernel), then
+            # First use of a decode bucket: run it plainly (this also loads every kernel), then
             # capture the same launches for the next time.  Capturing executes nothing.
-            batch = self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, host)
-            out = self.model.forward(batch, self.cache)
-            if not g["plain"]:
+            out = self.model.forward(batch(), self.cache)
+            if is_decode and not g["plain"]:
                 torch.cuda.current_stream().synchronize()
-                self._capture(g, self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, None, capturing=True))
-                self.graphs_captured += is_decode and g["graph"] is not None
+                self._capture(g, batch(capturing=True))
+                self.graphs_captured += g["graph"] is not None
             return out[:W] if W else None
         g["graph"].replay()
         self._replayed = True

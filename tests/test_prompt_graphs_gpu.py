@@ -62,3 +62,67 @@ def test_pieces_that_replay_one_graph(model):
         slot = eng.new_sequence()
         assert rel_err(eng.step([StepEntry(slot, ids, list(range(330)))]), want) < TOL
         eng.release(slot)
+
+
+def test_pieces_that_replay_one_graph_with_one_place_each(model):
+    """As above with one wanted place a piece, which is what has a graph."""
+    from rocml_b200 import Engine, StepEntry
+    config, folder, plain = model
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=1024, max_slots=3, max_step_tokens=64)
+    ids = prompt(6, 330, config["vocab_size"])
+    want = plain.logits(ids)[[5, 100, 130, 200, 319, 329]]
+    for _ in range(2):
+        slot = eng.new_sequence()
+        assert rel_err(eng.step([StepEntry(slot, ids, [5, 100, 130, 200, 319, 329])]), want) < TOL
+        eng.release(slot)
+    assert len(eng._prompt_graphs) == 1          # (of 64 tokens; the rest of ten has come twice)
+
+
+def test_a_size_that_comes_back_is_captured_and_answers_alike(model):
+    """No capture for a size seen three times; the same bits before, when it is captured and from then on; never more graphs than
+    max_graphs, and sizes that take turns are not captured over and over."""
+    from rocml_b200 import Engine, StepEntry
+    config, folder, _ = model
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=1024, max_slots=3, max_graphs=2)
+    captured, capture = [], eng._capture
+    eng._capture = lambda g, batch: captured.append(batch.n_tokens) or capture(g, batch)
+    first = {}
+    for turn in range(7):
+        for n in (2, 30, 61, 100, 200):
+            slot = eng.new_sequence()
+            got = eng.step([StepEntry(slot, prompt(n, n, config["vocab_size"]), [n - 1])]).clone()
+            eng.release(slot)
+            assert torch.equal(first.setdefault(n, got), got), (turn, n)
+        assert len(captured) == (0 if turn < 3 else 2) and len(eng._prompt_graphs) == len(captured)
+
+
+def test_graphs_of_prompts_take_only_memory_that_is_left(model, monkeypatch):
+    """An engine that just fits keeps none, and is not refused for them."""
+    from rocml_b200 import Engine, MemoryBudget, StepEntry
+    config, folder, plain = model
+    refused = None
+    for spare in (0, 1, 2, 3):
+        monkeypatch.undo()
+        eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=1024, max_slots=3)
+        each = eng.model.workspace_bytes(256, 4)
+        if refused is None:
+            # the least free memory that is accepted, found through the refusals
+            lo, hi = 0, 4 << 30
+            while hi - lo > 1:
+                mid = (lo + hi) // 2
+                monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a, m=mid: (m, 180 << 30))
+                try:
+                    eng._check_budget(1024, 3)
+                    hi = mid
+                except MemoryBudget:
+                    lo = mid
+            refused = hi
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (refused + spare * each, 180 << 30))
+        assert eng._check_budget(1024, 3) == spare
+        eng = Engine(eng.model, max_tokens=1024, max_slots=3)
+        ids = prompt(8, 50, config["vocab_size"])
+        for _ in range(5):
+            slot = eng.new_sequence()
+            assert rel_err(eng.step([StepEntry(slot, ids, [49])]), plain.logits(ids)[-1:]) < TOL
+            eng.release(slot)
+        assert len(eng._prompt_graphs) == min(spare, 1)
