@@ -107,6 +107,7 @@ class StepBatch:
     want_rows: torch.Tensor
     host: Optional[HostBatch] = None
     capturing: bool = False
+    at_once: bool = True          # all layers as one kernel, where there is one, pay at these lengths (parts.decode_layers.pays)
     scratch: dict = field(default_factory=dict)
 
 

@@ -23,7 +23,7 @@ import torch
 from ..cache import SequenceCache
 from ..config import load_model_spec
 from ..errors import CacheError, ConfigError, KernelError, RocmlError
-from ..parts import BuildEnv
+from ..parts import BuildEnv, decode_layers
 from ..parts.plain import plain_layer
 from ..profile import profiler as _profiler
 from .batch import BatchBuffers, HostBatch, StepBatch, pack_entries
@@ -148,6 +148,7 @@ class Engine:
         self._prompt_graph_tokens = 0
         if self.use_graphs and self.env.act_dtype == torch.bfloat16 and all(plain_layer(b) for b in model.blocks):
             self._prompt_graph_tokens = _prompt_graph_tokens(max(b.weight_bytes() for b in model.blocks))
+        self._one_kernel = decode_layers.fits(model)
         self._prompt_sizes = GraphSizes(self._check_budget(max_tokens, max_slots))
         self.cache = SequenceCache(
             model.cache_requirements(), model.reads_cache_of(), max_tokens, max_slots,
@@ -161,7 +162,7 @@ class Engine:
             self._waves = sorted({kernels.decode_wave(g.req.n_kv_heads, self.device) for g in self.cache.kv_groups
                                   if g.req.head_dim == 128})
         self._eager: Dict[Tuple[int, int], BatchBuffers] = {}
-        self._graphs: "OrderedDict[Tuple[int, int], dict]" = OrderedDict()
+        self._graphs: "OrderedDict[Tuple[int, ...], dict]" = OrderedDict()
         self._prompt_graphs: "OrderedDict[Tuple[int, ...], dict]" = OrderedDict()
         self._capture_stream = None
         self.graphs_captured = 0
@@ -348,7 +349,9 @@ class Engine:
         if is_decode and self.use_graphs:
             ctx_pad = _ctx_bucket(max(kv_len))
             b_pad = _batch_bucket(B, ctx_pad, self._waves)
-            return self._run_graph(self._graphs, self.max_graphs, (b_pad, ctx_pad), packed, host, W, (b_pad, b_pad, b_pad, 1, ctx_pad, True))
+            at_once = self._at_once(b_pad, kv_len, ctx_pad)
+            key = (b_pad, ctx_pad) if at_once else (b_pad, ctx_pad, False)
+            return self._run_graph(self._graphs, self.max_graphs, key, packed, host, W, (b_pad, b_pad, b_pad, 1, ctx_pad, True), at_once)
         pads = _prompt_pads(T, B, W, max(kv_len)) if not is_decode and T <= self._prompt_graph_tokens and self._prompt_sizes.kept else None
         if pads is not None:
             if self._prompt_sizes.due(pads, self._prompt_graphs):
@@ -359,6 +362,10 @@ class Engine:
             self._prompt_sizes.note(pads)
             return out
         return self._run_eager(packed, host, slots, q_lens, T, B, W, is_decode)
+
+    def _at_once(self, n_tokens: int, kv_len, room: int) -> bool:
+        """``StepBatch.at_once`` of a decode step.  (Where there is no one kernel it says nothing: one graph a bucket.)"""
+        return not self._one_kernel or n_tokens > decode_layers.MAX_TOKENS or decode_layers.pays(n_tokens, self.model.hidden, max(kv_len), sum(kv_len), room)
 
     def _run_eager(self, packed, host, slots, q_lens, T, B, W, is_decode, pads=None) -> Optional[torch.Tensor]:
         kv_len = packed[4]
@@ -371,18 +378,19 @@ class Engine:
         if self._device_tokens is not None:
             buf.token_ids[:B].copy_(self._device_tokens, non_blocking=True)
         self.last_h2d_bytes = buf.h2d_bytes
-        out = self.model.forward(self._batch(buf, t_pad, b_pad, w_pad, max_q, max_kv, is_decode, host), self.cache)
+        at_once = not is_decode or self._at_once(T, kv_len, max_kv)
+        out = self.model.forward(self._batch(buf, t_pad, b_pad, w_pad, max_q, max_kv, is_decode, host, at_once), self.cache)
         return out[:W] if W else None
 
     @staticmethod
-    def _batch(buf: BatchBuffers, T, B, W, max_q, max_kv, is_decode, host, capturing=False) -> StepBatch:
+    def _batch(buf: BatchBuffers, T, B, W, max_q, max_kv, is_decode, host, at_once=True, capturing=False) -> StepBatch:
         return StepBatch(
             n_tokens=T, n_seqs=B, n_want=W, max_q_len=max_q, max_kv_len=max_kv, is_decode=is_decode,
             token_ids=buf.token_ids, positions=buf.positions, slot_of_token=buf.slot_of_token,
             seq_slot=buf.seq_slot, cu_q=buf.cu_q, kv_len=buf.kv_len, want_rows=buf.want_rows, host=host,
-            capturing=capturing)
+            capturing=capturing, at_once=at_once)
 
-    def _run_graph(self, graphs, kept: int, key, packed, host, W, pads) -> Optional[torch.Tensor]:
+    def _run_graph(self, graphs, kept: int, key, packed, host, W, pads, at_once=True) -> Optional[torch.Tensor]:
         """Replay the graph of ``key`` among ``graphs``, of which ``kept`` are kept, after capturing it if need be.  ``pads``: the
         tokens, sequences and wanted rows that it is sized for, the longest piece of a sequence, the longest sequence, whether it is
         a step of single tokens."""
@@ -408,7 +416,7 @@ class Engine:
             buf.token_ids[:B].copy_(self._device_tokens, non_blocking=True)
         self.last_h2d_bytes = buf.h2d_bytes
         def batch(capturing=False):
-            return self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, None if capturing else host, capturing=capturing)
+            return self._batch(buf, t_pad, b_pad, w_pad, max_q, ctx_pad, is_decode, None if capturing else host, at_once, capturing)
         if g["graph"] is None and not is_decode and not g["plain"]:
             self._capture(g, batch(capturing=True))              # (a prompt of this size has run before)
         if g["graph"] is None:

@@ -18,11 +18,37 @@ from .block import _defer_enabled
 from .norm import RMSNorm
 from .plain import plain_layer
 
-# Up to one tile of tokens the one kernel is the faster one: a step before and now, microseconds, 28 layers of 0.6b sizes with 1, 2 and 8
-# sequences 758, 853, 856 -> 667, 769, 764; 1.7b with 1 and 4 1,131, 1,159 -> 937, 1,006, with 8 of 700 to 1,300 tokens 1,280 -> 1,248;
-# 4b with 1 (900 tokens), 4 and 8 2,080, 2,114, 2,227 -> 1,971, 1,947, 2,068; 8b with 1 and 8 2,961, 3,096 -> 2,761, 3,058.  A second tile of
-# tokens: 0.6b with 16 884 -> 880, 8b 3,537 -> 4,000.
-MAX_TOKENS = 8
+MAX_TOKENS = 8         # a tile; with a second one (9 to 16 sequences) a step of 0.6b sizes took 880 us for 884, of 8b sizes 4,000 for 3,537
+# What the kernel's registers were measured with: activations of one pass over k for the products that read the stream or the heads, of three
+# for down.  Two passes and seven (32b sizes: 5,120 wide, 64 heads, 25,600) are 1 to 4 % slower than the layers' own kernels with one or two sequences, 5 to 12 %
+# with more.
+MAX_WIDTH, MAX_INTER = 4096, 12288
+# From here on (8b sizes, 4,096) a block reads so much activation with more than four sequences that only short contexts are faster.
+WIDE = 3072
+
+
+def pays(n_tokens: int, hidden: int, longest: int, total: int, room: int) -> bool:
+    """Whether a step of ``n_tokens`` sequences (padded), whose keys are ``total`` in all and ``longest`` at most, in a batch sized for ``room`` keys
+    a sequence, is faster as one kernel.  Its attention cuts every sequence into as many parts as if all were the longest, and a
+    part stays with its block: few long sequences among short ones leave most blocks idle, which the layers' own
+    attention does not (it deals out all sequences' pages beyond 4,096 keys, and finer parts before).  One kernel over the layers' own, 28 layers of 0.6b and 1.7b sizes,
+    36 of 4b and 8b, device time of a whole step:
+    * one sequence, up to 32,000 keys: 0.79 to 0.99;
+    * two: up to 8,192 keys 0.87 to 1.00, one long and one short 0.89 to 0.99, with 16,000 and a short one 1.02;
+    * three and four, one long among short ones: up to 2,048 keys 0.81 to 1.01, 3,060 0.96 to 1.03, 4,090 1.00 to 1.04; as long as another, or falling to
+      half of the longest: up to 8,192 0.72 to 1.02 (0.89 to 1.02 at 8b sizes), 16,000 0.95 to 1.10;
+    * five to eight, 8b sizes: 250 keys 0.98 to 0.99, 500 and more 1.01 to 1.15; narrower ones, one long: 500 keys 0.93 to 1.01, 760 0.94 to 1.02, 2,040 1.00 to 1.06, 8,190 1.14 to 1.5;
+      five of a length or six falling to a half: 1,530 keys 0.95 to 1.00, 2,040 0.96 to 1.04; eight of a length: 8,192 0.87 to 1.00."""
+    if n_tokens <= 1:
+        return True
+    if n_tokens <= 2:
+        return room <= 8192
+    full = total / (n_tokens * longest)          # how much of the batch's places times the longest is there
+    if n_tokens <= 4:
+        return room <= (8192 if full >= 0.5 else 2048)
+    if hidden > WIDE:
+        return room <= 256
+    return room <= (8192 if full >= 0.9 else 1536 if full >= 0.4 else 512)
 
 
 def enabled() -> bool:
@@ -65,9 +91,15 @@ def _block_fits(block, first, hidden: int) -> bool:
         _norm(block.mixer_norm, first.mixer_norm) and _norm(block.ff_norm, first.mixer_norm)
 
 
+def fits(model) -> bool:
+    """Whether this model's decode steps may run as the one kernel, as far as its layers' kind and widths say."""
+    return model.env.act_dtype == torch.bfloat16 and all(
+        plain_layer(b) and max(model.hidden, b.mixer.nq * b.mixer.hd) <= MAX_WIDTH and b.ff.inter <= MAX_INTER for b in model.blocks)
+
+
 def takes(model, batch, cache) -> bool:
     """Whether this step's layers run as the one kernel."""
-    if not batch.is_decode or batch.n_tokens > MAX_TOKENS or model.env.act_dtype != torch.bfloat16 or _profiler.ACTIVE is not None \
+    if not batch.is_decode or batch.n_tokens > MAX_TOKENS or not batch.at_once or not fits(model) or _profiler.ACTIVE is not None \
             or not enabled():
         return False
     first = None
@@ -81,7 +113,8 @@ def takes(model, batch, cache) -> bool:
             return False
     if first is None:
         return False
-    # every block should have a unit (16 rows) of the first product and of gate | up
+    # Every block has a unit (16 rows) of the first product and of gate | up.  (Not where the two ways meet: at 256 to 1,024 wide layers with 64 to 192 units the one
+    # kernel takes 0.58 to 0.93 of the others' time too.)
     sms = torch.cuda.get_device_properties(model.env.device).multi_processor_count
     return first.mixer.qkv.n >= 16 * sms and 2 * first.ff.inter >= 16 * sms
 

@@ -196,3 +196,32 @@ def test_decode_through_the_engine(tmp_path, monkeypatch, graphs):
             ref = plain.logits(x)[n: n + len(got)].to(torch.float64)
             err = ((torch.stack(got).double().cpu() - ref).abs() / ref.abs().amax(dim=-1, keepdim=True)).max()
             assert float(err) < TOL, float(err)
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_lengths_decide_which_way_a_step_goes(tmp_path, monkeypatch, graphs):
+    """One long sequence among seven short ones runs layer by layer, a batch of a length as one kernel, in one engine after another."""
+    from plain_qwen3 import PlainQwen3
+    from rocml_b200 import Engine, StepEntry, kernels
+    config = {**CONFIGS["E"], "use_sliding_window": False, "layer_types": ["full_attention"] * 2, "num_attention_heads": 16,
+              "num_key_value_heads": 2, "intermediate_size": 1216, "max_position_embeddings": 2048}
+    folder = str(tmp_path / "m")
+    write_model(folder, config, seed=13, std=0.05)
+    plain = PlainQwen3(folder, dtype=torch.float64)
+    calls = []
+    real = kernels.decode_layers
+    monkeypatch.setattr(kernels, "decode_layers", lambda *a, **k: calls.append(a[0].shape[0]) or real(*a, **k))
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=4096, use_graphs=graphs)
+    for lens, taken in (([600] + [20] * 7, False), ([200] * 8, True), ([600], True), ([599] + [21] * 7, False)):
+        calls.clear()
+        ids = [prompt(70 + i, n, config["vocab_size"]) for i, n in enumerate(lens)]
+        slots = [eng.new_sequence() for _ in ids]
+        eng.step([StepEntry(s, x[:-3], []) for s, x in zip(slots, ids)])
+        rows = torch.stack([eng.step([StepEntry(s, [x[t]], [0]) for s, x in zip(slots, ids)]).clone() for t in (-3, -2, -1)], dim=1)
+        assert (bool(calls) == taken) or (graphs and not calls), lens          # (a replay of an earlier capture calls nothing)
+        for x, got in zip(ids, rows):
+            ref = plain.logits(x)[-3:].to(torch.float64)
+            assert float(((got.double().cpu() - ref).abs() / ref.abs().amax(dim=-1, keepdim=True)).max()) < TOL
+        for s in slots:
+            eng.release(s)
+    kernels.check_status("cuda:0")
