@@ -209,8 +209,7 @@ class Model:
                     x0.copy_(resid)
         pending = None
         sched = self.spec.schedule
-        if decode_layers.takes(self, batch, cache):
-            decode_layers.forward(self, resid, batch, cache)
+        if decode_layers.takes(self, batch, cache) and decode_layers.forward(self, resid, batch, cache):
             sched = ()
         for i, e in enumerate(sched):
             block = self.blocks[e.layer]

@@ -776,7 +776,7 @@ def decode_layers_splits(pairs: int, max_kv_len: int, device) -> int:
 
 def decode_layers(resid: torch.Tensor, first_norm: torch.Tensor, layers, nq: int, nkv: int, inter: int, head_eps: float, scale: float,
                   cos_sin: Optional[torch.Tensor], seq_slot: torch.Tensor, kv_len: torch.Tensor, block_table: torch.Tensor,
-                  splits: int = 1, wait_limit: int = 0) -> None:
+                  splits: int = 1, wait_limit: int = 0) -> bool:
     """All layers of a decode step of at most 16 tokens, one of each sequence, in one persistent kernel (bfloat16 weights and cache,
     heads of 128).  ``resid`` [T, H] float32 is the residual stream and receives the result; ``first_norm`` [H] the weight of the
     first layer's first norm.  ``layers``: for each layer (qkv [(nq + 2 nkv) * 128, H], o [H, nq * 128], gate_up [2 * inter, H] (blocks
@@ -785,11 +785,11 @@ def decode_layers(resid: torch.Tensor, first_norm: torch.Tensor, layers, nq: int
     made the layer's input).  Row t of the step belongs to sequence t: ``seq_slot`` (-1: nobody's, its stream is left without meaning),
     ``kv_len`` with the new token, ``block_table`` [slots, pages].  The new keys and values are written to their pages.  ``splits``: parts of
     a sequence's pages that blocks take.  ``wait_limit``: clock cycles after which a wait gives up and the device's status word says so
-    (0: about two seconds)."""
+    (0: about two seconds).  Returns False, and nothing has been launched, for sizes or alignments that the kernel does not take."""
     T, H = resid.shape
     dev = resid.device
     if not 1 <= T <= 16 or not layers or nkv < 1 or nq % nkv or nq // nkv > 8 or H % 64 or inter % 64:
-        raise KernelError(f"decode_layers: {T} tokens, {len(layers)} layers, {nq} heads on {nkv}, {H} and {inter} wide are not taken")
+        return False
     if resid.dtype != torch.float32 or not resid.is_contiguous():
         raise KernelError("decode_layers: the stream must be contiguous float32 [T, H]")
     if first_norm.dtype != layers[0][4].dtype or first_norm.numel() != H or not first_norm.is_contiguous():
@@ -833,7 +833,11 @@ def decode_layers(resid: torch.Tensor, first_norm: torch.Tensor, layers, nq: int
     p.first_norm, p.resid, p.xhat, p.sumsq, p.qkv, p.attn, p.h = (_ptr(t) for t in (first_norm, resid, xhat, sumsq, qkv_rows, attn, h))
     p.part_o, p.part_ml, p.counters, p.status = _ptr(part_o), _ptr(part_ml), _ptr(counters), _ptr(status_word(dev))
     p.wait_limit, p.layer = int(wait_limit), rows
-    _check(_lib().rb_decode_layers(ctypes.byref(p), _stream()), "decode_layers")
+    rc = _lib().rb_decode_layers(ctypes.byref(p), _stream())
+    if rc in (10001, 10003):
+        return False
+    _check(rc, "decode_layers")
+    return True
 
 
 @_profiled(lambda a, facts: (a["part_acc"].numel() * 4 + a["part_ml"].numel() * 4 + a["n_tokens"] * a["nq"] * a["hd"] * _esz(a["out"]), 0))

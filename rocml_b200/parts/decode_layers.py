@@ -119,8 +119,9 @@ def takes(model, batch, cache) -> bool:
     return first.mixer.qkv.n >= 16 * sms and 2 * first.ff.inter >= 16 * sms
 
 
-def forward(model, resid, batch, cache) -> None:
-    """Run the layers on the step's residual stream ``resid`` [T, H] float32, which holds the embedding's rows."""
+def forward(model, resid, batch, cache) -> bool:
+    """Run the layers on the step's residual stream ``resid`` [T, H] float32, which holds the embedding's rows.  False where the kernel
+    declines: nothing has run then, and the layers' own kernels take the step."""
     blocks = [model.blocks[e.layer] for e in model.spec.schedule]
     m, inter = blocks[0].mixer, blocks[0].ff.inter
     splits = kernels.decode_layers_splits(batch.n_tokens * m.nkv, batch.max_kv_len, resid.device)
@@ -130,6 +131,6 @@ def forward(model, resid, batch, cache) -> None:
         layers.append((b.mixer.qkv.weight, b.mixer.o.weight, b.ff.gate_up.weight, b.ff.down.weight, b.ff_norm.weight,
                        nxt.weight if nxt is not None else None, b.mixer.q_norm_w, b.mixer.k_norm_w, view.k, view.v,
                        b.ff_norm.eps, b.mixer_norm.eps))
-    kernels.decode_layers(resid, blocks[0].mixer_norm.weight, layers, m.nq, m.nkv, inter, m.qk_norm_eps, m.scale,
-                          m.position.cos_sin(batch) if m.position.inv_freq is not None else None,
-                          batch.seq_slot, batch.kv_len, cache.views[0].block_table, splits)
+    return kernels.decode_layers(resid, blocks[0].mixer_norm.weight, layers, m.nq, m.nkv, inter, m.qk_norm_eps, m.scale,
+                                 m.position.cos_sin(batch) if m.position.inv_freq is not None else None,
+                                 batch.seq_slot, batch.kv_len, cache.views[0].block_table, splits)

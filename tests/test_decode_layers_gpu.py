@@ -225,3 +225,44 @@ def test_lengths_decide_which_way_a_step_goes(tmp_path, monkeypatch, graphs):
         for s in slots:
             eng.release(s)
     kernels.check_status("cuda:0")
+
+
+def test_what_the_kernel_declines_leaves_the_stream_alone():
+    """A weight off 16 bytes, and more query heads a key/value head than a block takes."""
+    from rocml_b200 import kernels
+    lens, H, inter = [30, 9], 512, 1216
+    for nq, nkv, shift in ((16, 2, 1), (18, 2, 0)):
+        layers, x, table, cs = make(2, H, inter, nq, nkv, lens)
+        for L in layers:
+            w = torch.empty(H * nq * 128 + 1, dtype=torch.bfloat16, device=DEV)[shift:][:H * nq * 128].view(H, nq * 128)
+            L["o"] = w.copy_(L["o"])
+        took = []
+        real, kernels.decode_layers = kernels.decode_layers, lambda *a: took.append(real(*a))
+        try:
+            got, args = run(layers, x, table, cs, lens, nq, nkv, inter, 1e-6, True, 1)
+        finally:
+            kernels.decode_layers = real
+        assert took == [False] and torch.equal(got, x)
+        for L, a in zip(layers, args):
+            assert torch.equal(a[8].view(torch.int16), L["ck"].view(torch.int16)) and torch.equal(a[9].view(torch.int16), L["cv"].view(torch.int16))
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_a_step_that_the_kernel_declines_runs_layer_by_layer(tmp_path, monkeypatch, graphs):
+    """The library refuses the step: the answers are those of the layers' own kernels, bit for bit."""
+    from rocml_b200 import Engine, StepEntry, kernels
+    config = {**CONFIGS["E"], "use_sliding_window": False, "layer_types": ["full_attention"] * 2, "num_attention_heads": 16,
+              "num_key_value_heads": 2, "intermediate_size": 1216}
+    folder = str(tmp_path / "m")
+    write_model(folder, config, seed=9, std=0.05)
+    ids = prompt(70, 40, config["vocab_size"])
+    rows, refused = {}, []
+    monkeypatch.setattr(kernels._lib(), "rb_decode_layers", lambda *a: refused.append(1) or 10003)
+    for on in ("1", "0"):
+        monkeypatch.setenv("RB_DECODE_LAYERS", on)
+        eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=1024, use_graphs=graphs)
+        slot = eng.new_sequence()
+        eng.step([StepEntry(slot, ids[:35], [])])
+        rows[on] = torch.stack([eng.step([StepEntry(slot, [i], [0])]).clone() for i in ids[35:]])
+        assert bool(refused) == (on == "1") or on == "0"
+    assert torch.equal(rows["1"], rows["0"])
