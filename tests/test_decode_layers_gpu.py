@@ -107,6 +107,10 @@ CASES = [
     ([3] * 16, 4608, 8256, 40, 8, 1),                                   # three and five passes
     ([130, 7, 64], 5120, 25600, 64, 8, 2),                              # more units a block than are kept: groups
     ([900], 768, 2560, 8, 8, 1),                                        # more stages of keys than the ring has
+    ([600, 1], 192, 320, 8, 2, 9),                                      # parts that are merged in two rounds of eight, the second ragged
+    ([2300], 256, 512, 8, 4, 18),                                       # three rounds
+    ([3000, 800, 100, 17], 512, 1216, 16, 4, 9),                        # lengths as unequal as they come, with parts that have no page
+    ([1040], 128, 192, 2, 1, 16),                                       # two whole rounds
 ]
 
 
@@ -266,3 +270,25 @@ def test_a_step_that_the_kernel_declines_runs_layer_by_layer(tmp_path, monkeypat
         rows[on] = torch.stack([eng.step([StepEntry(slot, [i], [0])]).clone() for i in ids[35:]])
         assert bool(refused) == (on == "1") or on == "0"
     assert torch.equal(rows["1"], rows["0"])
+
+
+def test_a_long_sequence_through_the_engine(tmp_path, monkeypatch):
+    """One sequence of some 2,300 tokens: its pages are taken in more than eight parts."""
+    from plain_qwen3 import PlainQwen3
+    from rocml_b200 import Engine, StepEntry, kernels
+    config = {**CONFIGS["E"], "use_sliding_window": False, "layer_types": ["full_attention"] * 2, "num_attention_heads": 16,
+              "num_key_value_heads": 2, "intermediate_size": 1216, "max_position_embeddings": 4096}
+    folder = str(tmp_path / "m")
+    write_model(folder, config, seed=11, std=0.05)
+    ids = prompt(3, 2310, config["vocab_size"])
+    ref = PlainQwen3(folder, dtype=torch.float64).logits(ids)[-8:].to(torch.float64)
+    parts = []
+    real = kernels.decode_layers
+    monkeypatch.setattr(kernels, "decode_layers", lambda *a, **k: parts.append(a[12]) or real(*a, **k))
+    eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=2560)
+    slot = eng.new_sequence()
+    eng.step([StepEntry(slot, ids[:-8], [])])
+    got = torch.cat([eng.step([StepEntry(slot, [i], [0])]).clone() for i in ids[-8:]])
+    kernels.check_status("cuda:0")
+    assert parts and min(parts) > 8
+    assert float(((got.double().cpu() - ref).abs() / ref.abs().amax(dim=-1, keepdim=True)).max()) < TOL
