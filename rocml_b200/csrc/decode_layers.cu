@@ -1,4 +1,4 @@
-// All layers of a decode step of a plain dense decoder in ONE persistent kernel (bfloat16, up to 16 tokens, one of each
+// All layers of a decode step of a plain dense decoder in ONE persistent kernel (bfloat16, up to eight tokens, one of each
 // sequence): norm, q | k | v, attention over the paged cache, output projection, norm, gate | up with SiLU, down.
 //
 // A step of a few tokens is bound by reading the weights once.  As five kernels a layer, each of which first waits for the one
@@ -64,8 +64,8 @@ constexpr int MAX_LAYERS = 38;                // of a launch: what its parameter
 constexpr float NEG_BIG = -1e30f;
 constexpr float LOG2E = 1.4426950408889634f;
 static_assert(STAGE == 2 * SK * HD * 2 && STAGES % CW == 0, "a stage holds 16 keys and 16 values");
-template <int NT>
-constexpr int CPW = NT == 1 ? 2 : 1;          // stages a warp takes of a unit: what it holds activations for (64 registers)
+constexpr int TT = 8;                         // tokens of the MMA's tile
+constexpr int CPW = 2;                        // stages a warp takes of a unit: what it holds activations for (64 registers)
 
 struct LayerPtrs {
     const void *ff_norm, *next_norm;                     // the norm behind the mixer, and the next layer's first (null: none)
@@ -162,26 +162,24 @@ __device__ __forceinline__ uint32_t bits_any(const void* p, int f32, int i) {
 }
 __device__ __forceinline__ float value_any(uint32_t bits, int f32) { return __uint_as_float(f32 ? bits : bits << 16); }
 
-template <int NT>
 struct Smem {
     uint8_t ring[STAGES][STAGE];
     union {
-        float part[2][CW][NT * 8][TOK];       // the warps' sums of the units in work, two rounds in turn
+        float part[2][CW][TT][TOK];           // the warps' sums of the units in work, two rounds in turn
         float o[CW][MERGE_HEADS][HD];         // the warps' partial attention results
     };
-    float keep[GROUP][NT * 8][UR];            // sums of earlier passes
+    float keep[GROUP][TT][UR];                // sums of earlier passes
     __nv_bfloat16 q[8][HD];                   // query heads, swizzled rows
     __nv_bfloat16 k_new[HD], v_new[HD];
     float m[CW + 1][MAX_G], l[CW + 1][MAX_G]; // the warps' and the new key's maxima and sums
-    float rstd[NT * 8];
+    float rstd[TT];
     uint64_t full[STAGES], empty[STAGES];
     Step step;
-    int slot[NT * 8], old[NT * 8], page[NT * 8];      // of every sequence: its slot, the keys of earlier steps, the new key's page
+    int slot[TT], old[TT], page[TT];          // of every sequence: its slot, the keys of earlier steps, the new key's page
     int abort, last;
 };
-template <int NT>
-constexpr int SMEM = (int)sizeof(Smem<NT>);
-static_assert(SMEM<2> <= 227 * 1024, "a block's shared memory");
+constexpr int SMEM = (int)sizeof(Smem);
+static_assert(SMEM <= 227 * 1024, "a block's shared memory");
 
 // What every warp keeps while it walks through the ring: producer and computing warps make the same steps in the same order.
 struct Walk {
@@ -255,14 +253,13 @@ struct Item {
 // ---- the producer ------------------------------------------------------------------------------------------
 // One thread walks, so that a stage costs a few instructions (a warp in step, with an arrival each: 340 to 460 cycles a stage, which set the
 // pace of the whole step).
-template <int NT>
 struct Producer {
-    Smem<NT>& s;
+    Smem& s;
     Walk w;
     Waits waits;
     int issued = 0;
 
-    __device__ Producer(Smem<NT>& s, Waits waits) : s(s), waits(waits) {}
+    __device__ Producer(Smem& s, Waits waits) : s(s), waits(waits) {}
 
     // The next stage is free, and its barrier knows what will land in it; false: given up.  (Once a wait has run out no
     // stage is handed back, see Compute::taken, so that none is armed while a copy into it may be on its way, and the drain at the end
@@ -354,9 +351,8 @@ struct Producer {
 };
 
 // ---- the warps that compute -----------------------------------------------------------------------------------
-template <int NT>
 struct Compute {
-    Smem<NT>& s;
+    Smem& s;
     Walk w;
     Waits waits;
     const Step& p;
@@ -364,7 +360,7 @@ struct Compute {
     unsigned turn = 0;                        // rounds of units summed so far: which half of s.part
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
 
-    __device__ Compute(Smem<NT>& s, Waits waits) : s(s), waits(waits), p(s.step) {}
+    __device__ Compute(Smem& s, Waits waits) : s(s), waits(waits), p(s.step) {}
 
     // The stage's copy has landed (or a wait has run out); and whether the stage may be handed back when it has been read: not once a wait
     // has run out, since the copy may then still be on its way.  Two uses of a stage are the same warp's or have a barrier of the
@@ -394,34 +390,28 @@ struct Compute {
         compute_sync();
     }
 
-    // 1/RMS of every token's row, from the units' sums of squares: a warp a token (two with 16 tokens).  The loads of the first 256 units
+    // 1/RMS of every token's row, from the units' sums of squares: a warp a token.  The loads of the first 256 units
     // go out ahead of the first unit's products, the sums follow behind them.
-    struct Squares { float v[NT][8]; };
+    struct Squares { float v[8]; };
     __device__ void ask_squares(Squares& q) {
         const int n = p.H / UR, T = p.T;
         const float* from = p.sumsq + (warp * n + lane);
 #pragma unroll
-        for (int i = 0; i < NT; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                q.v[i][j] = 0.f;
-                load_if(warp + i * CW < T && j * 32 + lane < n, q.v[i][j], from + (i * CW * n + j * 32));
-            }
+        for (int j = 0; j < 8; ++j) {
+            q.v[j] = 0.f;
+            load_if(warp < T && j * 32 + lane < n, q.v[j], from + j * 32);
+        }
     }
     __device__ void row_scales(const Squares& q, float eps) {
         const int n = p.H / UR;
+        if (warp < p.T) {
+            float sum = 0.f;
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            const int t = warp + i * CW;
-            if (t < p.T) {
-                float sum = 0.f;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) sum += q.v[i][j];
+            for (int j = 0; j < 8; ++j) sum += q.v[j];
 #pragma unroll 1
-                for (int u = 256 + lane; u < n; u += 32) sum += __ldcg(p.sumsq + (t * n + u));
-                sum = warp_sum(sum);
-                if (lane == 0) s.rstd[t] = rsqrtf(sum * p.inv_H + eps);
-            }
+            for (int u = 256 + lane; u < n; u += 32) sum += __ldcg(p.sumsq + (warp * n + u));
+            sum = warp_sum(sum);
+            if (lane == 0) s.rstd[warp] = rsqrtf(sum * p.inv_H + eps);
         }
     }
 
@@ -496,7 +486,7 @@ struct Compute {
         int first, mine, group, my_unit, my_stage;      // (unit and stage of those in work)
         bool scaled;
         float eps;
-        const __nv_bfloat16* row[NT];
+        const __nv_bfloat16* row;
         Out out;
     };
     __device__ void prepare(Job& job, int i) {
@@ -507,23 +497,22 @@ struct Compute {
         job.mine = w.share(ps, job.first);
         job.group = ps.passes == 1 ? job.mine : GROUP;
         job.my_unit = warp / ps.warps;
-        job.my_stage = (warp - job.my_unit * ps.warps) * CPW<NT>;
+        job.my_stage = (warp - job.my_unit * ps.warps) * CPW;
         job.scaled = phase == QKV || phase == GATED;
         job.eps = phase == QKV ? L.in_eps : L.ff_eps;
         const __nv_bfloat16* x = phase == OUT ? p.attn : (phase == DOWN ? p.h : p.xhat);
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) job.row[nt] = x + (min(nt * 8 + gq, T - 1) * ps.K + job.my_stage * KC + tq * 16);
-        job.out = output(phase, phase == OUT ? L.ff_norm : L.next_norm, threadIdx.x / UR % (8 * NT));
+        job.row = x + (min(gq, T - 1) * ps.K + job.my_stage * KC + tq * 16);
+        job.out = output(phase, phase == OUT ? L.ff_norm : L.next_norm, threadIdx.x / UR % TT);
     }
 
     __device__ void product(Job& job) {
-        constexpr int C = CPW<NT>, OUTS = UR * 8 * NT, A = NT == 1 ? 4 : 2;
+        constexpr int C = CPW, OUTS = UR * TT, A = 4;
         const Plan& ps = p.plan[job.phase];
         const int first = job.first, mine = job.mine, group = job.group, my_unit = job.my_unit, my_stage = job.my_stage, K = ps.K;
         // the lane's row of the four 8 x 8 matrices of a 16 x 16 A operand: rows 0..7 and 8..15 of two neighbouring chunks
         const uint32_t lane_ring = sm100::smem_u32(s.ring[0]) + (lane & 15) * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
         // who sums what: a thread row r of token t of one of the units in work, and (short sums) of the next but one
-        const int r = threadIdx.x & 15, t = threadIdx.x / UR % (8 * NT);
+        const int r = threadIdx.x & 15, t = threadIdx.x / UR % TT;
         Out& out = job.out;
 #pragma unroll 1
         for (int g0 = 0; g0 < mine; g0 += group)
@@ -534,18 +523,15 @@ struct Compute {
                 // the tile beyond the last token repeat it and are dropped.
                 const int blocks = (min(nc, my_stage + C) - my_stage) * (KC / KB);
                 const int nb = min(blocks, K / KB - (c0 + my_stage) * (KC / KB));
-                uint4 B[C * (KC / KB)][NT][2];
+                uint4 B[C * (KC / KB)][2];
+                const __nv_bfloat16* row = job.row + c0 * KC;
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    const __nv_bfloat16* row = job.row[nt] + c0 * KC;
+                for (int j = 0; j < C * (KC / KB); ++j)
 #pragma unroll
-                    for (int j = 0; j < C * (KC / KB); ++j)
-#pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            B[j][nt][half] = make_uint4(0u, 0u, 0u, 0u);
-                            load_if(j < nb, B[j][nt][half], row + j * KB + half * 8);
-                        }
-                }
+                    for (int half = 0; half < 2; ++half) {
+                        B[j][half] = make_uint4(0u, 0u, 0u, 0u);
+                        load_if(j < nb, B[j][half], row + j * KB + half * 8);
+                    }
                 bool scales = job.scaled && g0 == 0 && pass == 0;
                 Squares squares;
                 if (scales) ask_squares(squares);
@@ -556,11 +542,9 @@ struct Compute {
                     const int units = min(ps.units, end - i);
                     int unit = threadIdx.x / OUTS;
                     if (last && unit < units) begin(out, first + (i + unit) * (int)gridDim.x, r);
-                    float acc[NT][A][4];                      // A chains of MMAs, added at the end
+                    float acc[A][4];                          // A chains of MMAs, added at the end
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                        for (int k = 0; k < A * 4; ++k) acc[nt][k >> 2][k & 3] = 0.f;
+                    for (int k = 0; k < A * 4; ++k) acc[k >> 2][k & 3] = 0.f;
                     if (my_unit < units) {
                         Walk at = w;
                         at.skip(my_unit * nc + my_stage);
@@ -579,29 +563,24 @@ struct Compute {
                                             ldmatrix_x4((a ^ (k * 32)) + j * (UR * 128), m[j & 1][k][0], m[j & 1][k][1], m[j & 1][k][2], m[j & 1][k][3]);
                                     if (j > 0 && c * (KC / KB) + j - 1 < nb)
 #pragma unroll
-                                        for (int k = 0; k < 4; ++k)
-#pragma unroll
-                                            for (int nt = 0; nt < NT; ++nt) {
-                                                const uint4 b = B[c * (KC / KB) + (j > 0 ? j - 1 : 0)][nt][k >> 1];
-                                                mma_tiles::mma_bf16(acc[nt][k % A], m[(j & 1) ^ 1][k], k & 1 ? b.z : b.x, k & 1 ? b.w : b.y);
-                                            }
+                                        for (int k = 0; k < 4; ++k) {
+                                            const uint4 b = B[c * (KC / KB) + (j > 0 ? j - 1 : 0)][k >> 1];
+                                            mma_tiles::mma_bf16(acc[k % A], m[(j & 1) ^ 1][k], k & 1 ? b.z : b.x, k & 1 ? b.w : b.y);
+                                        }
                                 }
                                 give_back(at, whole);
                                 at.skip(1);
                             }
                         // the warps' sums meet; the other half of s.part is free: its readers have passed this barrier's predecessor
+                        float* to = &s.part[turn & 1][warp][tq * 2][gq];
 #pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) {
-                            float* to = &s.part[turn & 1][warp][nt * 8 + tq * 2][gq];
+                        for (int a = 2; a < A; ++a)
 #pragma unroll
-                            for (int a = 2; a < A; ++a)
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) acc[nt][a & 1][k] += acc[nt][a][k];
-                            to[0] = acc[nt][0][0] + acc[nt][1][0];
-                            to[TOK] = acc[nt][0][1] + acc[nt][1][1];
-                            to[8] = acc[nt][0][2] + acc[nt][1][2];
-                            to[TOK + 8] = acc[nt][0][3] + acc[nt][1][3];
-                        }
+                            for (int k = 0; k < 4; ++k) acc[a & 1][k] += acc[a][k];
+                        to[0] = acc[0][0] + acc[1][0];
+                        to[TOK] = acc[0][1] + acc[1][1];
+                        to[8] = acc[0][2] + acc[1][2];
+                        to[TOK + 8] = acc[0][3] + acc[1][3];
                     }
                     if (scales) row_scales(squares, job.eps);
                     scales = false;
@@ -615,7 +594,7 @@ struct Compute {
                         float sum = 0.f;
 #pragma unroll
                         for (int k = 0; k < CW; ++k)
-                            if (k < ps.warps) sum += from[k * (8 * NT * TOK)];
+                            if (k < ps.warps) sum += from[k * (TT * TOK)];
                         if (ps.passes > 1) {
                             float* kept = &s.keep[i - g0][t][r];
                             if (pass > 0) sum += *kept;
@@ -922,10 +901,9 @@ struct Compute {
     }
 };
 
-template <int NT>
 __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_constant__ Params params) {
     extern __shared__ __align__(1024) uint8_t raw[];
-    Smem<NT>& s = *reinterpret_cast<Smem<NT>*>(raw);
+    Smem& s = *reinterpret_cast<Smem*>(raw);
     if ((sm100::smem_u32(raw) & 1023) != 0) {              // the swizzle's atoms (a block's shared memory has always begun on one)
         if (threadIdx.x == 0) atomicExch(params.step.status, RB_ERR_BAD_ALIGN);
         return;
@@ -954,12 +932,12 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
     if (threadIdx.x >= CTHREADS) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (threadIdx.x == CTHREADS) {
-            Producer<NT> producer(s, waits);
+            Producer producer(s, waits);
             producer.run(s.step, params);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
-        Compute<NT> compute(s, waits);
+        Compute compute(s, waits);
         compute.run();
     }
 }
@@ -1028,7 +1006,7 @@ struct rb_DecodeStep {
 // not take these sizes or pointers and nothing was launched.
 extern "C" int rb_decode_layers(const void* step, void* stream) {
     const rb_DecodeStep& q = *static_cast<const rb_DecodeStep*>(step);
-    if (q.T < 1 || q.T > 16 || q.layers < 1 || q.splits < 1 || q.n_pages < 1 || q.H % 64 || q.I % 64 || q.H <= 0 || q.I <= 0 || q.nkv < 1 ||
+    if (q.T < 1 || q.T > TT || q.layers < 1 || q.splits < 1 || q.n_pages < 1 || q.H % 64 || q.I % 64 || q.H <= 0 || q.I <= 0 || q.nkv < 1 ||
         q.nq % q.nkv || q.nq / q.nkv > MAX_G)
         return RB_ERR_BAD_SIZE;
     // (indices are 32-bit)
@@ -1047,8 +1025,7 @@ extern "C" int rb_decode_layers(const void* step, void* stream) {
     if (e != cudaSuccess) return (int)e;
     const Ready* ready = nullptr;
     int rc = g_ready.get(device, &ready, [&](Ready& r) {
-        cudaError_t a = cudaFuncSetAttribute(decode_layers_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM<1>);
-        if (a == cudaSuccess) a = cudaFuncSetAttribute(decode_layers_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM<2>);
+        cudaError_t a = cudaFuncSetAttribute(decode_layers_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (a == cudaSuccess) a = cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, device);
         return (int)a;
     });
@@ -1066,15 +1043,14 @@ extern "C" int rb_decode_layers(const void* step, void* stream) {
     p.wait_limit = (unsigned)(q.wait_limit > 0 && q.wait_limit < sm100::RB_WAIT_CYCLES ? q.wait_limit : sm100::RB_WAIT_CYCLES);
     const int work[PHASES] = {(q.nq + 2 * q.nkv) * HD / UR, 0, q.H / UR, 2 * q.I / UR, q.H / UR};
     const int inputs[PHASES] = {q.H, KC, q.nq * HD, q.H, q.I};
-    const int a_warp = q.T <= 8 ? CPW<1> : CPW<2>;
     for (int i = 0; i < PHASES; ++i) {
         Plan& a = p.plan[i];
         a.each = work[i] / ready->sms; a.rest = work[i] % ready->sms;
         a.K = inputs[i]; a.stages = (a.K + KC - 1) / KC;
-        a.passes = (a.stages + CW * a_warp - 1) / (CW * a_warp);
+        a.passes = (a.stages + CW * CPW - 1) / (CW * CPW);
         a.per = (a.stages + a.passes - 1) / a.passes;
-        a.warps = (a.per + a_warp - 1) / a_warp;
-        a.units = a.warps > 4 ? 1 : (a.warps > 2 ? 2 : (q.T <= 8 ? 4 : 2));
+        a.warps = (a.per + CPW - 1) / CPW;
+        a.units = a.warps > 4 ? 1 : (a.warps > 2 ? 2 : 4);
     }
     const unsigned long long cached = (unsigned long long)q.n_pages * q.nkv * RB_PAGE;
     for (int i0 = 0; i0 < q.layers; i0 += MAX_LAYERS) {
@@ -1097,14 +1073,14 @@ extern "C" int rb_decode_layers(const void* step, void* stream) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(ready->sms);
         cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = p.T <= 8 ? SMEM<1> : SMEM<2>;
+        cfg.dynamicSmemBytes = SMEM;
         cfg.stream = (cudaStream_t)stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeCooperative;
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = p.T <= 8 ? cudaLaunchKernelEx(&cfg, decode_layers_kernel<1>, params) : cudaLaunchKernelEx(&cfg, decode_layers_kernel<2>, params);
+        e = cudaLaunchKernelEx(&cfg, decode_layers_kernel, params);
         if (e != cudaSuccess) return (int)e;
     }
     return RB_OK;

@@ -777,7 +777,7 @@ def decode_layers_splits(pairs: int, max_kv_len: int, device) -> int:
 def decode_layers(resid: torch.Tensor, first_norm: torch.Tensor, layers, nq: int, nkv: int, inter: int, head_eps: float, scale: float,
                   cos_sin: Optional[torch.Tensor], seq_slot: torch.Tensor, kv_len: torch.Tensor, block_table: torch.Tensor,
                   splits: int = 1, wait_limit: int = 0) -> bool:
-    """All layers of a decode step of at most 16 tokens, one of each sequence, in one persistent kernel (bfloat16 weights and cache,
+    """All layers of a decode step of at most eight tokens, one of each sequence, in one persistent kernel (bfloat16 weights and cache,
     heads of 128).  ``resid`` [T, H] float32 is the residual stream and receives the result; ``first_norm`` [H] the weight of the
     first layer's first norm.  ``layers``: for each layer (qkv [(nq + 2 nkv) * 128, H], o [H, nq * 128], gate_up [2 * inter, H] (blocks
     of 16 gate rows and the 16 up rows of the same outputs), down [H, inter], norm behind the mixer, next layer's first norm (None: no
@@ -788,7 +788,7 @@ def decode_layers(resid: torch.Tensor, first_norm: torch.Tensor, layers, nq: int
     (0: about two seconds).  Returns False, and nothing has been launched, for sizes or alignments that the kernel does not take."""
     T, H = resid.shape
     dev = resid.device
-    if not 1 <= T <= 16 or not layers or nkv < 1 or nq % nkv or nq // nkv > 8 or H % 64 or inter % 64:
+    if not 1 <= T <= 8 or not layers or nkv < 1 or nq % nkv or nq // nkv > 8 or H % 64 or inter % 64:
         return False
     if resid.dtype != torch.float32 or not resid.is_contiguous():
         raise KernelError("decode_layers: the stream must be contiguous float32 [T, H]")

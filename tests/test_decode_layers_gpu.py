@@ -101,10 +101,10 @@ CASES = [
     ([300], 512, 1216, 16, 8, 5),                                       # parts, and five pages for them
     ([1, 700, 65], 576, 1088, 6, 3, 4),                                 # a sequence with fewer pages than parts; k 64 past a stage
     ([40, 0, 100, 0], 1024, 192, 5, 5, 2),                              # places without a sequence; four units in work
-    ([10 + 37 * i for i in range(9)], 320, 512, 14, 2, 1),              # a second tile of tokens
-    ([200 - 11 * i for i in range(16)], 2112, 704, 12, 4, 3),
+    ([10 + 37 * i for i in range(8)], 320, 512, 14, 2, 1),              # seven heads a group
+    ([200 - 11 * i for i in range(8)], 2112, 704, 12, 4, 3),
     ([77, 5], 4160, 4672, 33, 33, 1),                                   # two passes over k; 33 heads
-    ([3] * 16, 4608, 8256, 40, 8, 1),                                   # three and five passes
+    ([3] * 8, 4608, 8256, 40, 8, 1),                                   # two and three passes
     ([130, 7, 64], 5120, 25600, 64, 8, 2),                              # more units a block than are kept: groups
     ([900], 768, 2560, 8, 8, 1),                                        # more stages of keys than the ring has
     ([600, 1], 192, 320, 8, 2, 9),                                      # parts that are merged in two rounds of eight, the second ragged
