@@ -37,13 +37,6 @@ constexpr int MAX_CLUSTER = 16;   // blocks of one (sequence, head group) that c
 constexpr float NEG_BIG = -1e30f;
 constexpr float LOG2E = 1.4426950408889634f;
 
-// 2^x on the special-function unit, one instruction (x <= 0 here, -inf gives 0); the library's exp2f
-// adds range handling that the softmax does not need.
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 // Blocks of one (sequence, head group) as one thread-block cluster (CL): see the merge below.
 __device__ __forceinline__ void cluster_sync_all() {
@@ -249,11 +242,6 @@ constexpr int PROP_MAX_SEQS = 256;
 // half the accumulator registers of the layout with 16 head rows, of which a group of 4 fills a quarter.
 // P leaves the first product with keys along the lanes' groups and enters the second with keys along a
 // lane's pairs: one movmatrix per 8 keys transposes it in registers.
-__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
-    uint32_t d;
-    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
-    return d;
-}
 
 // A row's result from its accumulated values A, sum L and maximum M (in powers of two: scores carry the factor
 // log2 e); with a sink score the denominator has the term e^sink as well.

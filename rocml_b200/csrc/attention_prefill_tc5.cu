@@ -33,6 +33,7 @@
 #include <unordered_map>
 
 using namespace sm100;
+using rb::ex2;
 
 namespace {
 constexpr int BMQ = 128;      // query rows per block
@@ -60,13 +61,6 @@ struct Sizes {
     static constexpr int TMEM_COLS = HD <= 128 ? 256 : 512;
 };
 
-// 2^x on the special-function unit, one instruction (x <= 0 here, -inf gives 0); the library's exp2f
-// adds range handling that the softmax does not need.
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 // Two float32 operations in one instruction (sm_100): the softmax threads are bound by the instructions
 // they issue, and a pair of neighbouring scores sits in a pair of neighbouring registers anyway.
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
@@ -442,23 +436,6 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    });
-    return fn;
-}
-
 // [rows, cols] bf16 with row stride ld (elements), read in boxes of box_rows x 64 columns, 128-byte swizzle.
 int make_map(const void* ptr, long long rows, long long cols, long long ld, int box_rows, CUtensorMap* out) {
     struct Key {
@@ -478,7 +455,7 @@ int make_map(const void* ptr, long long rows, long long cols, long long ld, int 
         auto it = cache.find(key);
         if (it != cache.end()) { *out = it->second; return RB_OK; }
     }
-    EncodeTiledFn fn = encode_fn();
+    sm100::EncodeTiledFn fn = sm100::encode_fn();
     if (!fn) return RB_ERR_NO_DRIVER_FN;
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)ld * 2};

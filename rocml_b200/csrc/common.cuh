@@ -163,6 +163,13 @@ __device__ __forceinline__ float gelu_tanh(float z) {
 }
 // gelu as it is: z / 2 * (1 + erf(z / sqrt(2)))
 __device__ __forceinline__ float gelu_erf(float z) { return 0.5f * z * (1.f + erff(z * 0.7071067811865476f)); }
+// 2^x on the special-function unit, one instruction (for x <= 0 as in a softmax, where -inf gives 0); the library's
+// exp2f adds range handling that a softmax does not need.
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
 
 // Four neighbouring elements at once (the pointer on 4 elements' alignment).

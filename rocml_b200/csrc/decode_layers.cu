@@ -42,6 +42,7 @@
 using namespace rb;
 using mma_tiles::ldmatrix_x4;
 using mma_tiles::ldmatrix_x4_trans;
+using mma_tiles::movmatrix_trans;
 using mma_tiles::pack_bf16;
 using mma_tiles::tile_addr;
 
@@ -116,16 +117,6 @@ struct Params {
 };
 static_assert(sizeof(Params) <= 32764, "what a launch's parameters may hold");
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
-    uint32_t d;
-    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
-    return d;
-}
 __device__ __forceinline__ void load_unit(uint32_t dst, const CUtensorMap* map, int row, int kb, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %3, %5}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(row), "r"(kb) : "memory");
@@ -945,19 +936,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
 struct Ready { int sms = 0; };
 PerDevice<Ready> g_ready;
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-    static const EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
-        return ok ? (EncodeTiledFn)p : nullptr;
-    }();
-    return fn;
-}
 int encode(const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, CUtensorMap* out) {
-    const EncodeTiledFn fn = encode_fn();
+    const sm100::EncodeTiledFn fn = sm100::encode_fn();
     if (fn == nullptr) return RB_ERR_NO_DRIVER_FN;
     const cuuint32_t one[4] = {1, 1, 1, 1};
     const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -1140,23 +1140,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 namespace {
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    });
-    return fn;
-}
-
 struct MapKey {
     const void* ptr;
     long long rows, K, ld;
@@ -1187,7 +1170,7 @@ int tensor_map(const void* ptr, long long rows, long long K, long long ld, int b
         auto it = cache.find(key);
         if (it != cache.end()) { *out = it->second; return RB_OK; }
     }
-    EncodeTiledFn fn = encode_fn();
+    sm100::EncodeTiledFn fn = sm100::encode_fn();
     if (!fn) return RB_ERR_NO_DRIVER_FN;
     cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};

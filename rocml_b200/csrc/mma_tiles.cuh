@@ -56,4 +56,11 @@ __device__ __forceinline__ void load_tile(__nv_bfloat16* tile, const __nv_bfloat
     }
 }
 
+
+// The transpose of an 8 x 8 tile of 16-bit values, a register a lane (a warp).
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
+    uint32_t d;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
 }  // namespace mma_tiles
