@@ -41,7 +41,8 @@ def _model_args(p):
 
 def _profile_args(p):
     p.add_argument("--profile", action="store_true",
-                   help="time every kernel and print the table against the device's limits after the run")
+                   help="time every kernel and print the table against the device's limits after the run (steps run "
+                        "layer by layer for it, also those that are one kernel otherwise)")
     p.add_argument("--profile-json", default=None, metavar="PATH", help="write that table as JSON")
     p.add_argument("--profile-layers", action="store_true", help="with --profile: also the table by layer")
 

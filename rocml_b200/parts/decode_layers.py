@@ -2,8 +2,11 @@
 
 The kernel stands for the layers of a plain dense decoder: pre-norm blocks of grouped-query attention (heads of 128 with or
 without per-head norm and rotation, every earlier key visible) and a SiLU-gated feed-forward, RMS norms, bfloat16 weights
-without biases, all layers alike.  Any other layer, more than eight tokens and a step under the profiler (which times the
-kernels of a layer one by one) run layer by layer as always.
+without biases, all layers alike.  Any other layer, more than eight tokens, lengths at which it does not pay (``pays``) and a step under the profiler (which times the
+kernels of a layer one by one, so its table shows kernels that the step does not launch otherwise) run layer by layer as always.
+
+The kernel holds every multiprocessor from the first layer to the last: what other streams have queued waits for a whole step instead of
+running beside its kernels.  ``RB_DECODE_LAYERS=0``, read when a step's size is first run or captured, avoids that.
 """
 from __future__ import annotations
 
