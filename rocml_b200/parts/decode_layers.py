@@ -36,25 +36,23 @@ def pays(n_tokens: int, hidden: int, longest: int, total: int, room: int) -> boo
     part stays with its block: few long sequences among short ones leave most blocks idle.  The layers' own attention has finer parts, and from four sequences of
     more than 4,096 keys on it deals all pages out equally, which costs more where they are equal anyway: the rule has a step there.
     One kernel over the layers' own, 28 layers of 0.6b and 1.7b sizes, 36 of 4b and 8b, device time of a whole step:
-    * one sequence, up to 32,000 keys: 0.79 to 0.99;
-    * two: one long and one short, up to 8,192 keys 0.89 to 0.99, 16,000 1.02; of a length, up to 16,380 0.86 to 1.00;
+    * one and two sequences, up to 32,000 keys: 0.79 to 1.01;
     * three and four: one long among short ones, up to 2,048 keys 0.81 to 1.01, 3,060 0.96 to 1.03, 4,090 1.00 to 1.04, 6,000 and 8,190 0.83 to 1.01; falling to
-      half of the longest, up to 4,096 0.73 to 1.02; of a length, up to 16,380 0.72 to 1.02;
+      half of the longest, up to 4,096 0.73 to 1.02; three of a length, up to 16,380 0.81 to 1.02; four, up to 32,000 0.72 to 1.01, falling to 0.8 0.92 to 0.97;
+      one long with 24,000 1.18 to 1.41;
     * five to eight, up to 4,096 keys: 8b sizes 0.98 to 0.99 with 250 and 1.01 to 1.12 with 500 and more; narrower ones, one long 0.93 to 1.01 with 500, 0.94 to 1.02 with 760,
       1.00 to 1.06 with 2,040; five of a length or six falling to half 0.93 to 1.00 up to 1,530, 0.96 to 1.04 with 2,040; eight of a length 0.88 to 1.00;
     * five to eight beyond: one long 1.14 to 1.50 with 8,190, five of a length 1.08 to 1.14; six of a length or eight falling to half 0.96 to 1.00, seven 0.86 to 0.97,
-      eight 0.78 to 0.92, with 10,000 0.88 to 0.94."""
-    if n_tokens <= 1:
+      eight 0.78 to 0.92, with 16,380 0.92 to 0.96, with 32,000 0.95 to 1.01; eight falling to 0.8, 16,380 0.97 to 1.00, 24,000 1.00 to 1.02."""
+    if n_tokens <= 2:
         return True
     full = total / (n_tokens * longest)          # how much of the batch's places times the longest is there
-    if n_tokens <= 2:
-        return room <= (16384 if full >= 0.9 else 8192)
     if n_tokens <= 4:
         if full >= 0.7:
-            return room <= 16384
+            return full >= 0.9 or room <= 16384
         return room <= (4096 if full >= 0.5 else 2048) or 4096 < room <= 8192
     if room > 4096:
-        return room <= (10240 if full >= 0.9 else 8192) and full >= 0.7
+        return full >= (0.7 if room <= 8192 else 0.9 if room <= 16384 else 0.95)
     if hidden > WIDE:
         return room <= 256
     return room <= (4096 if full >= 0.9 else 1536 if full >= 0.4 else 512)
