@@ -166,6 +166,37 @@ def test_a_wait_that_runs_out_is_reported():
     assert float(((got.double() - ref).abs() / ref.abs().amax(dim=-1, keepdim=True)).max()) < TOL
 
 
+def test_a_step_whose_waits_run_out_ends_soon():
+    """Thirty layers, many rounds of the ring each: once a wait has run out the others give up at their next look, so the kernel ends in no more than a few
+    steps' time (a step takes about 1 ms)."""
+    from rocml_b200 import KernelError, kernels
+    lens, H, inter, nq, nkv = [90, 200], 2048, 6144, 16, 8
+    layers, x, table, cs = make(2, H, inter, nq, nkv, lens)
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    real, times = kernels.decode_layers, []
+
+    def often(resid, first, args, *rest):
+        # (thirty layers: the two alternate, the last has no next norm)
+        args = [args[0]] * 29 + [args[1]]
+        a.record()
+        real(resid, first, args, *rest)
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b))
+    kernels.decode_layers = often
+    try:
+        for limit in (0, 1, 1):
+            run(layers, x, table, cs, lens, nq, nkv, inter, 1e-6, True, 2, wait_limit=limit)
+            if limit:
+                with pytest.raises(KernelError, match="wait"):
+                    kernels.check_status(DEV)
+            else:
+                kernels.check_status(DEV)
+    finally:
+        kernels.decode_layers = real
+    assert times[2] < 20.0, times
+
+
 @pytest.mark.parametrize("graphs", [False, True])
 def test_decode_through_the_engine(tmp_path, monkeypatch, graphs):
     """Sequences of unequal lengths decoded together, two ending early; the same with the layers' own kernels, which a model too
